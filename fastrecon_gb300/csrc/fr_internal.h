@@ -168,8 +168,9 @@ int kspace_prepare(fr_plan p, const float *d_kdata, const float *d_dcf, int chan
 int sample_ranges_run(fr_plan p, int *d_start, int *d_end, cudaStream_t s);
 // sos_mode: 2 = the whole SoS (sqrt, / deapod); for coils in slabs 0 = store
 // the plain sum of |x|^2, | 1 = add to the sum already in d_out.
+// shifted: the images are read as shift_run would leave them.
 int sos_run(const float *d_imgs, int channels, int dim, const unsigned *size, const unsigned *recon,
-            const float *d_deapod, float *d_out, cudaStream_t s, int sos_mode = 2);
+            const float *d_deapod, float *d_out, cudaStream_t s, int sos_mode = 2, bool shifted = false);
 int shift_run(float *d_imgs, int channels, int dim, const unsigned *size, cudaStream_t s);
 int crop_run(const float *d_imgs, int channels, int dim, const unsigned *size, const unsigned *crop,
              float *d_out, cudaStream_t s);

@@ -248,9 +248,9 @@ int recon_run(fr_recon r, const float *d_traj, const float *d_dcf, const float *
             if (r->timing && c0 + cs == C) cudaEventRecord(r->ev[3], s);
         } else {
             if (!st) st = fr_fft_execute(r->fft, g, stream);
-            if (!st && !r->checkerboard) st = shift_run(g, cs, r->d.dim, sz, s);
             if (r->timing && c0 + cs == C) cudaEventRecord(r->ev[3], s);
-            if (!st) st = sos_run(g, cs, r->d.dim, sz, r->d.out_size, deapod, d_image, s, mode);
+            // an odd grid's fftShift is in the reads of the SoS
+            if (!st) st = sos_run(g, cs, r->d.dim, sz, r->d.out_size, deapod, d_image, s, mode, !r->checkerboard);
         }
     }
     if (r->timing) {
