@@ -10,12 +10,13 @@
 //    is read through L1/L2 (consecutive samples of a readout share cells).
 //  * Pipe-Menon DCF (Pipe & Menon, MRM 41:179-186, 1999):
 //        w <- w / (C w),  C w = degrid(grid(w)),
-//    with grid(w) a real-valued tile scatter over the plan's bins (shared-
-//    memory accumulation, one flush per tile, no global atomics) and the
-//    degridding fused with the division.
+//    with grid(w) a real-valued tile scatter over the plan's bins, from its
+//    tap lists where it has them (shared-memory accumulation, one flush per
+//    tile, no global atomics) and the degridding fused with the division.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "fr_device.cuh"
 #include "fr_internal.h"
@@ -195,9 +196,130 @@ struct RealGridParams {
     int dim, G, L;
     int tile[3], ntile[3], K;
     float smax, kc;
+    // the plan's tap lists (grid_real_taps_kernel)
+    const unsigned long long *trecs;  // sample | first word << 32 | taps << 40
+    const unsigned *taps;
+    const float *lutw;  // L weights
+    int tap_words;
 };
 
 constexpr int kRealWarps = 8;
+
+// The scatter from the plan's tap lists.  A warp holds 32 records, numbers
+// their groups of 4 taps by a warp scan and deals them 32 per pass, so that
+// every lane has taps to add whatever the records' boxes are (a warp per
+// record, as in grid_real_kernel, leaves most lanes without a tap and spends
+// its time on the box arithmetic).  A lane's group is one 16-byte load when
+// its run starts on a 4-word boundary.  CTAs take work items in turn, so that
+// the weights and the cells' grid offsets (`offs`) are staged once, not per
+// item: most items are a few hundred records.
+// Bound: the shared pipe (table reads at random banks and the float adds,
+// which are compare-and-swap loops), 66 % busy; then the tap words' bytes
+// (about 170 B a sample).  3.1 M samples on a 320^3 grid: 1353 us with a warp
+// per record, 500 us so.  Measured slower: 64-bit fixed-point adds (also
+// compare-and-swap here, 654 us), a half-warp per record with a tile copy each
+// and no atomics (845 us); two 32-bit fixed-point adds were faster (420 us) but
+// hold 38 bits under the item's largest weight, too few for weights of any range.
+constexpr int kRealTapWarps = 4;
+
+__global__ void __launch_bounds__(kRealTapWarps * 32) grid_real_taps_kernel(RealGridParams P, int nitems)
+{
+    extern __shared__ float4 smr[];
+    __shared__ int4 table[kRealTapWarps][32];
+    float *acc = reinterpret_cast<float *>(smr);
+    int *offs = reinterpret_cast<int *>(acc + P.K);
+    float *lutw = reinterpret_cast<float *>(offs + P.K);
+    const int Tx = P.tile[0], Ty = P.tile[1], Tz = P.tile[2];
+    const size_t G = (size_t)P.G;
+    const int Gz = P.dim == 3 ? P.G : 1;
+    for (int i = threadIdx.x; i < P.K; i += blockDim.x) {
+        const int lx = i % Tx, r = i / Tx, ly = r % Ty, lz = r / Ty;
+        offs[i] = (lz * P.G + ly) * P.G + lx;  // below 64 * 4096^2
+        acc[i] = 0.f;
+    }
+    for (int i = threadIdx.x; i < P.L; i += blockDim.x) lutw[i] = P.lutw[i];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned cmask = (1u << kTapCellBits) - 1u;
+    __syncthreads();
+    for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+        const WorkItem it = P.items[item];
+        const unsigned long long *trecs = P.trecs + it.begin;
+        for (int j0 = warp * 32; j0 < it.count; j0 += kRealTapWarps * 32) {
+            const unsigned long long rw = j0 + lane < it.count ? __ldg(trecs + j0 + lane) : 0ull;
+            const int nt = (int)((rw >> 40) & 0xFF);
+            const int np = (nt + 3) >> 2;
+            const unsigned nz = __ballot_sync(0xffffffffu, np > 0);
+            int incl = np;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            const int excl = incl - np;
+            const int total = __shfl_sync(0xffffffffu, incl, 31);
+            if (np > 0)
+                table[warp][__popc(nz & ((1u << lane) - 1u))] =
+                    make_int4((int)(unsigned)rw, (int)(((rw >> 32) & 0xFF) | ((unsigned)nt << 8)), excl,
+                              __float_as_int(P.w[(unsigned)rw]));
+            __syncwarp();
+            int recbase = 0;
+            for (int p0 = 0; p0 < total; p0 += 32) {
+                // bit i of starts: a record's first group is group p0 + i
+                const bool in_pass = np > 0 && excl >= p0 && excl < p0 + 32;
+                const unsigned starts = __reduce_or_sync(0xffffffffu, in_pass ? 1u << (excl - p0) : 0u);
+                const int cr = recbase + __popc(starts & (0xffffffffu >> (31 - lane))) - 1;
+                recbase += __popc(starts);
+                if (p0 + lane < total) {
+                    const int4 e = table[warp][cr];
+                    const int gi = 4 * (p0 + lane - e.z);
+                    const int nl = min((e.y >> 8) - gi, 4);
+                    const size_t tb = (size_t)(unsigned)e.x * (size_t)P.tap_words + (size_t)((e.y & 0xFF) + gi);
+                    unsigned tg[4] = {0u, 0u, 0u, 0u};
+                    if ((tb & 3) == 0) {  // slots are multiples of 4 words: the group stays in the slot
+                        const uint4 q = __ldg(reinterpret_cast<const uint4 *>(P.taps + tb));
+                        tg[0] = q.x;
+                        tg[1] = q.y;
+                        tg[2] = q.z;
+                        tg[3] = q.w;
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (k < nl) tg[k] = __ldg(P.taps + tb + k);
+                    }
+                    const float v = __int_as_float(e.w);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (k < nl)
+                            atomicAdd(&acc[min(tg[k] & cmask, (unsigned)(P.K - 1))],
+                                      lutw[min(tg[k] >> kTapCellBits, (unsigned)(P.L - 1))] * v);
+                }
+            }
+            __syncwarp();  // the next batch rewrites the table
+        }
+        __syncthreads();
+        // flush, and zero for the next item
+        const int t = it.tile;
+        const int ty = t / P.ntile[0], tz = ty / P.ntile[1];
+        const int ox = (t - ty * P.ntile[0]) * Tx, oy = (ty - tz * P.ntile[1]) * Ty, oz = tz * Tz;
+        float *dst = it.slot >= 0 ? P.partials + (size_t)it.slot * P.K : P.grid + ((size_t)oz * G + oy) * G + ox;
+        const bool inside = ox + Tx <= P.G && oy + Ty <= P.G && oz + Tz <= Gz;
+        for (int i = threadIdx.x; i < P.K; i += blockDim.x) {
+            const float v = acc[i];
+            acc[i] = 0.f;
+            if (it.slot >= 0) {
+                dst[i] = v;
+            } else {
+                bool in = inside;
+                if (!inside) {
+                    const int lx = i % Tx, r = i / Tx;
+                    in = ox + lx < P.G && oy + r % Ty < P.G && oz + r / Ty < Gz;
+                }
+                if (in) dst[offs[i]] = v;
+            }
+        }
+        __syncthreads();
+    }
+}
 
 __global__ void __launch_bounds__(kRealWarps * 32) grid_real_kernel(RealGridParams P)
 {
@@ -265,26 +387,65 @@ __global__ void reduce_real_splits_kernel(RealGridParams P)
         const int lx = i % P.tile[0], r = i / P.tile[0], ly = r % P.tile[1], lz = r / P.tile[1];
         const int gx = ox + lx, gy = oy + ly, gz = oz + lz;
         if (gx >= P.G || gy >= P.G || gz >= Gz) continue;
+        // slot after slot, 8 loads in flight (3.1 M samples, 320^3: 31 -> 10 us)
         float v = 0.f;
-        for (int k = 0; k < st.nslots; ++k) v = __fadd_rn(v, base[(size_t)k * P.K + i]);
+        int k = 0;
+        for (; k + 8 <= st.nslots; k += 8) {
+            float a[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) a[u] = base[(size_t)(k + u) * P.K + i];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v = __fadd_rn(v, a[u]);
+        }
+        for (; k < st.nslots; ++k) v = __fadd_rn(v, base[(size_t)k * P.K + i]);
         P.grid[((size_t)gz * G + gy) * G + gx] = v;
     }
 }
 
-// Degrid a real grid at each sample and divide the sample's weight by it.
-__global__ void __launch_bounds__(256) pipe_update_kernel(DegridParams P, const float *__restrict__ g, float *w)
+// The cells of a footprint along one axis: clamped range (GridLut.cpp:98-106),
+// ends at distance kHW dropped where that is exact (they never pass dk < kHW).
+__device__ __forceinline__ void footprint(const DegridParams &P, int trim, float c, int &s, int &e)
 {
-    extern __shared__ float4 lutS[];
-    for (int i = threadIdx.x; i < P.L; i += blockDim.x) lutS[i] = P.lut_e[i];
+    comp_range(c, P.hw, P.G, s, e);
+    if (trim && s <= e) {
+        if (!(fabsf(__fsub_rn((float)s, c)) < P.hw)) ++s;
+        if (s <= e && !(fabsf(__fsub_rn((float)e, c)) < P.hw)) --e;
+    }
+}
+
+// Degrid a real grid at each sample and divide the sample's weight by it.
+// XR >= 2 hw bounds the cells along x, whose dx^2 are computed once (+inf past
+// the footprint); thresholds and weights are read as single words.
+// Bound: the L1 data pipe, for the scattered rows and the weight table.  3.1 M
+// samples on a 320^3 grid: 340 us with the table as float4 entries (87 % of the
+// pipe), 250 us so.  Measured slower: a row's cells as two aligned float4
+// (396 us), the tile's cells staged in shared memory (600 us: staging, and
+// half-filled warps at a median of 119 records per tile), the tap lists (361 us).
+template <int XR>
+__global__ void __launch_bounds__(256) pipe_update_kernel(DegridParams P, int trim, const float *__restrict__ lutw,
+                                                          const float *__restrict__ g, float *w)
+{
+    extern __shared__ float tabs[];  // thr [L] (index k + 1 from thr[k] on), weights [L]
+    float *thr = tabs, *lut = tabs + P.L;
+    for (int i = threadIdx.x; i < P.L; i += blockDim.x) {
+        thr[i] = P.lut_e[i].x;
+        lut[i] = lutw[i];
+    }
     __syncthreads();
     const size_t G = (size_t)P.G;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < P.n;
          i += (long long)gridDim.x * blockDim.x) {
         const float4 p = P.traj[i];
         int xs, xe, ys, ye, zs = 0, ze = 0;
-        comp_range(p.x, P.hw, P.G, xs, xe);
-        comp_range(p.y, P.hw, P.G, ys, ye);
-        if (P.dim == 3) comp_range(p.z, P.hw, P.G, zs, ze);
+        footprint(P, trim, p.x, xs, xe);
+        footprint(P, trim, p.y, ys, ye);
+        if (P.dim == 3) footprint(P, trim, p.z, zs, ze);
+        float dx2[XR];
+#pragma unroll
+        for (int k = 0; k < XR; ++k) {
+            const float dx = __fsub_rn((float)(xs + k), p.x);
+            dx2[k] = xs + k <= xe ? __fmul_rn(dx, dx) : __int_as_float(0x7f800000);
+        }
         float acc = 0.f;
         for (int z = zs; z <= ze; ++z) {
             const float dz = P.dim == 3 ? __fsub_rn((float)z, p.z) : 0.f;
@@ -292,12 +453,17 @@ __global__ void __launch_bounds__(256) pipe_update_kernel(DegridParams P, const 
             for (int y = ys; y <= ye; ++y) {
                 const float dy = __fsub_rn((float)y, p.y);
                 const float dzy = __fadd_rn(dz2, __fmul_rn(dy, dy));
-                const float *grow = g + ((size_t)z * G + (size_t)y) * G;
-                for (int x = xs; x <= xe; ++x) {
-                    const float dx = __fsub_rn((float)x, p.x);
-                    float wt;
-                    if (lut_weight(__fadd_rn(dzy, __fmul_rn(dx, dx)), lutS, P.smax, P.kc, P.L, wt))
-                        acc = fmaf(wt, grow[x], acc);
+                const float *row = g + ((size_t)z * G + (size_t)y) * G + xs;
+#pragma unroll
+                for (int k = 0; k < XR; ++k) {
+                    const float s2 = __fadd_rn(dzy, dx2[k]);
+                    if (s2 < P.smax) {
+                        float a;
+                        asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(s2));
+                        const int k0 = min((int)fmaf(a, P.kc, 0.25f), P.L - 1);
+                        const float wt = lut[k0 + (s2 >= thr[k0] ? 1 : 0)];  // thr[L - 1] is +inf
+                        acc = fmaf(wt, __ldg(row + k), acc);
+                    }
                 }
             }
         }
@@ -425,12 +591,27 @@ int grid_real_run(fr_plan p, const float *d_w, float *d_grid, cudaStream_t s)
     if (p->nslots > 0 && p->real_partials.reserve((size_t)p->nslots * P.K * 4)) return FR_ERR_CUDA;
     P.partials = p->real_partials.as<float>();
     if (p->nitems == 0) return FR_OK;
+    P.trecs = p->trecs.as<unsigned long long>();
+    P.taps = p->taps.as<unsigned>();
+    P.lutw = p->lut_d.as<float>();
+    P.tap_words = p->tap_words;
     const size_t smem = (size_t)P.L * 16 + (size_t)P.K * 4;
     if (smem > 227 * 1024) return fail(FR_ERR_UNSUPPORTED, "tile too large for the real-valued scatter");
-    if (smem > 48 * 1024)
-        FR_CUDA(cudaFuncSetAttribute(grid_real_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    grid_real_kernel<<<(unsigned)p->nitems, kRealWarps * 32, smem, s>>>(P);
-    FR_CHECK_LAUNCH("grid_real_kernel");
+    if (p->tap_words > 0) {  // plans without tap lists evaluate each record's box
+        const size_t tsmem = (size_t)P.L * 4 + (size_t)P.K * 8;
+        if (tsmem > 40 * 1024)
+            FR_CUDA(cudaFuncSetAttribute(grid_real_taps_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem));
+        int per_sm = 0;
+        FR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grid_real_taps_kernel, kRealTapWarps * 32, tsmem));
+        const long long nb = std::min<long long>(p->nitems, (long long)std::max(per_sm, 1) * sm_count());
+        grid_real_taps_kernel<<<(unsigned)nb, kRealTapWarps * 32, tsmem, s>>>(P, (int)p->nitems);
+        FR_CHECK_LAUNCH("grid_real_taps_kernel");
+    } else {
+        if (smem > 48 * 1024)
+            FR_CUDA(cudaFuncSetAttribute(grid_real_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        grid_real_kernel<<<(unsigned)p->nitems, kRealWarps * 32, smem, s>>>(P);
+        FR_CHECK_LAUNCH("grid_real_kernel");
+    }
     if (p->nsplits > 0) {
         reduce_real_splits_kernel<<<(unsigned)p->nsplits, 256, 0, s>>>(P);
         FR_CHECK_LAUNCH("reduce_real_splits_kernel");
@@ -446,14 +627,23 @@ int dcf_pipe_run(fr_plan p, int iterations, float *d_w, cudaStream_t s)
     const size_t cells = p->dim == 3 ? (size_t)p->G * p->G * p->G : (size_t)p->G * p->G;
     if (p->real_grid.reserve(cells * 4)) return FR_ERR_CUDA;
     DegridParams P = degrid_params(p);
-    const size_t smem = (size_t)P.L * 16;
+    const size_t smem = (size_t)P.L * 8;
+    // most cells along an axis: an open interval of length 2 hw holds at most
+    // ceil(2 hw); without the exact trim floor(2 hw) + 1, where the rounding of
+    // c - hw and c + hw (below 2^-11) can add one if 2 hw is just below an integer
+    const int trim = p->prefilter;
+    const int reach = trim ? (int)std::ceil(2.0 * p->hw) : (int)std::floor(2.0 * p->hw + 1e-3) + 1;
+    auto kern = reach <= 4 ? pipe_update_kernel<4> : reach <= 5 ? pipe_update_kernel<5>
+                : reach <= 9 ? pipe_update_kernel<9> : pipe_update_kernel<14>;  // widths up to 13
     if (smem > 48 * 1024)
-        FR_CUDA(cudaFuncSetAttribute(pipe_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int bx = (int)std::min<long long>((P.n + 255) / 256, (long long)sm_count() * 8);
+        FR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    FR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
+    const int bx = (int)std::min<long long>((P.n + 255) / 256, (long long)sm_count() * std::max(per_sm, 1));  // one wave
     for (int it = 0; it < iterations; ++it) {
         int st = grid_real_run(p, d_w, p->real_grid.as<float>(), s);
         if (st) return st;
-        pipe_update_kernel<<<bx, 256, smem, s>>>(P, p->real_grid.as<float>(), d_w);
+        kern<<<bx, 256, smem, s>>>(P, trim, p->lut_d.as<float>(), p->real_grid.as<float>(), d_w);
         FR_CHECK_LAUNCH("pipe_update_kernel");
     }
     return FR_OK;
