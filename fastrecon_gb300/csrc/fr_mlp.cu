@@ -12,12 +12,10 @@
 //    parameters widened into shared memory once per CTA; first-layer units
 //    are produced one at a time and scattered into the 64 second-layer
 //    accumulators held in registers.
-//  * backward: mlp_train_kernel does the forward pass and the per-sample
-//    reverse pass (dL/dy, the two hidden-layer deltas) and writes the
-//    per-sample activations and deltas; mlp_grad_kernel reduces the
-//    outer products over a block of samples into one partial gradient per
-//    CTA; mlp_reduce_kernel sums the partials in a fixed order (the
-//    gradient is deterministic).
+//  * backward: mlp_step_kernel does the forward and reverse pass of tiles of
+//    64 samples in shared memory and keeps the gradient of its tiles in
+//    registers, one partial gradient per CTA; mlp_reduce_kernel sums the
+//    partials in a fixed order (the gradient is deterministic).
 //  * mlp_adam_kernel: Adam on the master copy, then the BF16 copy.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -41,7 +39,6 @@ constexpr int OFF_B3 = OFF_W3 + NH;
 constexpr int NP = OFF_B3 + 1;
 static_assert(NP == FR_MLP_PARAMS, "parameter layout");
 
-constexpr int kGradSamples = 256;  // samples reduced by one mlp_grad_kernel CTA
 constexpr int kFwdThreads = 128;
 
 // Widen the BF16 parameters into shared memory, W2 transposed (row i of the
@@ -80,22 +77,6 @@ __device__ __forceinline__ void axpy_row(const float *ps, int i, float v, float 
         acc[4 * q + 2] = fmaf(c.z, v, acc[4 * q + 2]);
         acc[4 * q + 3] = fmaf(c.w, v, acc[4 * q + 3]);
     }
-}
-
-// sum_j W2[j][i] * d[j] (row i of the transposed copy).
-__device__ __forceinline__ float dot_row(const float *ps, int i, const float *d)
-{
-    const float4 *w = reinterpret_cast<const float4 *>(ps + OFF_W2 + i * NH);
-    float a = 0.f;
-#pragma unroll
-    for (int q = 0; q < NH / 4; ++q) {
-        const float4 c = w[q];
-        a = fmaf(c.x, d[4 * q], a);
-        a = fmaf(c.y, d[4 * q + 1], a);
-        a = fmaf(c.z, d[4 * q + 2], a);
-        a = fmaf(c.w, d[4 * q + 3], a);
-    }
-    return a;
 }
 
 // Second-layer activations h2 (in place of the pre-activations) and the output.
@@ -258,149 +239,253 @@ __global__ void __launch_bounds__(kMmaThreads) mlp_forward_mma_kernel(const __nv
     }
 }
 
-// Forward + per-sample reverse pass of the (optionally weighted) mean squared
-// error (1/n) sum_s c_s (y_s - t_s)^2.  Writes H1, H2, D1, D2 (64 x n each,
-// unit-major so that a warp's stores are coalesced), DY (n) and one partial
-// sum of squared residuals per CTA.  First-layer units are recomputed where
-// needed, so only one 64-wide register array is live.
-__global__ void __launch_bounds__(kFwdThreads) mlp_train_kernel(const __nv_bfloat16 *__restrict__ pb,
-                                                                const float *__restrict__ x,
-                                                                const float *__restrict__ t,
-                                                                const float *__restrict__ cw, long long n,
-                                                                float *H1, float *H2, float *D1, float *D2, float *DY,
-                                                                float *loss_part)
+// Forward and reverse pass of the (optionally weighted) mean squared error
+// (1/n) sum_s c_s (y_s - t_s)^2 and its gradient, tiles of 64 samples: the
+// three 64 x 64 x 64 products of a tile (W2 h1, W2^T d2, d2 h1^T) from shared
+// memory, a 4 x 4 block per thread, in FP32; the gradient stays in registers
+// from tile to tile and leaves as one partial per CTA.  Activations and deltas
+// are held unit-major ([unit][sample], rows of kRow floats, so that 8 lanes on
+// 8 rows cover the banks).
+// Bound: FP32 issue (0.8 M FMA and 8192 tanh a tile), then the latency of one
+// tile.  16,384 samples: 92 us for the gradient kernel (64 CTAs, activations
+// and deltas through memory) and 29 us for the pass before it, 31 us so; the
+// whole step with Adam 124 -> 37 us.
+constexpr int kTile = 64;              // samples per tile
+constexpr int kRow = kTile + 4;        // floats per shared row
+constexpr int kStepThreads = 256;      // 16 x 16 blocks of 4 x 4
+constexpr int kStepSmem = (4 * NH * kRow + kTile * NI + 2 * kTile + NH * NI + 3 * NH + 4) * 4;
+static_assert(NH == 64 && kTile == 64, "16 x 16 threads of 4 x 4 outputs");
+
+__device__ __forceinline__ void outer4(float (&c)[4][4], const float4 a, const float4 b)
 {
-    __shared__ __align__(16) float ps[NP + 3];
-    __shared__ float red[kFwdThreads / 32];
-    load_params(pb, ps);
-    const float inv_n = 1.f / (float)n;
-    float lsum = 0.f;
-    for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < n; s += (long long)gridDim.x * blockDim.x) {
-        float xs[NI], a[NH];
+    const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-        for (int k = 0; k < NI; ++k) xs[k] = x[s * NI + k];
-        const float out = forward_sample(ps, xs, a);
-        const float r = out - t[s];
-        const float c = cw ? cw[s] : 1.f;
-        lsum = fmaf(c * r, r, lsum);
-        const float dy = 2.f * c * r * inv_n;
-        DY[s] = dy;
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < NH; ++j) {
-            H2[(size_t)j * n + s] = a[j];
-            a[j] = dy * ps[OFF_W3 + j] * (1.f - a[j] * a[j]);  // delta of layer 2
-            D2[(size_t)j * n + s] = a[j];
-        }
-#pragma unroll 1
-        for (int i = 0; i < NH; ++i) {
-            const float h = unit1(ps, xs, i);
-            H1[(size_t)i * n + s] = h;
-            D1[(size_t)i * n + s] = dot_row(ps, i, a) * (1.f - h * h);
-        }
-    }
-    for (int d = 16; d; d >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, d);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = lsum;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float v = 0.f;
-        for (int w = 0; w < kFwdThreads / 32; ++w) v += red[w];
-        loss_part[blockIdx.x] = v;
-    }
+        for (int j = 0; j < 4; ++j) c[i][j] = fmaf(av[i], bv[j], c[i][j]);
 }
 
-// Partial gradient of samples [b*256, b*256+256): 256 threads, each owning
-// 16 entries of gW2 and at most 3 of the other parameters.
-__global__ void __launch_bounds__(256) mlp_grad_kernel(const float *__restrict__ x, long long n,
-                                                       const float *__restrict__ H1, const float *__restrict__ H2,
-                                                       const float *__restrict__ D1, const float *__restrict__ D2,
-                                                       const float *__restrict__ DY, float *partials)
+__global__ void __launch_bounds__(kStepThreads, 2) mlp_step_kernel(const __nv_bfloat16 *__restrict__ pb,
+                                                                   const float *__restrict__ x,
+                                                                   const float *__restrict__ t,
+                                                                   const float *__restrict__ cw, long long n,
+                                                                   float *__restrict__ partials,
+                                                                   float *__restrict__ loss_part)
 {
-    constexpr int CH = 32;  // samples staged per step
-    __shared__ __align__(16) float sh1[CH][NH], sh2[CH][NH], sd1[CH][NH], sd2[CH][NH];
-    __shared__ float sx[CH][NI], sdy[CH];
-    const int tid = threadIdx.x;
-    const int j2 = tid >> 2, i2 = (tid & 3) * 16;  // gW2 rows j2, columns i2..i2+15
-    float g2[16];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) g2[k] = 0.f;
-    float g1[NI];  // gW1 row tid (tid < 64)
-#pragma unroll
-    for (int k = 0; k < NI; ++k) g1[k] = 0.f;
-    float gb = 0.f;  // b1 (tid < 64), b2 (64..127), W3 (128..191), b3 (192)
-    const long long s0 = (long long)blockIdx.x * kGradSamples;
-    const long long s1 = min(s0 + kGradSamples, n);
-    for (long long c = s0; c < s1; c += CH) {
-        const int m = (int)(s1 - c < CH ? s1 - c : CH);
-        __syncthreads();
-        for (int e = tid; e < CH * NH; e += 256) {
-            const int q = e / CH, r = e % CH;
-            const bool ok = r < m;
-            const size_t g = (size_t)q * n + (size_t)(c + r);
-            sh1[r][q] = ok ? H1[g] : 0.f;
-            sh2[r][q] = ok ? H2[g] : 0.f;
-            sd1[r][q] = ok ? D1[g] : 0.f;
-            sd2[r][q] = ok ? D2[g] : 0.f;
+    extern __shared__ float4 sm4[];
+    float *w2 = reinterpret_cast<float *>(sm4);  // [j][i]
+    float *w2t = w2 + NH * kRow;                 // [i][j]
+    float *h1 = w2t + NH * kRow;                 // [i][s]
+    float *d2 = h1 + NH * kRow;                  // [j][s]
+    float *xs = d2 + NH * kRow;                  // [s][NI]
+    float *ts = xs + kTile * NI;                 // targets
+    float *cs = ts + kTile;                      // sample weights (0 past the batch)
+    float *w1 = cs + kTile;                      // [i][NI]
+    float *b1 = w1 + NH * NI, *b2 = b1 + NH, *w3 = b2 + NH, *b3 = w3 + NH;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    for (int p = tid; p < NP; p += kStepThreads) {
+        const float v = __bfloat162float(pb[p]);
+        if (p < OFF_B1) w1[p] = v;
+        else if (p < OFF_W2) b1[p - OFF_B1] = v;
+        else if (p < OFF_B2) {
+            const int j = (p - OFF_W2) / NH, i = (p - OFF_W2) % NH;
+            w2[j * kRow + i] = v;
+            w2t[i * kRow + j] = v;
+        } else if (p < OFF_W3) b2[p - OFF_B2] = v;
+        else if (p < OFF_B3) w3[p - OFF_W3] = v;
+        else b3[0] = v;
+    }
+    const float inv_n = 1.f / (float)n;
+    // gradients of this thread: W2[ty + 16 a][tx + 16 b]; W1 and b1 of units
+    // 4 tx + k, W3 and b2 of units 4 tx + k (over its samples), b3, loss
+    float g2[4][4] = {}, g1[4][NI] = {}, gb1[4] = {}, gw3[4] = {}, gb2[4] = {}, gb3 = 0.f, lsum = 0.f;
+    const long long ntile = (n + kTile - 1) / kTile;
+    for (long long tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+        const long long s0 = tile * kTile;
+        __syncthreads();  // tables staged; the last tile's rows no longer read
+        for (int e = tid; e < kTile * NI; e += kStepThreads) xs[e] = s0 * NI + e < n * NI ? x[s0 * NI + e] : 0.f;
+        if (tid < kTile) {
+            const bool in = s0 + tid < n;
+            ts[tid] = in ? t[s0 + tid] : 0.f;
+            cs[tid] = in ? (cw ? cw[s0 + tid] : 1.f) : 0.f;
         }
-        for (int e = tid; e < CH * NI; e += 256) {
-            const int r = e / NI, q = e % NI;
-            sx[r][q] = r < m ? x[(size_t)(c + r) * NI + q] : 0.f;
-        }
-        if (tid < CH) sdy[tid] = tid < m ? DY[c + tid] : 0.f;
         __syncthreads();
-        for (int r = 0; r < CH; ++r) {
-            const float d = sd2[r][j2];
-            const float4 *h = reinterpret_cast<const float4 *>(&sh1[r][i2]);
+        {  // first layer: sample tid % 64, units 16 (tid / 64) + k
+            const int s = tid & 63, i0 = (tid >> 6) * 16;
+            float xv[NI];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float4 v = h[k];
-                g2[4 * k] = fmaf(d, v.x, g2[4 * k]);
-                g2[4 * k + 1] = fmaf(d, v.y, g2[4 * k + 1]);
-                g2[4 * k + 2] = fmaf(d, v.z, g2[4 * k + 2]);
-                g2[4 * k + 3] = fmaf(d, v.w, g2[4 * k + 3]);
-            }
-            if (tid < NH) {
-                const float d1 = sd1[r][tid];
+            for (int k = 0; k < NI; ++k) xv[k] = xs[s * NI + k];
+#pragma unroll 4
+            for (int i = i0; i < i0 + 16; ++i) {
+                float a = b1[i];
 #pragma unroll
-                for (int k = 0; k < NI; ++k) g1[k] = fmaf(d1, sx[r][k], g1[k]);
-                gb += d1;
-            } else if (tid < 2 * NH) {
-                gb += sd2[r][tid - NH];
-            } else if (tid < 3 * NH) {
-                gb = fmaf(sdy[r], sh2[r][tid - 2 * NH], gb);
-            } else if (tid == 3 * NH) {
-                gb += sdy[r];
+                for (int k = 0; k < NI; ++k) a = fmaf(w1[i * NI + k], xv[k], a);
+                h1[i * kRow + s] = tanhf(a);
             }
+        }
+        __syncthreads();
+        {  // second layer and output: samples 4 ty + i, units 4 tx + j
+            float a[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) a[i][j] = b2[4 * tx + j];
+#pragma unroll 8
+            for (int k = 0; k < NH; ++k)
+                outer4(a, *reinterpret_cast<const float4 *>(h1 + k * kRow + 4 * ty),
+                       *reinterpret_cast<const float4 *>(w2t + k * kRow + 4 * tx));
+            const float4 wv = *reinterpret_cast<const float4 *>(w3 + 4 * tx);
+            const float w[4] = {wv.x, wv.y, wv.z, wv.w};
+            float dy[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float o = 0.f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    a[i][j] = tanhf(a[i][j]);
+                    o = fmaf(w[j], a[i][j], o);
+                }
+#pragma unroll
+                for (int d = 1; d < 16; d <<= 1) o += __shfl_xor_sync(0xffffffffu, o, d);
+                const float r = (o + b3[0]) - ts[4 * ty + i], c = cs[4 * ty + i];
+                dy[i] = 2.f * c * r * inv_n;
+                if (tx == 0) {
+                    lsum = fmaf(c * r, r, lsum);
+                    gb3 += dy[i];
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float v[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    gw3[j] = fmaf(dy[i], a[i][j], gw3[j]);
+                    v[i] = dy[i] * w[j] * (1.f - a[i][j] * a[i][j]);
+                    gb2[j] += v[i];
+                }
+                *reinterpret_cast<float4 *>(d2 + (4 * tx + j) * kRow + 4 * ty) = make_float4(v[0], v[1], v[2], v[3]);
+            }
+        }
+        __syncthreads();
+        {  // first layer's deltas: samples 4 ty + i, units 4 tx + j
+            float a[4][4] = {};
+#pragma unroll 8
+            for (int k = 0; k < NH; ++k)
+                outer4(a, *reinterpret_cast<const float4 *>(d2 + k * kRow + 4 * ty),
+                       *reinterpret_cast<const float4 *>(w2 + k * kRow + 4 * tx));
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 hv = *reinterpret_cast<const float4 *>(h1 + (4 * tx + j) * kRow + 4 * ty);
+                const float h[4] = {hv.x, hv.y, hv.z, hv.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float d = a[i][j] * (1.f - h[i] * h[i]);
+                    gb1[j] += d;
+#pragma unroll
+                    for (int k = 0; k < NI; ++k) g1[j][k] = fmaf(d, xs[(4 * ty + i) * NI + k], g1[j][k]);
+                }
+            }
+        }
+        // W2's gradient: rows ty + 16 a of d2, rows tx + 16 b of h1
+#pragma unroll 4
+        for (int s = 0; s < kTile; s += 4) {
+            float4 dv[4], hv[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                dv[a] = *reinterpret_cast<const float4 *>(d2 + (ty + 16 * a) * kRow + s);
+                hv[a] = *reinterpret_cast<const float4 *>(h1 + (tx + 16 * a) * kRow + s);
+            }
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    g2[a][b] = fmaf(dv[a].x, hv[b].x, g2[a][b]);
+                    g2[a][b] = fmaf(dv[a].y, hv[b].y, g2[a][b]);
+                    g2[a][b] = fmaf(dv[a].z, hv[b].z, g2[a][b]);
+                    g2[a][b] = fmaf(dv[a].w, hv[b].w, g2[a][b]);
+                }
         }
     }
     float *out = partials + (size_t)blockIdx.x * NP;
 #pragma unroll
-    for (int k = 0; k < 16; ++k) out[OFF_W2 + j2 * NH + i2 + k] = g2[k];
-    if (tid < NH) {
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int k = 0; k < NI; ++k) out[OFF_W1 + tid * NI + k] = g1[k];
-        out[OFF_B1 + tid] = gb;
-    } else if (tid < 2 * NH) {
-        out[OFF_B2 + tid - NH] = gb;
-    } else if (tid < 3 * NH) {
-        out[OFF_W3 + tid - 2 * NH] = gb;
-    } else if (tid == 3 * NH) {
-        out[OFF_B3] = gb;
+        for (int b = 0; b < 4; ++b) out[OFF_W2 + (ty + 16 * a) * NH + tx + 16 * b] = g2[a][b];
+    // the rest over the 16 ty: the warp's two by a shuffle, the 8 warps in
+    // shared memory ([warp][unit][W1 row, b1, W3, b2], then b3 and loss)
+    constexpr int NV = NI + 3;
+    __syncthreads();
+    float *red = w2;
+    float *rows = red + 8 * NH * NV;
+    const int warp = tid >> 5;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        float v[NV];
+#pragma unroll
+        for (int k = 0; k < NI; ++k) v[k] = g1[j][k];
+        v[NI] = gb1[j];
+        v[NI + 1] = gw3[j];
+        v[NI + 2] = gb2[j];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            v[k] += __shfl_xor_sync(0xffffffffu, v[k], 16);
+            if ((tid & 16) == 0) red[(warp * NH + 4 * tx + j) * NV + k] = v[k];
+        }
+    }
+    gb3 += __shfl_xor_sync(0xffffffffu, gb3, 16);
+    lsum += __shfl_xor_sync(0xffffffffu, lsum, 16);
+    if ((tid & 31) == 0) {
+        rows[2 * warp] = gb3;
+        rows[2 * warp + 1] = lsum;
+    }
+    __syncthreads();
+    for (int e = tid; e < NH * NV; e += kStepThreads) {
+        const int u = e / NV, k = e % NV;
+        float v = 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v += red[(q * NH + u) * NV + k];
+        out[k < NI ? OFF_W1 + u * NI + k : k == NI ? OFF_B1 + u : k == NI + 1 ? OFF_W3 + u : OFF_B2 + u] = v;
+    }
+    if (tid < 2) {
+        float v = 0.f;
+        for (int q = 0; q < 8; ++q) v += rows[2 * q + tid];
+        if (tid == 0) out[OFF_B3] = v;
+        else loss_part[blockIdx.x] = v;
     }
 }
 
-__global__ void mlp_reduce_kernel(const float *__restrict__ partials, int nblocks, const float *__restrict__ loss_part,
-                                  int nloss, float inv_n, float *grad, float *loss)
+// Sum of the CTAs' partial gradients, 32 parameters per CTA: thread (slice,
+// parameter) sums every 8th partial, then the 8 slices in order.  The last CTA
+// sums the loss.  (One thread per
+// parameter over 64 partials: 8 us; 256 partials so: 7 us.)
+__global__ void __launch_bounds__(256) mlp_reduce_kernel(const float *__restrict__ partials, int nparts,
+                                                         const float *__restrict__ loss_part, float inv_n, float *grad,
+                                                         float *loss)
 {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < NP) {
-        float a = 0.f;
-        for (int b = 0; b < nblocks; ++b) a += partials[(size_t)b * NP + p];
-        grad[p] = a;
+    __shared__ float part[8][33];
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+    const bool is_loss = blockIdx.x == gridDim.x - 1;
+    const int p = blockIdx.x * 32 + lane;
+    float a = 0.f;
+    if (is_loss) {
+        for (int b = slice * 32 + lane; b < nparts; b += 256) a += loss_part[b];
+    } else if (p < NP) {
+#pragma unroll 4
+        for (int b = slice; b < nparts; b += 8) a += partials[(size_t)b * NP + p];
     }
-    if (p == 0 && loss) {
-        float a = 0.f;
-        for (int b = 0; b < nloss; ++b) a += loss_part[b];
-        *loss = a * inv_n;
+    part[slice][lane] = a;
+    __syncthreads();
+    if (slice == 0) {
+        float v = 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v += part[q][lane];
+        if (is_loss) {
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+            if (lane == 0 && loss) *loss = v * inv_n;
+        } else if (p < NP) {
+            grad[p] = v;
+        }
     }
 }
 
@@ -440,15 +525,18 @@ bool mlp_use_simt()
     return e && std::atoi(e) != 0;
 }
 
-int train_blocks(long long n) { return (int)std::max<long long>(1, std::min<long long>((n + kFwdThreads - 1) / kFwdThreads, (long long)sm_count_mlp() * 8)); }
+// CTAs of the training step: one per tile up to two per SM.
+int step_blocks(size_t n)
+{
+    return (int)std::min<long long>((long long)((n + kTile - 1) / kTile), 2ll * sm_count_mlp());
+}
 
 }  // namespace
 
 size_t mlp_workspace_bytes(size_t n)
 {
-    const size_t gblocks = (n + kGradSamples - 1) / kGradSamples;
-    const size_t a = (4 * (size_t)NH + 1) * n * 4;
-    return a + std::max<size_t>(gblocks, 1) * NP * 4 + (size_t)train_blocks((long long)std::max<size_t>(n, 1)) * 4 + 256;
+    // a partial gradient and loss per CTA
+    return (size_t)step_blocks(std::max<size_t>(n, 1)) * (NP + 1) * 4 + 256;
 }
 
 int mlp_forward_run(const void *d_params, const float *d_x, size_t n, int exp_out, int residual, float scale,
@@ -476,22 +564,14 @@ int mlp_backward_run(const void *d_params, const float *d_x, const float *d_t, c
                      float *d_grad, float *d_loss, cudaStream_t s)
 {
     if (n == 0) return fail(FR_ERR_INVALID_ARGUMENT, "empty batch");
-    float *H1 = static_cast<float *>(ws);
-    float *H2 = H1 + (size_t)NH * n;
-    float *D1 = H2 + (size_t)NH * n;
-    float *D2 = D1 + (size_t)NH * n;
-    float *DY = D2 + (size_t)NH * n;
-    float *partials = DY + n;
-    const int gblocks = (int)((n + kGradSamples - 1) / kGradSamples);
-    float *loss_part = partials + (size_t)gblocks * NP;
-    const int tb = train_blocks((long long)n);
-    mlp_train_kernel<<<tb, kFwdThreads, 0, s>>>(static_cast<const __nv_bfloat16 *>(d_params), d_x, d_t, d_w, (long long)n,
-                                                H1, H2, D1, D2, DY, loss_part);
-    FR_CHECK_LAUNCH("mlp_train_kernel");
-    mlp_grad_kernel<<<gblocks, 256, 0, s>>>(d_x, (long long)n, H1, H2, D1, D2, DY, partials);
-    FR_CHECK_LAUNCH("mlp_grad_kernel");
-    mlp_reduce_kernel<<<(NP + 255) / 256, 256, 0, s>>>(partials, gblocks, loss_part, tb, 1.f / (float)n, d_grad,
-                                                      d_loss);
+    const int nb = step_blocks(n);
+    float *partials = static_cast<float *>(ws);
+    float *loss_part = partials + (size_t)nb * NP;
+    FR_CUDA(cudaFuncSetAttribute(mlp_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmem));
+    mlp_step_kernel<<<nb, kStepThreads, kStepSmem, s>>>(static_cast<const __nv_bfloat16 *>(d_params), d_x, d_t, d_w,
+                                                        (long long)n, partials, loss_part);
+    FR_CHECK_LAUNCH("mlp_step_kernel");
+    mlp_reduce_kernel<<<(NP + 31) / 32 + 1, 256, 0, s>>>(partials, nb, loss_part, 1.f / (float)n, d_grad, d_loss);
     FR_CHECK_LAUNCH("mlp_reduce_kernel");
     return FR_OK;
 }
