@@ -6,8 +6,10 @@
 //    for 3D radial), computed in double like the CPU restatement.
 //  * fr_degrid: interpolation of a multi-coil grid at the samples, the adjoint
 //    of gridding (same clamped cell range and exact LUT index as the scatter,
-//    GridLut.cpp:98-136).  One thread per sample and block of coils; the grid
-//    is read through L1/L2 (consecutive samples of a readout share cells).
+//    GridLut.cpp:98-136).  Tile by tile: a part of a tile's cells, all coils,
+//    in shared memory, a few lanes per sample.  Kernels wider than 5 cells and
+//    trajectories with few samples per tile: a thread per sample and block of
+//    coils, the grid read through L1/L2.
 //  * Pipe-Menon DCF (Pipe & Menon, MRM 41:179-186, 1999):
 //        w <- w / (C w),  C w = degrid(grid(w)),
 //    with grid(w) a real-valued tile scatter over the plan's bins, from its
@@ -112,6 +114,248 @@ __global__ void __launch_bounds__(256) degrid_kernel(DegridParams P)
 #pragma unroll
         for (int c = 0; c < CB; ++c)
             if (c0 + c < P.channels) P.out[(size_t)(c0 + c) * P.n + i] = acc[c];
+    }
+}
+
+// The cells of a footprint along one axis: clamped range (GridLut.cpp:98-106),
+// ends at distance kHW dropped where that is exact (they never pass dk < kHW).
+__device__ __forceinline__ void footprint(const DegridParams &P, int trim, float c, int &s, int &e)
+{
+    comp_range(c, P.hw, P.G, s, e);
+    if (trim && s <= e) {
+        if (!(fabsf(__fsub_rn((float)s, c)) < P.hw)) ++s;
+        if (s <= e && !(fabsf(__fsub_rn((float)e, c)) < P.hw)) --e;
+    }
+}
+
+// Degridding from shared memory.  A CTA takes one part (`box` cells) of one
+// work item's tile and one group of coils: it stages the cells that samples
+// starting in the part can reach as [cell][coil] (each value of the grid is
+// read from its plane once, not once per tap), collects the item's samples
+// that start there, and gives each sample LP lanes, two coils a lane.  Per
+// plane of a footprint the lanes share the R x R candidates' geometry, list the
+// taps inside the radius, and add weight x cell from the list, in the order of
+// degrid_kernel.
+// Cells are 4 * odd floats apart, so that staging (lanes along x) covers the
+// banks; LP = 8 lanes read one cell's 128 bytes at a time.
+// Bound: issue (geometry and list a quarter of it), barriers between scan, staging
+// and sums, the shared pipe (a cell row per tap), staging (a part's halo: a
+// 4 x 8 x 8 part of 12 coils reads 2.5 times its cells).  1.9 M samples, 12 coils,
+// 192^3 grid: 3034 us with a thread per sample and 4 coils gathering from the
+// planes through L1, 1166 us so (53 % issue, 51 % of the shared pipe).
+struct TileDegrid {
+    const unsigned long long *recs;
+    const WorkItem *items;
+    int tile[3], ntile[3];
+    int box[3], nbox[3];  // part of a tile, parts per tile
+    int trim;
+    int coils;            // coils per group (even)
+    int stride;           // floats per staged cell
+    const float *lutw;
+};
+constexpr int kDegridThreads = 512;
+constexpr int kDegridRound = 512;    // records looked at between two barriers
+__host__ __device__ constexpr int degrid_list(int R) { return ((R * R + 3) & ~3) + 2; }  // list entries per sample
+
+template <int LP, int R>
+__global__ void __launch_bounds__(kDegridThreads, 2) degrid_tiles_kernel(DegridParams P, TileDegrid T)
+{
+    constexpr int S = 32 / LP, NR = (R * R + LP - 1) / LP, LE = degrid_list(R);
+    extern __shared__ float4 smd[];
+    __shared__ int nq;
+    const int B[3] = {T.box[0] + R - 1, T.box[1] + R - 1, P.dim == 3 ? T.box[2] + R - 1 : 1};
+    float *blk = reinterpret_cast<float *>(smd);
+    int2 *lists = reinterpret_cast<int2 *>(blk + (size_t)B[0] * B[1] * B[2] * T.stride);
+    float *thr = reinterpret_cast<float *>(lists + (kDegridThreads / LP) * LE);
+    float *lut = thr + P.L;
+    // {sample, its footprint: first cell in the part, 5 bits an axis, cells, 3 bits}
+    uint2 *queue = reinterpret_cast<uint2 *>(lut + P.L + (P.L & 1));
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+
+    const WorkItem it = T.items[blockIdx.x];
+    const int c0 = blockIdx.z * T.coils, nc = min(T.coils, P.channels - c0);
+    int o[3], hi[3];  // first cell of the part, first past it
+    {
+        const int ty = it.tile / T.ntile[0], tz = ty / T.ntile[1];
+        const int t3[3] = {it.tile - ty * T.ntile[0], ty - tz * T.ntile[1], tz};
+        int b = blockIdx.y;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int k = b % T.nbox[d];
+            b /= T.nbox[d];
+            o[d] = t3[d] * T.tile[d] + k * T.box[d];
+            hi[d] = min(o[d] + T.box[d], (t3[d] + 1) * T.tile[d]);
+        }
+    }
+    const int G = P.G, Gz = P.dim == 3 ? P.G : 1;
+    bool staged = false;
+    const unsigned long long *recs = T.recs + it.begin;
+    for (int base = 0; base < it.count; base += kDegridRound) {
+        if (tid == 0) nq = 0;
+        __syncthreads();
+        const int n = min(it.count - base, kDegridRound);
+        for (int j = warp * 32; j < n; j += kDegridThreads) {
+            bool home = false;
+            unsigned sidx = 0u, fp = 0u;
+            if (j + lane < n) {
+                sidx = (unsigned)recs[base + j + lane];
+                const float4 p = P.traj[sidx];
+                const float c[3] = {p.x, p.y, p.z};
+                int st[3] = {0, 0, 0}, e[3] = {0, 0, 0};
+                bool some = true;
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    if (d < P.dim) {
+                        footprint(P, T.trim, c[d], st[d], e[d]);
+                        some = some && st[d] <= e[d];
+                    }
+                if (!some) {  // no taps: its untrimmed start is still in exactly one tile
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+                        if (d < P.dim) {
+                            comp_range(c[d], P.hw, P.G, st[d], e[d]);
+                            e[d] = st[d] - 1;
+                        }
+                }
+                home = true;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    home = home && st[d] >= o[d] && st[d] < hi[d];
+                    fp |= (unsigned)(st[d] - o[d]) << (6 * d) | (unsigned)(e[d] - st[d] + 1) << (18 + 3 * d);
+                }
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, home);
+            int at = 0;
+            if (lane == 0 && m) at = atomicAdd(&nq, __popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (home) queue[at + __popc(m & ((1u << lane) - 1u))] = make_uint2(sidx, fp);
+        }
+        __syncthreads();
+        const int count = nq;
+        if (count > 0 && !staged) {
+            staged = true;
+            for (int i = tid; i < P.L; i += kDegridThreads) {
+                thr[i] = P.lut_e[i].x;
+                lut[i] = T.lutw[i];
+            }
+            // a row of the block per 16 lanes, coil after coil; the copies are
+            // asynchronous (all of a thread's are in flight at once)
+            for (int r = tid >> 4; r < B[1] * B[2]; r += kDegridThreads / 16) {
+                const int lz = r / B[1], ly = r - lz * B[1];
+                const bool row = o[1] + ly < G && o[2] + lz < Gz;
+                for (int lx = tid & 15; lx < B[0]; lx += 16) {
+                    const bool in = row && o[0] + lx < G;
+                    const float2 *src = P.grid + (size_t)c0 * P.cells +
+                                        (in ? ((size_t)(o[2] + lz) * G + (o[1] + ly)) * (size_t)G + (o[0] + lx) : 0);
+                    float *dst = blk + (size_t)(r * B[0] + lx) * T.stride;
+                    unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+                    for (int c = 0; c < T.coils; ++c, d += 8, src += P.cells) {
+                        // past the grid or the last coil: nothing is read, zeros are written
+                        const bool some = in && c < nc;
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d),
+                                     "l"(some ? src : P.grid), "r"(some ? 8 : 0)
+                                     : "memory");
+                    }
+                }
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+        }
+        const int l = lane % LP, g = lane / LP;
+        const bool mine = 2 * l < T.coils;  // this lane's coils c0 + 2 l, c0 + 2 l + 1
+        int2 *list = lists + (warp * S + g) * LE;
+        for (int q0 = warp * S; q0 < count; q0 += (kDegridThreads / 32) * S) {
+            const bool live = q0 + g < count;
+            const uint2 qe = queue[live ? q0 + g : q0];
+            const unsigned sidx = qe.x, fp = qe.y;
+            const float4 p = P.traj[sidx];
+            const int bx = fp & 63, by = (fp >> 6) & 63, bz = (fp >> 12) & 63;
+            const int nx = (fp >> 18) & 7, ny = (fp >> 21) & 7, nz = (fp >> 24) & 7;
+            // the lane's candidates of a plane: l, l + LP, ... (x fastest)
+            float dx2[NR], dy2[NR];
+            int off[NR];
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                const int k = l + LP * r, iy = k / R, ix = k - iy * R;
+                const float dx = __fsub_rn((float)(o[0] + bx + ix), p.x), dy = __fsub_rn((float)(o[1] + by + iy), p.y);
+                dx2[r] = ix < nx && iy < ny ? __fmul_rn(dx, dx) : __int_as_float(0x7f800000);
+                dy2[r] = __fmul_rn(dy, dy);
+                // byte offset in a plane of the block, parity of x + y above
+                off[r] = ((by + iy) * B[0] + bx + ix) * T.stride * 4 +
+                         (P.checkerboard ? (o[0] + bx + ix + o[1] + by + iy) & 1 : 0);
+            }
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+            for (int iz = 0; iz < (P.dim == 3 ? R : 1); ++iz) {
+                const int z = o[2] + bz + iz;
+                const float dz = P.dim == 3 ? __fsub_rn((float)z, p.z) : 0.f;
+                const float dz2 = iz < nz ? __fmul_rn(dz, dz) : __int_as_float(0x7f800000);
+                const int plane = (bz + iz) * B[0] * B[1] * T.stride * 4;
+                const int zodd = P.checkerboard ? z & 1 : 0;
+                int nt = 0;
+#pragma unroll
+                for (int r = 0; r < NR; ++r) {
+                    const float s2 = __fadd_rn(__fadd_rn(dz2, dy2[r]), dx2[r]);
+                    const bool ok = live && s2 < P.smax;
+                    const unsigned m = (__ballot_sync(0xffffffffu, ok) >> (g * LP)) & ((1u << LP) - 1u);
+                    if (ok) {
+                        float a;
+                        asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(s2));
+                        const int k0 = min((int)fmaf(a, P.kc, 0.25f), P.L - 1);
+                        const float wt = lut[k0 + (s2 >= thr[k0] ? 1 : 0)];  // thr[L - 1] is +inf
+                        list[nt + __popc(m & ((1u << l) - 1u))] =
+                            make_int2((off[r] & ~1) + plane, __float_as_int((off[r] ^ zodd) & 1 ? -wt : wt));
+                    }
+                    nt += __popc(m);
+                }
+                __syncwarp();
+                if (mine) {
+                    const char *cell = reinterpret_cast<const char *>(blk + 4 * l);
+                    auto add = [&](int at, float w) {
+                        const float4 v = *reinterpret_cast<const float4 *>(cell + at);
+                        acc.x = fmaf(w, v.x, acc.x);
+                        acc.y = fmaf(w, v.y, acc.y);
+                        acc.z = fmaf(w, v.z, acc.z);
+                        acc.w = fmaf(w, v.w, acc.w);
+                    };
+                    int k = 0;
+#pragma unroll 2
+                    for (; k + 2 <= nt; k += 2) {
+                        const int4 e = *reinterpret_cast<const int4 *>(list + k);
+                        add(e.x, __int_as_float(e.y));
+                        add(e.z, __int_as_float(e.w));
+                    }
+                    if (k < nt) add(list[k].x, __int_as_float(list[k].y));
+                }
+                __syncwarp();
+            }
+            if (live && 2 * l < nc) {
+                float2 *out = P.out + (size_t)(c0 + 2 * l) * P.n + sidx;
+                *out = make_float2(acc.x, acc.y);
+                if (2 * l + 1 < nc) out[P.n] = make_float2(acc.z, acc.w);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Samples without a cell in reach have no bin record: their values are zero.
+__global__ void __launch_bounds__(256) degrid_outside_kernel(DegridParams P)
+{
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < P.n;
+         i += (long long)gridDim.x * blockDim.x) {
+        const float4 p = P.traj[i];
+        int s, e;
+        comp_range(p.x, P.hw, P.G, s, e);
+        bool out = s > e;
+        comp_range(p.y, P.hw, P.G, s, e);
+        out = out || s > e;
+        if (P.dim == 3) {
+            comp_range(p.z, P.hw, P.G, s, e);
+            out = out || s > e;
+        }
+        if (out)
+            for (int c = 0; c < P.channels; ++c) P.out[(size_t)c * P.n + i] = make_float2(0.f, 0.f);
     }
 }
 
@@ -402,17 +646,6 @@ __global__ void reduce_real_splits_kernel(RealGridParams P)
     }
 }
 
-// The cells of a footprint along one axis: clamped range (GridLut.cpp:98-106),
-// ends at distance kHW dropped where that is exact (they never pass dk < kHW).
-__device__ __forceinline__ void footprint(const DegridParams &P, int trim, float c, int &s, int &e)
-{
-    comp_range(c, P.hw, P.G, s, e);
-    if (trim && s <= e) {
-        if (!(fabsf(__fsub_rn((float)s, c)) < P.hw)) ++s;
-        if (s <= e && !(fabsf(__fsub_rn((float)e, c)) < P.hw)) --e;
-    }
-}
-
 // Degrid a real grid at each sample and divide the sample's weight by it.
 // XR >= 2 hw bounds the cells along x, whose dx^2 are computed once (+inf past
 // the footprint); thresholds and weights are read as single words.
@@ -503,6 +736,116 @@ DegridParams degrid_params(fr_plan p)
     return P;
 }
 
+// Most cells of a footprint along an axis: an open interval of length 2 hw
+// holds at most ceil(2 hw); without the exact trim floor(2 hw) + 1, where the
+// rounding of c - hw and c + hw (below 2^-11 for grids up to 4096) can add one
+// if 2 hw is just below an integer.
+int footprint_reach(fr_plan p)
+{
+    return p->prefilter ? (int)std::ceil(2.0 * p->hw) : (int)std::floor(2.0 * p->hw + 1e-3) + 1;
+}
+
+template <int LP, int R>
+int launch_degrid_tiles(const DegridParams &P, const TileDegrid &T, dim3 grid, size_t smem, cudaStream_t s)
+{
+    auto kern = degrid_tiles_kernel<LP, R>;
+    FR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<grid, kDegridThreads, smem, s>>>(P, T);
+    FR_CHECK_LAUNCH("degrid_tiles_kernel");
+    return FR_OK;
+}
+
+// The tiled degridding; -1 where a thread per sample is the better form.  The
+// lines are where the two crossed over 1 to 30 coils, 1 k to 5 M samples, widths 3
+// to 5 (times: thread per sample / tiled, us):
+//  * 3D: from 4 coils (a sample's lanes share its geometry over two coils each: 1
+//    coil 240 / 347), with under 8 from 4 M values (4 coils, 192 k samples 78 / 85,
+//    2.6 M 2666 / 1460), else from 1 M (16 coils, 19 k samples 35 / 47, 64 k 133 /
+//    78: too few CTAs below).  Staging a part is paid by its samples: from 100 per
+//    work item (12 coils, 180^3: 67 a tile 589 / 636, 160 a tile 2021 / 880), from
+//    40 when 4 coils of the grid are past the L2 cache, whose hits the other form
+//    lives on (12 coils, 300^3: 32 a tile 2874 / 2335, 48 a tile 4362 / 2501).
+//  * the other widths need more: 3 (fewer taps per staged cell) a grid that is not
+//    cached, 6 coils and 150 a tile (12 coils, 144^3 278 / 378; 210^3 1787 /
+//    1176), 5 a grid past the cache (16 coils, 144^3 1516 / 1601, 210^3 at 20
+//    coils 11164 / 5792); a cached grid 6 coils in groups that fill three
+//    quarters of their lanes (17 coils, width 5: 1628 / 1757).
+//  * 2D (always cached): from 12 coils (8 coils 56 / 58, 16 coils 97 / 67), 100 k
+//    samples (20 coils, 75 k 25 / 44) and 32 k cells (a 90^2 grid sits in L1: 54 /
+//    60), width over 3 (53 / 57).
+//  * never footprints over 5 cells (the lists), over 1024 table entries, or a
+//    tile that leaves no part of at most kDegridBlock bytes.
+constexpr size_t kDegridBlock = 96 * 1024;  // two CTAs per SM
+bool tiled_degrid_pays(fr_plan p, int R, long long cells, int channels, int pairs, int LP)
+{
+    const long long n = (long long)p->n, values = n * channels;
+    const long long each = n / std::max<long long>(p->nitems_occupied, 1);  // samples per work item
+    const bool full = 4 * pairs >= 3 * LP;
+    if (R > 5 || p->L > 1024 || values < 1ll << 20) return false;
+    if (p->dim == 2) return channels >= 12 && n >= 100000 && cells >= 1 << 15 && R >= 4 && full && each >= 100;
+    const long long four = cells * 32;  // bytes of 4 coils of the grid
+    const bool cached = four < 100ll << 20, past = four > 190ll << 20;
+    if (channels < 4 || (channels < 8 && values < 1ll << 22)) return false;
+    if (R <= 3) return !cached && channels >= 6 && each >= 150;
+    if (R == 5) return past && each >= 100;
+    return past ? each >= 40 : each >= 100 && (!cached || (channels >= 6 && full));
+}
+
+int degrid_tiles(fr_plan p, const DegridParams &P, cudaStream_t s)
+{
+    if (p->nitems_occupied == 0) return -1;
+    const int R = footprint_reach(p);
+    TileDegrid T;
+    T.recs = p->pairs.as<unsigned long long>();
+    T.items = p->items.as<WorkItem>();
+    T.trim = p->prefilter;
+    T.lutw = p->lut_d.as<float>();
+    // groups of at most 16 coils, even, of near equal size
+    const int groups = (P.channels + 15) / 16;
+    T.coils = ((P.channels + groups - 1) / groups + 1) & ~1;
+    const int pairs = T.coils / 2, LP = pairs <= 2 ? 2 : pairs <= 4 ? 4 : 8;
+    if (!tiled_degrid_pays(p, R, P.cells, P.channels, pairs, LP)) return -1;
+    T.stride = 4 * (pairs | 1);
+    const int RR = R <= 4 ? 4 : 5;
+    long long parts = 1;
+    for (int d = 0; d < 3; ++d) {
+        T.tile[d] = T.box[d] = p->tile[d];
+        T.ntile[d] = p->ntile[d];
+        T.nbox[d] = 1;
+    }
+    auto bytes = [&] {
+        size_t b = (size_t)T.stride * 4;
+        for (int d = 0; d < p->dim; ++d) b *= (size_t)(T.box[d] + RR - 1);
+        return b;
+    };
+    while (bytes() > kDegridBlock) {  // halve the longest axis, the outermost first
+        int d = p->dim - 1;
+        for (int k = p->dim - 2; k >= 0; --k)
+            if (T.box[k] > T.box[d]) d = k;
+        if (T.box[d] <= 2) return -1;
+        T.box[d] = (T.box[d] + 1) / 2;
+        T.nbox[d] = (T.tile[d] + T.box[d] - 1) / T.box[d];
+    }
+    for (int d = 0; d < 3; ++d) parts *= T.nbox[d];
+    if (parts > 65535 || groups > 65535) return -1;
+    const size_t smem = bytes() + (size_t)(kDegridThreads / LP) * degrid_list(RR) * 8 + (size_t)(P.L + 1) * 8 + kDegridRound * 8;
+    const dim3 grid((unsigned)p->nitems_occupied, (unsigned)parts, (unsigned)groups);
+    degrid_outside_kernel<<<(int)std::min<long long>((P.n + 255) / 256, (long long)sm_count() * 8), 256, 0, s>>>(P);
+    FR_CHECK_LAUNCH("degrid_outside_kernel");
+    if (RR == 4) {
+        switch (LP) {
+        case 2: return launch_degrid_tiles<2, 4>(P, T, grid, smem, s);
+        case 4: return launch_degrid_tiles<4, 4>(P, T, grid, smem, s);
+        default: return launch_degrid_tiles<8, 4>(P, T, grid, smem, s);
+        }
+    }
+    switch (LP) {
+    case 2: return launch_degrid_tiles<2, 5>(P, T, grid, smem, s);
+    case 4: return launch_degrid_tiles<4, 5>(P, T, grid, smem, s);
+    default: return launch_degrid_tiles<8, 5>(P, T, grid, smem, s);
+    }
+}
+
 }  // namespace
 
 int dcf_analytic_run(const float *d_traj, size_t n, int dim, float power, float *d_out, cudaStream_t s)
@@ -525,6 +868,8 @@ int degrid_run(fr_plan p, const float *d_grid, int channels, float *d_out, cudaS
     P.grid = reinterpret_cast<const float2 *>(d_grid);
     P.channels = channels;
     P.out = reinterpret_cast<float2 *>(d_out);
+    const int tiled = degrid_tiles(p, P, s);
+    if (tiled >= 0) return tiled;
     constexpr int CB = 4;
     const size_t smem = (size_t)P.L * 16;
     if (smem > 48 * 1024)
@@ -628,11 +973,7 @@ int dcf_pipe_run(fr_plan p, int iterations, float *d_w, cudaStream_t s)
     if (p->real_grid.reserve(cells * 4)) return FR_ERR_CUDA;
     DegridParams P = degrid_params(p);
     const size_t smem = (size_t)P.L * 8;
-    // most cells along an axis: an open interval of length 2 hw holds at most
-    // ceil(2 hw); without the exact trim floor(2 hw) + 1, where the rounding of
-    // c - hw and c + hw (below 2^-11) can add one if 2 hw is just below an integer
-    const int trim = p->prefilter;
-    const int reach = trim ? (int)std::ceil(2.0 * p->hw) : (int)std::floor(2.0 * p->hw + 1e-3) + 1;
+    const int trim = p->prefilter, reach = footprint_reach(p);
     auto kern = reach <= 4 ? pipe_update_kernel<4> : reach <= 5 ? pipe_update_kernel<5>
                 : reach <= 9 ? pipe_update_kernel<9> : pipe_update_kernel<14>;  // widths up to 13
     if (smem > 48 * 1024)
