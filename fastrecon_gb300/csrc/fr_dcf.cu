@@ -361,66 +361,77 @@ __global__ void __launch_bounds__(256) degrid_outside_kernel(DegridParams P)
 
 // -- streaming acquisition: incremental regridding -----------------------------
 // The gridded change dcf * (new - old) of the samples [begin, begin + count)
-// added into the grid with global atomic adds: thread per (sample, block of
-// CB coils), the same cell range, LUT index and checkerboard signs as the
-// scatter and the degridding.
+// added into the grid with global atomic adds, and the new values put in the
+// old ones' place: a warp per sample, the same cell range, LUT index and
+// checkerboard signs as the scatter and the degridding.  A lane per cell of the
+// footprint (x fastest: 4 lanes of a row share its sectors), so that the
+// weights are computed once for all coils; a lane per coil for the values,
+// which the warp broadcasts coil by coil; (re, im) in one 8-byte reduction.
+// Bound: the L2's reductions.  12,288 samples, 16 coils, 192^3 grid: 93 us with a
+// thread per sample and 4 coils (192 CTAs, scalar adds, and a copy after it),
+// 31 us so (with the copy 104 -> 33).
 struct UpdateParams {
     DegridParams g;          // geometry, LUT, grid size, checkerboard flag
-    const float2 *old_k;     // channels x n: the k-space the grid was made from
+    float2 *old_k;           // channels x n: the k-space the grid was made from, updated
     const float2 *new_k;     // channels x count: the new values
     const float *dcf;        // n
     float2 *grid;            // channels x cells
     long long begin, count;
 };
+constexpr int kUpdateWarps = 8;
 
-template <int CB>
-__global__ void __launch_bounds__(256) grid_update_kernel(UpdateParams U)
+__device__ __forceinline__ void red_add2(float2 *p, float x, float y)
+{
+    asm volatile("red.relaxed.gpu.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(x), "f"(y) : "memory");
+}
+
+__global__ void __launch_bounds__(kUpdateWarps * 32) grid_update_kernel(UpdateParams U)
 {
     extern __shared__ float4 lutS[];
     const DegridParams &P = U.g;
     for (int i = threadIdx.x; i < P.L; i += blockDim.x) lutS[i] = P.lut_e[i];
     __syncthreads();
-    const int c0 = blockIdx.y * CB;
     const size_t G = (size_t)P.G;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < U.count;
-         i += (long long)gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    for (long long i = blockIdx.x * (long long)kUpdateWarps + (threadIdx.x >> 5); i < U.count;
+         i += (long long)gridDim.x * kUpdateWarps) {
         const long long sidx = U.begin + i;
         const float4 p = P.traj[sidx];
         const float d = U.dcf[sidx];
-        float2 v[CB];
-#pragma unroll
-        for (int c = 0; c < CB; ++c) {
-            v[c] = make_float2(0.f, 0.f);
-            if (c0 + c < P.channels) {
-                const float2 a = U.new_k[(size_t)(c0 + c) * U.count + i];
-                const float2 b = U.old_k[(size_t)(c0 + c) * P.n + sidx];
-                v[c] = make_float2(__fmul_rn(d, __fsub_rn(a.x, b.x)), __fmul_rn(d, __fsub_rn(a.y, b.y)));
-            }
-        }
         int xs, xe, ys, ye, zs = 0, ze = 0;
         comp_range(p.x, P.hw, P.G, xs, xe);
         comp_range(p.y, P.hw, P.G, ys, ye);
         if (P.dim == 3) comp_range(p.z, P.hw, P.G, zs, ze);
-        for (int z = zs; z <= ze; ++z) {
-            const float dz = P.dim == 3 ? __fsub_rn((float)z, p.z) : 0.f;
-            const float dz2 = __fmul_rn(dz, dz);
-            for (int y = ys; y <= ye; ++y) {
-                const float dy = __fsub_rn((float)y, p.y);
-                const float dzy = __fadd_rn(dz2, __fmul_rn(dy, dy));
-                const size_t row = ((size_t)z * G + (size_t)y) * G;
-                for (int x = xs; x <= xe; ++x) {
-                    const float dx = __fsub_rn((float)x, p.x);
-                    float w;
-                    if (!lut_weight(__fadd_rn(dzy, __fmul_rn(dx, dx)), lutS, P.smax, P.kc, P.L, w)) continue;
+        const int nx = max(xe - xs + 1, 0), ny = max(ye - ys + 1, 0), nz = max(ze - zs + 1, 0);
+        const int ncell = nx * ny * nz;
+        for (int c0 = 0; c0 < P.channels; c0 += 32) {
+            float2 v = make_float2(0.f, 0.f);
+            if (c0 + lane < P.channels) {
+                const float2 a = U.new_k[(size_t)(c0 + lane) * U.count + i];
+                float2 *o = U.old_k + (size_t)(c0 + lane) * P.n + sidx;
+                const float2 b = *o;
+                v = make_float2(__fmul_rn(d, __fsub_rn(a.x, b.x)), __fmul_rn(d, __fsub_rn(a.y, b.y)));
+                *o = a;
+            }
+            const int nc = min(32, P.channels - c0);
+            for (int k0 = 0; k0 < ncell; k0 += 32) {
+                const int k = k0 + lane;
+                bool ok = k < ncell;
+                float w = 0.f;
+                float2 *cell = U.grid;
+                if (ok) {
+                    const int r = k / nx, ix = k - r * nx, iz = r / ny, iy = r - iz * ny;
+                    const int x = xs + ix, y = ys + iy, z = zs + iz;
+                    const float dx = __fsub_rn((float)x, p.x), dy = __fsub_rn((float)y, p.y);
+                    const float dz = P.dim == 3 ? __fsub_rn((float)z, p.z) : 0.f;
+                    const float dzy = __fadd_rn(__fmul_rn(dz, dz), __fmul_rn(dy, dy));
+                    ok = lut_weight(__fadd_rn(dzy, __fmul_rn(dx, dx)), lutS, P.smax, P.kc, P.L, w);
                     if (P.checkerboard && ((x + y + z) & 1)) w = -w;
-#pragma unroll
-                    for (int c = 0; c < CB; ++c) {
-                        if (c0 + c < P.channels) {
-                            float *g = reinterpret_cast<float *>(U.grid + (size_t)(c0 + c) * P.cells + row + x);
-                            atomicAdd(g, __fmul_rn(w, v[c].x));
-                            atomicAdd(g + 1, __fmul_rn(w, v[c].y));
-                        }
-                    }
+                    cell += (size_t)c0 * P.cells + ((size_t)z * G + (size_t)y) * G + (size_t)x;
+                }
+                for (int c = 0; c < nc; ++c, cell += P.cells) {
+                    const float vx = __shfl_sync(0xffffffffu, v.x, c), vy = __shfl_sync(0xffffffffu, v.y, c);
+                    if (ok) red_add2(cell, __fmul_rn(w, vx), __fmul_rn(w, vy));
                 }
             }
         }
@@ -891,23 +902,18 @@ int grid_update_run(fr_plan p, float *d_kdata, const float *d_new, size_t begin,
     UpdateParams U;
     U.g = degrid_params(p);
     U.g.channels = channels;
-    U.old_k = reinterpret_cast<const float2 *>(d_kdata);
+    U.old_k = reinterpret_cast<float2 *>(d_kdata);
     U.new_k = reinterpret_cast<const float2 *>(d_new);
     U.dcf = d_dcf;
     U.grid = reinterpret_cast<float2 *>(d_grid);
     U.begin = (long long)begin;
     U.count = (long long)count;
-    constexpr int CB = 4;
     const size_t smem = (size_t)U.g.L * 16;
     if (smem > 48 * 1024)
-        FR_CUDA(cudaFuncSetAttribute(grid_update_kernel<CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int bx = (int)std::min<long long>(((long long)count + 255) / 256, (long long)sm_count() * 8);
-    dim3 grid(bx, (channels + CB - 1) / CB);
-    grid_update_kernel<CB><<<grid, 256, smem, s>>>(U);
+        FR_CUDA(cudaFuncSetAttribute(grid_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int bx = (int)std::min<long long>(((long long)count + kUpdateWarps - 1) / kUpdateWarps, (long long)sm_count() * 32);
+    grid_update_kernel<<<bx, kUpdateWarps * 32, smem, s>>>(U);
     FR_CHECK_LAUNCH("grid_update_kernel");
-    // then the k-space itself: row c of the new values into coil c at `begin`
-    FR_CUDA(cudaMemcpy2DAsync(d_kdata + 2 * begin, p->n * 8, d_new, count * 8, count * 8, (size_t)channels,
-                              cudaMemcpyDeviceToDevice, s));
     return FR_OK;
 }
 
