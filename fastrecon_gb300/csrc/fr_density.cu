@@ -30,14 +30,44 @@ __device__ __forceinline__ int nearest_cell(float x, int G)
     return min(max(c, 0), G - 1);
 }
 
-__global__ void cell_hist_kernel(const float4 *__restrict__ traj, long long n, int dim, int G, int *hist)
+// Samples per cell.  Every readout crosses the k-space centre, so a few cells
+// take one sample of each: counted straight into global memory their atomics
+// queue up (20,000 spokes: 110 us, most of it that queue).  A CTA first counts
+// in a table of its own (a slot belongs to the first cell that maps to it; the
+// cells every readout shares are there from the first readouts on), and adds
+// the slots to the grid at the end; cells without a slot go straight there.
+// 5.1 M samples on a 320^3 grid: 49 us.
+constexpr int kHistThreads = 1024, kHistSlots = 4096;
+
+__global__ void __launch_bounds__(kHistThreads) cell_hist_kernel(const float4 *__restrict__ traj, long long n, int dim,
+                                                                 int G, int *hist)
 {
+    __shared__ int key[kHistSlots], count[kHistSlots];
+    for (int i = threadIdx.x; i < kHistSlots; i += kHistThreads) {
+        key[i] = -1;
+        count[i] = 0;
+    }
+    __syncthreads();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float4 p = traj[i];
         const int x = nearest_cell(p.x, G), y = nearest_cell(p.y, G), z = dim == 3 ? nearest_cell(p.z, G) : 0;
-        atomicAdd(&hist[((size_t)z * G + y) * G + x], 1);
+        const int cell = (z * G + y) * G + x;  // fewer than 2^31 cells
+        const unsigned slot = ((unsigned)cell * 2654435761u) >> 20;
+        int k = key[slot];
+        if (k == -1) {
+            k = atomicCAS(&key[slot], -1, cell);
+            if (k == -1) k = cell;
+        }
+        if (k == cell)
+            atomicAdd(&count[slot], 1);
+        else
+            atomicAdd(&hist[cell], 1);
     }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kHistSlots; i += kHistThreads)
+        if (count[i]) atomicAdd(&hist[key[i]], count[i]);
 }
+static_assert(kHistSlots == 1 << 12, "the slot is the hash's top 12 bits");
 
 // Inclusive scan along x: one warp per row.
 __global__ void scan_x_kernel(int *a, long long rows, int G)
@@ -62,8 +92,50 @@ __global__ void scan_x_kernel(int *a, long long rows, int G)
     }
 }
 
+// Inclusive scan along x and y of the planes of a 3D grid in one pass, a CTA
+// per plane: thread = x (G <= 1024), the warps' totals through shared memory,
+// kRows rows at a time, the next kRows' loads in flight, the column sums in a
+// register.  Bound: HBM.  320^3: 197 us as a scan along x and one along y, 78
+// us so.  (2D has one plane, and takes the two.)
+constexpr int kRows = 8;
+__global__ void scan_xy_kernel(int *a, int G)
+{
+    __shared__ int tot[2][kRows][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, x = threadIdx.x;
+    int *plane = a + (size_t)blockIdx.x * G * G;
+    int col = 0, buf = 0, next[kRows];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) next[r] = x < G && r < G ? plane[(size_t)r * G + x] : 0;
+    for (int y0 = 0; y0 < G; y0 += kRows, buf ^= 1) {
+        int v[kRows];
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            v[r] = next[r];
+            const int y = y0 + kRows + r;
+            next[r] = x < G && y < G ? plane[(size_t)y * G + x] : 0;
+        }
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, v[r], d);
+                if (lane >= d) v[r] += u;
+            }
+            if (lane == 31) tot[buf][r][warp] = v[r];
+        }
+        __syncthreads();  // the other buffer is written only after the next one
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            col += v[r] + __reduce_add_sync(0xffffffffu, lane < min(warp, nw) ? tot[buf][r][lane] : 0);
+            if (x < G && y0 + r < G) plane[(size_t)(y0 + r) * G + x] = col;
+        }
+    }
+}
+
 // Inclusive scan along an outer axis: thread per column, sequential along
-// the axis (stride `step` elements), consecutive threads on consecutive x.
+// the axis (stride `step` elements), consecutive threads on consecutive x,
+// kAhead loads in flight.  320^3 along z: 149 us with one in flight, 51 us so.
+constexpr int kAhead = 8;
 __global__ void scan_outer_kernel(int *a, long long columns, int len, long long step, long long plane)
 {
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < columns;
@@ -71,9 +143,15 @@ __global__ void scan_outer_kernel(int *a, long long columns, int len, long long 
         // column c: x = c % step within a plane block, block = c / step
         int *p = a + (c / step) * plane + (c % step);
         int acc = 0;
-        for (int k = 0; k < len; ++k) {
-            acc += p[(size_t)k * step];
-            p[(size_t)k * step] = acc;
+        for (int k0 = 0; k0 < len; k0 += kAhead) {
+            int v[kAhead];
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) v[k] = k0 + k < len ? p[(size_t)(k0 + k) * step] : 0;
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+                acc += v[k];
+                if (k0 + k < len) p[(size_t)(k0 + k) * step] = acc;
+            }
         }
     }
 }
@@ -120,8 +198,14 @@ __global__ void kmax_kernel(const float4 *__restrict__ traj, long long n, int di
         if (dim >= 3) q = __fadd_rn(q, __fmul_rn(p.z, p.z));
         m = fmaxf(m, __fsqrt_rn(q));
     }
-    for (int d = 16; d; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
+    __shared__ unsigned part[32];
+    const unsigned w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));  // m >= 0
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = w;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const unsigned b = __reduce_max_sync(0xffffffffu, threadIdx.x < blockDim.x / 32 ? part[threadIdx.x] : 0u);
+        if (threadIdx.x == 0) atomicMax(out, b);
+    }
 }
 
 __global__ void features_kernel(const int *__restrict__ counts, const float4 *__restrict__ traj, long long n, int dim,
@@ -149,6 +233,14 @@ int blocks_for(long long n, int threads)
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     return (int)std::max<long long>(1, std::min<long long>((n + threads - 1) / threads, (long long)sms * 16));
+}
+
+int sm_count_density()
+{
+    int dev = 0, sms = 132;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
 }
 
 int make_radii(const int *radii, int nradii, Radii *R)
@@ -179,18 +271,22 @@ int density_counts_run(fr_plan p, const int *radii, int nradii, int *d_counts, c
     FR_CUDA(cudaMemsetAsync(sat, 0, cells * 4, s));
     const long long n = (long long)p->n;
     const float4 *traj = p->traj.as<float4>();
-    cell_hist_kernel<<<blocks_for(n, 256), 256, 0, s>>>(traj, n, p->dim, G, sat);
+    cell_hist_kernel<<<(int)std::min<long long>((n + kHistThreads - 1) / kHistThreads, sm_count_density()), kHistThreads, 0,
+                       s>>>(traj, n, p->dim, G, sat);
     FR_CHECK_LAUNCH("cell_hist_kernel");
-    const long long rows = (long long)(cells / G);
-    scan_x_kernel<<<blocks_for(rows * 32, 256), 256, 0, s>>>(sat, rows, G);
-    FR_CHECK_LAUNCH("scan_x_kernel");
-    // y: columns (z, x), stride G, planes of G*G
-    const long long gz = p->dim == 3 ? G : 1;
-    scan_outer_kernel<<<blocks_for(gz * G, 256), 256, 0, s>>>(sat, gz * G, G, G, (long long)G * G);
-    FR_CHECK_LAUNCH("scan_outer_kernel");
+    if (p->dim == 3 && G <= 1024) {
+        scan_xy_kernel<<<G, (G + 31) & ~31, 0, s>>>(sat, G);
+        FR_CHECK_LAUNCH("scan_xy_kernel");
+    } else {
+        const long long rows = (long long)(cells / G), gz = p->dim == 3 ? G : 1;
+        scan_x_kernel<<<blocks_for(rows * 32, 256), 256, 0, s>>>(sat, rows, G);
+        FR_CHECK_LAUNCH("scan_x_kernel");
+        // y: columns (z, x), stride G, planes of G*G
+        scan_outer_kernel<<<blocks_for(gz * G, 128), 128, 0, s>>>(sat, gz * G, G, G, (long long)G * G);
+        FR_CHECK_LAUNCH("scan_outer_kernel");
+    }
     if (p->dim == 3) {  // z: columns (y, x), stride G*G
-        scan_outer_kernel<<<blocks_for((long long)G * G, 256), 256, 0, s>>>(sat, (long long)G * G, G,
-                                                                            (long long)G * G, 0);
+        scan_outer_kernel<<<blocks_for((long long)G * G, 128), 128, 0, s>>>(sat, (long long)G * G, G, (long long)G * G, 0);
         FR_CHECK_LAUNCH("scan_outer_kernel");
     }
     box_count_kernel<<<blocks_for(n, 256), 256, 0, s>>>(traj, n, p->dim, G, sat, R, d_counts);
@@ -209,7 +305,7 @@ int dcf_features_run(const int *d_counts, const float *d_raw, size_t n, int dim,
     const unsigned *kb = nullptr;
     if (!(kmax > 0.f)) {
         FR_CUDA(cudaMemsetAsync(d_scratch, 0, 4, s));
-        kmax_kernel<<<blocks_for((long long)n, 256), 256, 0, s>>>(traj, (long long)n, dim, d_scratch);
+        kmax_kernel<<<std::min(blocks_for((long long)n, 512), sm_count_density() * 4), 512, 0, s>>>(traj, (long long)n, dim, d_scratch);
         FR_CHECK_LAUNCH("kmax_kernel");
         kb = d_scratch;
     }

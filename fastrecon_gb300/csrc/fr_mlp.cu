@@ -111,16 +111,85 @@ __global__ void __launch_bounds__(kFwdThreads) mlp_forward_kernel(const __nv_bfl
     }
 }
 
+// Two floats in one 64-bit register and their packed arithmetic (one issue
+// slot for both).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float ex2_approx(float a)
+{
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+__device__ __forceinline__ float rcp_approx(float a)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+// tanh of two values, branch-free: x + x t Q(t), t = x^2, below 0.55 (Q of degree
+// 4, a least-maximum relative fit: 1e-9, in floats within 0.72 ulp), and
+// 1 - 2 / (e^2x + 1) above (absolute error about 1e-7, falling with x; the limits
+// +-1 and NaN come out by themselves).  About 9 issue slots a value.
+__device__ __forceinline__ f32x2 tanh2(f32x2 x)
+{
+    const f32x2 one = pack2(1.f, 1.f);
+    const f32x2 t = mul2(x, x);
+    f32x2 q = fma2(t, pack2(-0.0062742396f, -0.0062742396f), pack2(0.021071678f, 0.021071678f));
+    q = fma2(q, t, pack2(-0.05385231f, -0.05385231f));
+    q = fma2(q, t, pack2(0.13332586f, 0.13332586f));
+    q = fma2(q, t, pack2(-0.33333316f, -0.33333316f));
+    const float2 p = unpack2(fma2(mul2(q, t), x, x));
+    const float2 a = unpack2(mul2(x, pack2(2.885390081777927f, 2.885390081777927f)));  // 2 / ln 2
+    const float2 e = unpack2(add2(pack2(ex2_approx(a.x), ex2_approx(a.y)), one));
+    const float2 h = unpack2(fma2(pack2(rcp_approx(e.x), rcp_approx(e.y)), pack2(-2.f, -2.f), one));
+    const float2 v = unpack2(x);
+    return pack2(fabsf(v.x) < 0.55f ? p.x : h.x, fabsf(v.y) < 0.55f ? p.y : h.y);
+}
+
 // The forward pass with the hidden layer (64 x 64) on the tensor cores:
 // mma.sync m16n8k16, BF16 operands, FP32 accumulation.  One warp holds a
-// tile of 16 samples: each lane evaluates, in FP32 as forward_sample does,
-// exactly the first-layer activations its A fragments hold (2 samples x 16
-// units), splits each into three BF16 terms hi + mid + lo (the residual of
-// a BF16 rounding, twice: together within ~2^-24 of the FP32 value), and the
-// warp accumulates W2 h1 = W2 hi + W2 mid + W2 lo into FP32 fragments that
-// start from b2; the weights are BF16 already, so every product is exact
-// and the sums carry FP32 rounding only.  The output layer reduces each
-// lane's 16 units and the 4 lanes of a row with shuffles.
+// tile of 16 samples: each lane evaluates, in FP32, exactly the first-layer
+// activations its A fragments hold (2 samples x 16 units, units in pairs),
+// splits each into three BF16 terms hi + mid + lo (the residual of a BF16
+// rounding, twice: together within ~2^-24 of the FP32 value), and the warp
+// accumulates W2 h1 = W2 hi + W2 mid + W2 lo into FP32 fragments that start
+// from b2; the weights are BF16 already, so every product is exact and the
+// sums carry FP32 rounding only.  The output layer reduces each lane's 16
+// units and the 4 lanes of a row with shuffles.
+// Bound: the pipes of tanh (special functions 45 %, FMA 39 % of the time), the
+// tensor pipe (34 %) and issue (51 %).  5.1 M samples: 775 us with W2 rows of
+// 128 bytes (8-way bank conflicts, the shared pipe 83 % busy), tanhf, and
+// first-layer weights read as single BF16; 600 us so.
 __device__ __forceinline__ unsigned pack_bf16(float lo_half, float hi_half)
 {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo_half, hi_half);
@@ -137,101 +206,104 @@ __device__ __forceinline__ void mma_bf16_16816(float *d, const unsigned *a, unsi
 }
 
 constexpr int kMmaThreads = 128;  // 4 warps, 16 samples each per step
+constexpr int kW2Row = NH + 8;    // BF16 per shared row of W2: rows 4 banks apart
 
-__global__ void __launch_bounds__(kMmaThreads) mlp_forward_mma_kernel(const __nv_bfloat16 *__restrict__ pb,
-                                                                      const float *__restrict__ x, long long n,
-                                                                      int exp_out, int residual, float scale,
-                                                                      float *__restrict__ y)
+__global__ void __launch_bounds__(kMmaThreads, 4) mlp_forward_mma_kernel(const __nv_bfloat16 *__restrict__ pb,
+                                                                         const float *__restrict__ x, long long n,
+                                                                         int exp_out, int residual, float scale,
+                                                                         float *__restrict__ y)
 {
-    __shared__ __align__(16) __nv_bfloat16 pw[NP + 7];
-    for (int p = threadIdx.x; p < NP; p += blockDim.x) pw[p] = pb[p];
+    __shared__ __align__(16) float w1[NH / 2][NI + 1][2];  // unit pairs: weights per input, then biases
+    __shared__ __align__(16) __nv_bfloat16 w2s[NH * kW2Row];
+    __shared__ __align__(16) float b2s[NH], w3s[NH];
+    __shared__ float b3s;
+    for (int p = threadIdx.x; p < NP; p += blockDim.x) {
+        const float v = __bfloat162float(pb[p]);
+        if (p < OFF_B1) w1[(p / NI) >> 1][p % NI][(p / NI) & 1] = v;
+        else if (p < OFF_W2) w1[(p - OFF_B1) >> 1][NI][(p - OFF_B1) & 1] = v;
+        else if (p < OFF_B2) w2s[(p - OFF_W2) / NH * kW2Row + (p - OFF_W2) % NH] = pb[p];
+        else if (p < OFF_W3) b2s[p - OFF_B2] = v;
+        else if (p < OFF_B3) w3s[p - OFF_W3] = v;
+        else b3s = v;
+    }
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int g = lane >> 2, tig = lane & 3;
-    const unsigned *w2 = reinterpret_cast<const unsigned *>(pw + OFF_W2);  // bf16 pairs of W2[j][i], i fastest
+    const unsigned *w2 = reinterpret_cast<const unsigned *>(w2s) + g * (kW2Row / 2) + tig;  // BF16 pairs, input fastest
     const long long ntile = (n + 15) / 16;
     const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
     for (long long tile = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); tile < ntile;
          tile += warps) {
         const long long s0 = tile * 16 + g, s1 = s0 + 8;
-        float x0[NI], x1[NI];
+        f32x2 xb[2][NI];  // rows g and g + 8, each input in both halves
 #pragma unroll
         for (int k = 0; k < NI; ++k) {
-            x0[k] = s0 < n ? x[s0 * NI + k] : 0.f;
-            x1[k] = s1 < n ? x[s1 * NI + k] : 0.f;
+            const float a = s0 < n ? x[s0 * NI + k] : 0.f, b = s1 < n ? x[s1 * NI + k] : 0.f;
+            xb[0][k] = pack2(a, a);
+            xb[1][k] = pack2(b, b);
         }
         float acc[8][4];
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
-            const int j = 8 * nt + 2 * tig;
-            acc[nt][0] = acc[nt][2] = __bfloat162float(pw[OFF_B2 + j]);
-            acc[nt][1] = acc[nt][3] = __bfloat162float(pw[OFF_B2 + j + 1]);
+            const float2 b = *reinterpret_cast<const float2 *>(b2s + 8 * nt + 2 * tig);
+            acc[nt][0] = acc[nt][2] = b.x;
+            acc[nt][1] = acc[nt][3] = b.y;
         }
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
-            // this lane's first-layer units: i0 + {0, 1} and i0 + 8 + {0, 1}
-            const int i0 = 16 * ks + 2 * tig;
-            float h[2][4];  // [sample row g / g + 8][unit i0, i0 + 1, i0 + 8, i0 + 9]
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int i = i0 + (u & 1) + (u >> 1) * 8;
-                float a0 = __bfloat162float(pw[OFF_B1 + i]), a1 = a0;
-#pragma unroll
-                for (int k = 0; k < NI; ++k) {
-                    const float wk = __bfloat162float(pw[OFF_W1 + i * NI + k]);
-                    a0 = fmaf(wk, x0[k], a0);
-                    a1 = fmaf(wk, x1[k], a1);
-                }
-                h[0][u] = tanhf(a0);
-                h[1][u] = tanhf(a1);
-            }
-            // three BF16 terms per activation; A registers: a0a1 row g k lo,
-            // a2a3 row g+8 k lo, a4a5 row g k hi, a6a7 row g+8 k hi
+            // this lane's first-layer units 16 ks + 2 tig + {0, 1} and 8 further;
+            // A registers: row g k lo, row g + 8 k lo, row g k hi, row g + 8 k hi
             unsigned A[3][4];
 #pragma unroll
-            for (int r = 0; r < 2; ++r)
+            for (int q = 0; q < 2; ++q) {
+                const float4 *wp = reinterpret_cast<const float4 *>(&w1[8 * ks + 4 * q + tig][0][0]);
+                const float4 wa = wp[0], wb = wp[1], wc = wp[2];
+                const f32x2 w[NI] = {pack2(wa.x, wa.y), pack2(wa.z, wa.w), pack2(wb.x, wb.y), pack2(wb.z, wb.w),
+                                     pack2(wc.x, wc.y)};
 #pragma unroll
-                for (int qq = 0; qq < 2; ++qq) {
-                    const float v0 = h[r][2 * qq], v1 = h[r][2 * qq + 1];
-                    const float hi0 = __bfloat162float(__float2bfloat16_rn(v0));
-                    const float hi1 = __bfloat162float(__float2bfloat16_rn(v1));
-                    const float r0 = __fsub_rn(v0, hi0), r1 = __fsub_rn(v1, hi1);
-                    const float md0 = __bfloat162float(__float2bfloat16_rn(r0));
-                    const float md1 = __bfloat162float(__float2bfloat16_rn(r1));
-                    const int reg = r + 2 * qq;
-                    A[0][reg] = pack_bf16(hi0, hi1);
-                    A[1][reg] = pack_bf16(md0, md1);
-                    A[2][reg] = pack_bf16(__fsub_rn(r0, md0), __fsub_rn(r1, md1));
+                for (int r = 0; r < 2; ++r) {
+                    f32x2 a = pack2(wc.z, wc.w);
+#pragma unroll
+                    for (int k = 0; k < NI; ++k) a = fma2(w[k], xb[r][k], a);
+                    f32x2 h = tanh2(a);
+                    // three BF16 terms of the pair
+#pragma unroll
+                    for (int t = 0; t < 3; ++t) {
+                        const float2 v = unpack2(h);
+                        const unsigned u = pack_bf16(v.x, v.y);
+                        A[t][r + 2 * q] = u;
+                        if (t < 2)
+                            h = fma2(pack2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)),
+                                     pack2(-1.f, -1.f), h);
+                    }
                 }
+            }
 #pragma unroll
             for (int nt = 0; nt < 8; ++nt) {
-                const int j = 8 * nt + g;  // B column = output unit
-                const unsigned b0 = w2[(j * NH + i0) >> 1], b1 = w2[(j * NH + i0 + 8) >> 1];
+                // B column = output unit 8 nt + g
+                const unsigned b0 = w2[8 * nt * (kW2Row / 2) + 8 * ks], b1 = w2[8 * nt * (kW2Row / 2) + 8 * ks + 4];
                 mma_bf16_16816(acc[nt], A[2], b0, b1);
                 mma_bf16_16816(acc[nt], A[1], b0, b1);
                 mma_bf16_16816(acc[nt], A[0], b0, b1);
             }
         }
-        float o0 = 0.f, o1 = 0.f;
+        f32x2 p0 = pack2(0.f, 0.f), p1 = p0;
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
-            const int j = 8 * nt + 2 * tig;
-            const float w3a = __bfloat162float(pw[OFF_W3 + j]), w3b = __bfloat162float(pw[OFF_W3 + j + 1]);
-            o0 = fmaf(w3a, tanhf(acc[nt][0]), o0);
-            o0 = fmaf(w3b, tanhf(acc[nt][1]), o0);
-            o1 = fmaf(w3a, tanhf(acc[nt][2]), o1);
-            o1 = fmaf(w3b, tanhf(acc[nt][3]), o1);
+            const float2 w = *reinterpret_cast<const float2 *>(w3s + 8 * nt + 2 * tig);
+            p0 = fma2(pack2(w.x, w.y), tanh2(pack2(acc[nt][0], acc[nt][1])), p0);
+            p1 = fma2(pack2(w.x, w.y), tanh2(pack2(acc[nt][2], acc[nt][3])), p1);
         }
+        float o0 = unpack2(p0).x + unpack2(p0).y, o1 = unpack2(p1).x + unpack2(p1).y;
         o0 += __shfl_xor_sync(0xffffffffu, o0, 1);
         o0 += __shfl_xor_sync(0xffffffffu, o0, 2);
         o1 += __shfl_xor_sync(0xffffffffu, o1, 1);
         o1 += __shfl_xor_sync(0xffffffffu, o1, 2);
         if (tig == 0) {
-            const float b3 = __bfloat162float(pw[OFF_B3]);
-            float out0 = __fadd_rn(o0, b3), out1 = __fadd_rn(o1, b3);
+            float out0 = __fadd_rn(o0, b3s), out1 = __fadd_rn(o1, b3s);
             if (residual) {  // the network predicts log-DCF + log density (radius 2)
-                out0 = __fsub_rn(out0, x0[1]);
-                out1 = __fsub_rn(out1, x1[1]);
+                out0 = __fsub_rn(out0, unpack2(xb[0][1]).x);
+                out1 = __fsub_rn(out1, unpack2(xb[1][1]).x);
             }
             if (s0 < n) y[s0] = exp_out ? __fmul_rn(scale, expf(out0)) : out0;
             if (s1 < n) y[s1] = exp_out ? __fmul_rn(scale, expf(out1)) : out1;
@@ -553,7 +625,7 @@ int mlp_forward_run(const void *d_params, const float *d_x, size_t n, int exp_ou
     }
     const long long tiles = ((long long)n + 15) / 16;
     const int mblocks = (int)std::max<long long>(
-        1, std::min<long long>((tiles + kMmaThreads / 32 - 1) / (kMmaThreads / 32), (long long)sm_count_mlp() * 16));
+        1, std::min<long long>((tiles + kMmaThreads / 32 - 1) / (kMmaThreads / 32), (long long)sm_count_mlp() * 4));
     mlp_forward_mma_kernel<<<mblocks, kMmaThreads, 0, s>>>(static_cast<const __nv_bfloat16 *>(d_params), d_x,
                                                           (long long)n, exp_out, residual, scale, d_y);
     FR_CHECK_LAUNCH("mlp_forward_mma_kernel");
