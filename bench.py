@@ -143,11 +143,11 @@ def make_inputs(w, torch, device):
 
 def scatter_kernel(taps: bool, coils: int) -> str:
     """The scatter kernel the recon launches: with tap lists, the tap-lane
-    scatter for coil groups of 16 (9 coils and more) unless
-    FR_SCATTER_WARP_LISTS=1, the per-warp tap-list scatter otherwise."""
+    scatter (but for at most 4 coils in 3D) unless FR_SCATTER_WARP_LISTS=1, the
+    per-warp tap-list scatter otherwise."""
     if not taps:
         return "grid_tiles_kernel"
-    if coils > 8 and os.environ.get("FR_SCATTER_WARP_LISTS", "0") in ("", "0"):
+    if coils > 4 and os.environ.get("FR_SCATTER_WARP_LISTS", "0") in ("", "0"):
         return "grid_lanes_kernel"
     return "grid_taps_kernel"
 

@@ -860,31 +860,38 @@ __global__ void __launch_bounds__(512, 2) grid_taps_kernel(GridParams P)
 }
 
 // ---------------------------------------------------------------------------
-// Tap-lane scatter (rows of 32 coil floats, the tap lists of the plan): each
-// lane owns a group of kLaneTaps taps of one bin record and adds them for all
-// 32 coil floats of its coil group, so the taps' cell rows and weights stay
-// in the lane's registers and no per-record tap list goes through shared
-// memory.
+// Tap-lane scatter (the tap lists of the plan): each lane owns a group of
+// kLaneTaps taps of one bin record and adds them for all NF coil floats of
+// its coil group, so the taps' cell rows and weights stay in the lane's
+// registers and no per-record tap list goes through shared memory.
 //
 // A warp holds 32 of its records at a time (a window): their tap groups are
 // numbered by a warp scan and dealt to the lanes 32 per pass, so a pass packs
 // the groups of several records (a record's groups are consecutive).  Each
-// record's 32 coil values (dcf * k) are first copied into a 128-byte slot of
-// the warp's staging area by a bulk (TMA) copy, issued by the lane holding
+// record's coil values (dcf * k) are first copied into a 128-byte slot of
+// the warp's staging area by bulk (TMA) copies, issued by the lane holding
 // the record and completing on the warp's mbarrier; the item's fixed-point
 // scale goes on the weights.
 //
-// Bank-conflict-free adds: at step t lane j adds coil float t ^ j of each of
-// its taps.  The tile is [cell][32] int32 with 128-byte rows, so the 32
-// lanes of one red.shared hit the 32 banks once each, whatever their cells;
-// the lane reads the same float t ^ j of its record's slot (again one bank
-// per lane).  The adds are those of grid_taps_kernel (same fixed-point
-// values), so a tile held by one work item grids to the same bits.
+// Bank-conflict-free adds: at step t lane j adds coil float (t ^ j) mod NF of
+// each of its taps.  The tile is [cell][32] int32 with 128-byte rows, so the
+// 32 lanes of one red.shared hit the 32 banks once each, whatever their cells
+// are, at float t ^ j of the row; the lane reads the same float of its
+// record's slot (again one bank per lane).  With NF = 16 or 8 (at most 8 or 4
+// coils) a row holds 2 or 4 copies of the cell, one per 16 or 8 lanes, and a
+// slot as many copies of the values: NF adds a tap instead of 32, the banks
+// still hit once each; the flush adds the copies up (integers: the same sums).
+// The adds are those of grid_taps_kernel (same fixed-point values), so a tile
+// held by one work item grids to the same bits.
+// Bound: the L1/shared data pipe.  8 coils, 2.6 M samples on a 240^3 grid: NF = 32 (half
+// the adds of empty coils) 1156 us, the per-warp lists 1156 us, NF = 16 932 us.
 // ---------------------------------------------------------------------------
-constexpr int kLaneWarps = 8;   // 256 threads per CTA
 constexpr int kLaneBatch = 32;  // records per warp window (one per lane)
 constexpr int kLaneTaps = 4;    // taps of one record per lane (one read of its values serves them all)
 static_assert(kLaneTaps == 4, "a lane's taps are loaded as one 16-byte word from aligned runs");
+// Warps per CTA: 8, two CTAs per SM, for tiles of up to 512 cells (64 KB); 16,
+// one CTA, for larger ones (the 32 x 32 tiles of 2D).
+constexpr int kLaneWarpsSmall = 8, kLaneWarpsLarge = 16;
 
 // Shared-memory layout of grid_lanes_kernel from its 128-byte aligned base:
 // tile [K][32] int32 | weights [L] | per warp: value slots [32][32] floats,
@@ -893,14 +900,14 @@ static_assert(kLaneTaps == 4, "a lane's taps are loaded as one 16-byte word from
 struct LaneSmem {
     unsigned lutw, stage, table, mbar, end;
 };
-__host__ __device__ __forceinline__ LaneSmem lane_smem_layout(long long K, int L)
+__host__ __device__ __forceinline__ LaneSmem lane_smem_layout(long long K, int L, int warps)
 {
     LaneSmem m;
     m.lutw = (unsigned)(K * 32 * 4);
     m.stage = m.lutw + (unsigned)((L * 4 + 127) & ~127);
-    m.table = m.stage + (unsigned)(kLaneWarps * kLaneBatch * 128);
-    m.mbar = m.table + (unsigned)(kLaneWarps * kLaneBatch * 16);
-    m.end = m.mbar + (unsigned)(kLaneWarps * 8);
+    m.table = m.stage + (unsigned)(warps * kLaneBatch * 128);
+    m.mbar = m.table + (unsigned)(warps * kLaneBatch * 16);
+    m.end = m.mbar + (unsigned)(warps * 8);
     return m;
 }
 
@@ -948,13 +955,35 @@ __device__ __forceinline__ bool mbar_wait(unsigned mbar, unsigned parity)
     return false;
 }
 
-// Flush of a [cell][32] tile (rows not swizzled): lane = (coil cl = lane & 15,
-// pair px = lane >> 4), so that one 8-byte shared load per lane covers the 32
-// banks and lanes cl, cl + 16 write the two halves of one 32-byte sector of
-// coil plane cl.  Units (tile row, two x pairs) are dealt to the warps.
-__device__ __forceinline__ void lanes_flush(const GridParams &P, unsigned acc, int cg, int ox, int oy, int oz, float inv)
+// (re, im) of coil cl at cell i of a [cell][32] tile: the sum of the row's
+// copies, `first` the copy to start from (lanes on different rows of the same
+// coil start from different copies, in different banks).
+template <int NF>
+__device__ __forceinline__ int2 lanes_cell(unsigned acc, int i, int cl, int first)
 {
-    const int Tx = P.tile[0], Ty = P.tile[1], Tz = P.tile[2];
+    constexpr int NC = 32 / NF;
+    const unsigned row = acc + ((unsigned)i << 7) + ((unsigned)cl << 3);
+    int2 v = make_int2(0, 0);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const int2 a = lds_i32x2(row + (unsigned)(((first + c) & (NC - 1)) * NF * 4));
+        v.x += a.x;
+        v.y += a.y;
+    }
+    return v;
+}
+
+// Flush of a [cell][32] tile (rows not swizzled): lane = (coil cl, x pair px),
+// NF / 2 coils by 64 / NF pairs, so that one 8-byte shared load per lane covers
+// the banks and consecutive pairs of a coil plane are written together (NF =
+// 32: the two halves of one 32-byte sector).  Runs of pairs are dealt to the
+// warps.
+template <int NF>
+__device__ __forceinline__ void lanes_flush(const GridParams &P, float *gridf, unsigned acc, int cg, int ox, int oy,
+                                            int oz, float inv)
+{
+    constexpr int NCL = NF / 2, NPX = 32 / NCL;
+    const int Tx = P.tile[0], Ty = P.tile[1];
     const int CG = P.coil_group;
     const int ncl = min(CG, P.channels - cg * CG);
     const size_t G = (size_t)P.G;
@@ -962,21 +991,22 @@ __device__ __forceinline__ void lanes_flush(const GridParams &P, unsigned acc, i
     const size_t cells = P.dim == 3 ? G * G * G : G * G;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nwarps = blockDim.x >> 5;
-    float *gridf = P.grid;
-    if ((Tx % 4) == 0 && (P.G % 2) == 0 && ((reinterpret_cast<uintptr_t>(gridf) & 15) == 0)) {
-        const int cl = lane & 15, px = lane >> 4;
-        const int ppr = Tx / 4;  // x pair-pairs per row
-        const int units = Ty * Tz * ppr;
+    const int K = P.K;
+    if ((Tx % 2) == 0 && (P.G % 2) == 0 && ((reinterpret_cast<uintptr_t>(gridf) & 15) == 0)) {
+        const int cl = lane % NCL, px = lane / NCL;
+        const int hx = Tx / 2, npair = K / 2;
         const size_t cstride4 = cells >> 1;
         float4 *grid4 = reinterpret_cast<float4 *>(gridf) + (size_t)(cg * CG + cl) * cstride4;
-        for (int u = warp; u < units; u += nwarps) {
-            const int r = u / ppr, pp = u - r * ppr;
-            const int lx = 4 * pp + 2 * px;
+        for (int u0 = warp * NPX; u0 < npair; u0 += nwarps * NPX) {
+            // the warp's pairs: within one row (u0 / hx) where hx is a multiple of NPX
+            const int u = u0 + px;
+            const int r = hx % NPX == 0 ? u0 / hx : u / hx;
+            const int lx = 2 * (u - r * hx);
             const int gx = ox + lx, gy = oy + r % Ty, gz = oz + r / Ty;
-            if (cl >= ncl || gx >= P.G || gy >= P.G || gz >= Gz) continue;
-            const int i = r * Tx + lx;
-            const int2 a = lds_i32x2(acc + ((unsigned)i << 7) + ((unsigned)cl << 3));
-            const int2 b = lds_i32x2(acc + ((unsigned)(i + 1) << 7) + ((unsigned)cl << 3));
+            if (cl >= ncl || u >= npair || gx >= P.G || gy >= P.G || gz >= Gz) continue;
+            const int i = 2 * u;
+            const int2 a = lanes_cell<NF>(acc, i, cl, px);
+            const int2 b = lanes_cell<NF>(acc, i + 1, cl, px);
             const float sa = P.checkerboard && ((gx + gy + gz) & 1) ? -inv : inv;
             const float sb = P.checkerboard ? -sa : inv;
             const float4 v = make_float4((float)a.x * sa, (float)a.y * sa, (float)b.x * sb, (float)b.y * sb);
@@ -984,22 +1014,21 @@ __device__ __forceinline__ void lanes_flush(const GridParams &P, unsigned acc, i
         }
         return;
     }
-    const int K = P.K;
     float2 *grid = reinterpret_cast<float2 *>(gridf);
     for (int idx = threadIdx.x; idx < ncl * K; idx += blockDim.x) {
         const int i = idx / ncl, cl = idx - i * ncl;
         const int lx = i % Tx, r = i / Tx;
         const int gx = ox + lx, gy = oy + r % Ty, gz = oz + r / Ty;
         if (gx >= P.G || gy >= P.G || gz >= Gz) continue;
-        const int2 a = lds_i32x2(acc + ((unsigned)i << 7) + ((unsigned)cl << 3));
+        const int2 a = lanes_cell<NF>(acc, i, cl, 0);
         const float sg = P.checkerboard && ((gx + gy + gz) & 1) ? -inv : inv;
         put_cells(&grid[(size_t)(cg * CG + cl) * cells + ((size_t)gz * G + (size_t)gy) * G + (size_t)gx],
                   make_float2((float)a.x * sg, (float)a.y * sg), P.accumulate);
     }
 }
 
-template <typename IT>
-__global__ void __launch_bounds__(kLaneWarps * 32, 2) grid_lanes_kernel(GridParams P)
+template <int NF, int NW, typename IT>
+__global__ void __launch_bounds__(NW * 32, 16 / NW) grid_lanes_kernel(GridParams P)
 {
     extern __shared__ float4 smem_raw[];
     float4 *smem4 = aligned_smem(smem_raw);
@@ -1007,15 +1036,19 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) grid_lanes_kernel(GridPara
     const int cg = blockIdx.y;
     const int K = P.K;
     const int CG = P.coil_group;
-    const LaneSmem L_ = lane_smem_layout(K, P.L);
+    const LaneSmem L_ = lane_smem_layout(K, P.L, NW);
     const unsigned acc = smem_addr(smem4);
 
     const int t = it.tile;
     const int ox = (t % P.ntile[0]) * P.tile[0];
     const int oy = ((t / P.ntile[0]) % P.ntile[1]) * P.tile[1];
     const int oz = (t / (P.ntile[0] * P.ntile[1])) * P.tile[2];
+    // a batch's items carry their frame
+    auto frame_grid = [&] {
+        return P.grid + (P.frame_off ? (size_t)P.items[blockIdx.x].pad * (size_t)P.grid_frame_floats : 0);
+    };
     if (it.count == 0) {
-        if (!P.skip_empty) write_cell_group<32>(P, P.grid, acc, cg, ox, oy, oz, true, nullptr);
+        if (!P.skip_empty) write_cell_group<NF>(P, frame_grid(), acc, cg, ox, oy, oz, true, nullptr);
         return;
     }
     const int lane = threadIdx.x & 31;
@@ -1024,9 +1057,9 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) grid_lanes_kernel(GridPara
     // the tile starts at zero, and so do the value slots of a partial coil
     // group (a slot's coils past the group's last are never copied)
     for (int i = threadIdx.x; i < K * 8; i += blockDim.x) smem4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (min(CG, P.channels - cg * CG) < 16) {  // copies of fewer than 128 bytes (a partial group)
+    if (min(CG, P.channels - cg * CG) < NF / 2) {  // copies of fewer than NF floats (a partial group)
         float4 *stage_all = reinterpret_cast<float4 *>(reinterpret_cast<unsigned char *>(smem4) + L_.stage);
-        for (int i = threadIdx.x; i < kLaneWarps * kLaneBatch * 8; i += blockDim.x)
+        for (int i = threadIdx.x; i < NW * kLaneBatch * 8; i += blockDim.x)
             stage_all[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     for (int i = threadIdx.x; i < P.L; i += blockDim.x) lutw_s[i] = P.lutw[i];
@@ -1050,7 +1083,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) grid_lanes_kernel(GridPara
     const unsigned cmask = (1u << kTapCellBits) - 1u;
     const unsigned lane4 = (unsigned)lane << 2;
 
-    const int nrec = warp < it.count ? (it.count - warp + kLaneWarps - 1) / kLaneWarps : 0;
+    const int nrec = warp < it.count ? (it.count - warp + NW - 1) / NW : 0;
     const unsigned long long *trecs = P.trecs + it.begin + warp;
     // global loads run one step ahead of their use: the record words after
     // the window while it runs, the tap words of the next pass during the
@@ -1058,7 +1091,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) grid_lanes_kernel(GridPara
     // bulk copies are in flight
     auto load_rw = [&](int k0) -> unsigned long long {
         const int k = k0 + lane;
-        return k < nrec ? __ldg(trecs + (size_t)kLaneWarps * k) : 0ull;
+        return k < nrec ? __ldg(trecs + (size_t)NW * k) : 0ull;
     };
     // Records go through a window of 32, one per lane.  A window processes
     // only whole passes of 32 tap groups (the warp's last window: all its
@@ -1103,13 +1136,16 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) grid_lanes_kernel(GridPara
             // copies, slot c for the c-th: lane 0 arms the mbarrier with the
             // window's bytes before any copy is issued
             if (nnz > 0) {
-                if (lane == 0) mbar_expect_tx(mbar, (unsigned)nnz * vbytes);
+                if (lane == 0) mbar_expect_tx(mbar, (unsigned)nnz * vbytes * (32 / NF));
                 __syncwarp();
                 if ((staged >> lane) & 1u) {
                     const int c = __popc(staged & ((1u << lane) - 1u));
                     table4[c] =
                         make_int4((int)(unsigned)rw, (int)(((rw >> 32) & 0xFF) | ((unsigned)nt << 8)), excl, 0);
-                    bulk_copy_g2s(stage + ((unsigned)c << 7), kt + (IT)(unsigned)rw * vstride, vbytes, mbar);
+#pragma unroll
+                    for (int q = 0; q < 32 / NF; ++q)  // a copy of the values per copy of the cells
+                        bulk_copy_g2s(stage + ((unsigned)c << 7) + (unsigned)(q * NF * 4), kt + (IT)(unsigned)rw * vstride,
+                                      vbytes, mbar);
                 }
             }
             rw = nrw;
@@ -1179,14 +1215,14 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) grid_lanes_kernel(GridPara
                     w[k] = k < nl ? __fmul_rn(lutw_s[min(t[k] >> kTapCellBits, (unsigned)(P.L - 1))], sc) : 0.f;
                 }
                 const unsigned va = (stage + ((unsigned)cr << 7)) | lane4;
-                float v[32];
+                float v[NF];
 #pragma unroll
-                for (int f = 0; f < 32; ++f) v[f] = lds_f32_v(va ^ ((unsigned)f << 2));
+                for (int f = 0; f < NF; ++f) v[f] = lds_f32_v(va ^ ((unsigned)f << 2));
 #pragma unroll
                 for (int k = 0; k < kLaneTaps; ++k) {
                     if (k < nl) {
 #pragma unroll
-                        for (int f = 0; f < 32; ++f) red_add_fx(a[k] ^ ((unsigned)f << 2), w[k], v[f]);
+                        for (int f = 0; f < NF; ++f) red_add_fx(a[k] ^ ((unsigned)f << 2), w[k], v[f]);
                     }
                 }
             }
@@ -1195,17 +1231,21 @@ __global__ void __launch_bounds__(kLaneWarps * 32, 2) grid_lanes_kernel(GridPara
     }
     __syncthreads();
     if (it.slot < 0) {
-        lanes_flush(P, acc, cg, ox, oy, oz, inv);
+        lanes_flush<NF>(P, frame_grid(), acc, cg, ox, oy, oz, inv);
     } else {
-        // partial tile in the [cell][32] layout the reduction reads (float g
-        // of cell c at g ^ ((c & 15) << 1)): float4 q of a row is plain quad
-        // q ^ ((c & 15) >> 1), pairs swapped for odd cells
-        float4 *dst = reinterpret_cast<float4 *>(P.partials + ((size_t)it.slot * P.ngroups + cg) * (size_t)K * 32);
-        for (int i4 = threadIdx.x; i4 < K * 8; i4 += blockDim.x) {
-            const int c = i4 >> 3, q = i4 & 7;
-            int4 a = lds_s32x4(acc + ((unsigned)c << 7) + ((unsigned)(q ^ ((c & 15) >> 1)) << 4));
-            if (c & 1) a = make_int4(a.z, a.w, a.x, a.y);
-            dst[i4] = make_float4((float)a.x * inv, (float)a.y * inv, (float)a.z * inv, (float)a.w * inv);
+        // partial tile in the [cell][NF] layout the reduction reads: float p
+        // of cell c is float p ^ swz(c) (whole pairs move)
+        float4 *dst = reinterpret_cast<float4 *>(P.partials + ((size_t)it.slot * P.ngroups + cg) * (size_t)K * NF);
+        for (int i4 = threadIdx.x; i4 < K * (NF / 4); i4 += blockDim.x) {
+            const int c = i4 / (NF / 4), p0 = 4 * (i4 % (NF / 4)), sw = swz<NF>(c);
+            if constexpr (NF == 32) {  // one copy: the plain quad, its pairs swapped for odd cells
+                int4 a = lds_s32x4(acc + ((unsigned)c << 7) + (unsigned)(4 * (p0 ^ (sw & ~3))));
+                if (sw & 2) a = make_int4(a.z, a.w, a.x, a.y);
+                dst[i4] = make_float4((float)a.x * inv, (float)a.y * inv, (float)a.z * inv, (float)a.w * inv);
+                continue;
+            }
+            const int2 a = lanes_cell<NF>(acc, c, (p0 ^ sw) >> 1, c), b = lanes_cell<NF>(acc, c, ((p0 + 2) ^ sw) >> 1, c);
+            dst[i4] = make_float4((float)a.x * inv, (float)a.y * inv, (float)b.x * inv, (float)b.y * inv);
         }
     }
 }
@@ -1418,6 +1458,8 @@ __global__ void __launch_bounds__(kTrThreads) transpose_kspace_kernel(const floa
     }
 }
 
+int profile_events(fr_plan p, cudaEvent_t **ev);
+
 template <int DIM, int R>
 int launch(fr_plan p, const GridParams &P, long long nitems, long long nsplits, cudaStream_t s)
 {
@@ -1427,71 +1469,119 @@ int launch(fr_plan p, const GridParams &P, long long nitems, long long nsplits, 
     if (smem > 48 * 1024) FR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int threads = 512;
     dim3 grid((unsigned)nitems, (unsigned)P.ngroups);
-    cudaEvent_t *ev = nullptr;
-    if (p->profile) {
-        if (p->prof_used * 2 + 2 > (int)p->prof_ev.size()) {
-            cudaEvent_t a, b;
-            FR_CUDA(cudaEventCreate(&a));
-            FR_CUDA(cudaEventCreate(&b));
-            p->prof_ev.push_back(a);
-            p->prof_ev.push_back(b);
-        }
-        ev = &p->prof_ev[p->prof_used * 2];
-        p->prof_used++;
-        FR_CUDA(cudaEventRecord(ev[0], s));
-    }
+    cudaEvent_t *ev;
+    const int st = profile_events(p, &ev);
+    if (st) return st;
+    if (ev) FR_CUDA(cudaEventRecord(ev[0], s));
     kern<<<grid, threads, smem, s>>>(P);
     FR_CHECK_LAUNCH("grid_tiles_kernel");
     if (ev) FR_CUDA(cudaEventRecord(ev[1], s));
     return launch_reduce<R>(P, nsplits, s);
 }
 
+// Scatter timing (fr_plan_profile): an event pair per launch.
+int profile_events(fr_plan p, cudaEvent_t **ev)
+{
+    *ev = nullptr;
+    if (!p || !p->profile) return FR_OK;
+    if (p->prof_used * 2 + 2 > (int)p->prof_ev.size()) {
+        cudaEvent_t a, b;
+        FR_CUDA(cudaEventCreate(&a));
+        FR_CUDA(cudaEventCreate(&b));
+        p->prof_ev.push_back(a);
+        p->prof_ev.push_back(b);
+    }
+    *ev = &p->prof_ev[p->prof_used * 2];
+    p->prof_used++;
+    return FR_OK;
+}
+
+// Per-item scales (every launched item, so the indices match blockIdx.x); the
+// bounds go to the scratch past the scales.
+int launch_item_scales(const GridParams &P, long long nitems, cudaStream_t s)
+{
+    const int threads = 256;
+    const long long blocks = (nitems * 32 + threads - 1) / threads;
+    const long long boff = (nitems + 1) & ~1ll;  // 8-byte aligned float2
+    float2 *bound = reinterpret_cast<float2 *>(const_cast<float *>(P.item_inv) + boff);
+    item_bound_kernel<<<(unsigned)blocks, threads, 0, s>>>(P.items, nitems, P.trecs, P.mag, bound);
+    FR_CHECK_LAUNCH("item_bound_kernel");
+    item_inv_kernel<<<(unsigned)std::min<long long>((nitems + threads - 1) / threads, 152 * 8), threads, 0, s>>>(
+        bound, nitems, P.lut_absmax, const_cast<float *>(P.item_inv));
+    FR_CHECK_LAUNCH("item_inv_kernel");
+    return FR_OK;
+}
+
+// 32-bit indices when the tap words and sample-major values allow them.
+bool index32(const GridParams &P)
+{
+    return (double)P.n * (double)P.tap_words < 2147483647.0 && (double)P.n * (double)(2 * P.kstride) < 2147483647.0;
+}
+
+// Warps per CTA of the tap-lane scatter for tiles of K cells; 0: no room.
+int lane_warps(long long K, int L)
+{
+    if (K <= 512 && lane_smem_layout(K, L, kLaneWarpsSmall).end + 128 <= 227 * 1024) return kLaneWarpsSmall;
+    if (lane_smem_layout(K, L, kLaneWarpsLarge).end + 128 <= 227 * 1024) return kLaneWarpsLarge;
+    return lane_smem_layout(K, L, kLaneWarpsSmall).end + 128 <= 227 * 1024 ? kLaneWarpsSmall : 0;
+}
+
+// Coil floats of the tap-lane scatter for a group of `coils` coils.
+int lane_floats(int coils) { return coils > 8 ? 32 : coils > 4 ? 16 : 8; }
+
+template <int NF, int NW>
+int launch_lanes_t(fr_plan p, const GridParams &P, long long nitems, cudaStream_t s)
+{
+    const size_t smem = lane_smem_layout(P.K, P.L, NW).end + 128;
+    auto kern = index32(P) ? grid_lanes_kernel<NF, NW, unsigned> : grid_lanes_kernel<NF, NW, unsigned long long>;
+    if (smem > 48 * 1024) FR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    dim3 grid((unsigned)nitems, (unsigned)P.ngroups);
+    cudaEvent_t *ev;
+    const int st = profile_events(p, &ev);
+    if (st) return st;
+    if (ev) FR_CUDA(cudaEventRecord(ev[0], s));
+    kern<<<grid, NW * 32, smem, s>>>(P);
+    FR_CHECK_LAUNCH("grid_lanes_kernel");
+    if (ev) FR_CUDA(cudaEventRecord(ev[1], s));
+    return FR_OK;
+}
+
+// The tap-lane scatter: P.coil_group is at most NF / 2 coils, the partial tiles
+// have NF floats per cell.
+int launch_lanes(fr_plan p, const GridParams &P, int NF, long long nitems, long long nsplits, cudaStream_t s)
+{
+    int st = launch_item_scales(P, nitems, s);
+    if (st) return st;
+    const bool large = lane_warps(P.K, P.L) == kLaneWarpsLarge;
+    switch (NF) {
+    case 8:
+        st = large ? launch_lanes_t<8, kLaneWarpsLarge>(p, P, nitems, s) : launch_lanes_t<8, kLaneWarpsSmall>(p, P, nitems, s);
+        return st ? st : launch_reduce<8>(P, nsplits, s);
+    case 16:
+        st = large ? launch_lanes_t<16, kLaneWarpsLarge>(p, P, nitems, s) : launch_lanes_t<16, kLaneWarpsSmall>(p, P, nitems, s);
+        return st ? st : launch_reduce<16>(P, nsplits, s);
+    default:
+        st = large ? launch_lanes_t<32, kLaneWarpsLarge>(p, P, nitems, s) : launch_lanes_t<32, kLaneWarpsSmall>(p, P, nitems, s);
+        return st ? st : launch_reduce<32>(P, nsplits, s);
+    }
+}
+
+// The per-warp tap lists.
 template <int R>
 int launch_taps(fr_plan p, const GridParams &P, long long nitems, long long nsplits, cudaStream_t s)
 {
-    // per-item scales first (every launched item, so the indices match
-    // blockIdx.x); the bounds go to the scratch past the scales
-    {
-        const int threads = 256;
-        const long long blocks = (nitems * 32 + threads - 1) / threads;
-        const long long boff = (nitems + 1) & ~1ll;  // 8-byte aligned float2
-        float2 *bound = reinterpret_cast<float2 *>(const_cast<float *>(P.item_inv) + boff);
-        item_bound_kernel<<<(unsigned)blocks, threads, 0, s>>>(P.items, nitems, P.trecs, P.mag, bound);
-        FR_CHECK_LAUNCH("item_bound_kernel");
-        item_inv_kernel<<<(unsigned)std::min<long long>((nitems + threads - 1) / threads, 152 * 8), threads, 0, s>>>(
-            bound, nitems, P.lut_absmax, const_cast<float *>(P.item_inv));
-        FR_CHECK_LAUNCH("item_inv_kernel");
-    }
-    // 32-bit indices when the tap words and sample-major values allow them
-    const bool idx32 = (double)P.n * (double)P.tap_words < 2147483647.0 &&
-                       (double)P.n * (double)(2 * P.kstride) < 2147483647.0;
-    // rows of 32 coil floats: the tap-lane scatter, unless a plan asks for
-    // the per-warp tap lists
-    const LaneSmem lm = lane_smem_layout(P.K, P.L);
-    const bool lanes = R == 32 && !p->scatter_warp_lists && lm.end + 128 <= 227 * 1024 && (P.kstride % 2) == 0;
-    const TapSmem m = tap_smem_layout(P.K, R, P.L);
-    const size_t smem = lanes ? lm.end + 128 : m.end + 128;
+    int st = launch_item_scales(P, nitems, s);
+    if (st) return st;
+    const size_t smem = tap_smem_layout(P.K, R, P.L).end + 128;
     if (smem > 227 * 1024) return fail(FR_ERR_UNSUPPORTED, "tap-list scatter does not fit in shared memory");
-    auto kern = lanes ? (idx32 ? grid_lanes_kernel<unsigned> : grid_lanes_kernel<unsigned long long>)
-                      : (idx32 ? grid_taps_kernel<R, unsigned> : grid_taps_kernel<R, unsigned long long>);
-    const int threads = lanes ? kLaneWarps * 32 : kWarps * 32;
+    auto kern = index32(P) ? grid_taps_kernel<R, unsigned> : grid_taps_kernel<R, unsigned long long>;
     if (smem > 48 * 1024) FR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dim3 grid((unsigned)nitems, (unsigned)P.ngroups);
-    cudaEvent_t *ev = nullptr;
-    if (p->profile) {
-        if (p->prof_used * 2 + 2 > (int)p->prof_ev.size()) {
-            cudaEvent_t a, b;
-            FR_CUDA(cudaEventCreate(&a));
-            FR_CUDA(cudaEventCreate(&b));
-            p->prof_ev.push_back(a);
-            p->prof_ev.push_back(b);
-        }
-        ev = &p->prof_ev[p->prof_used * 2];
-        p->prof_used++;
-        FR_CUDA(cudaEventRecord(ev[0], s));
-    }
-    kern<<<grid, threads, smem, s>>>(P);
-    FR_CHECK_LAUNCH(lanes ? "grid_lanes_kernel" : "grid_taps_kernel");
+    cudaEvent_t *ev;
+    if ((st = profile_events(p, &ev))) return st;
+    if (ev) FR_CUDA(cudaEventRecord(ev[0], s));
+    kern<<<grid, kWarps * 32, smem, s>>>(P);
+    FR_CHECK_LAUNCH("grid_taps_kernel");
     if (ev) FR_CUDA(cudaEventRecord(ev[1], s));
     return launch_reduce<R>(P, nsplits, s);
 }
@@ -1637,6 +1727,18 @@ int grid_run(fr_plan p, const float *d_kdata, const float *d_dcf, int channels, 
         const size_t words = (((size_t)nlaunch + 1) & ~(size_t)1) + 2 * (size_t)nlaunch;
         if (p->item_inv.reserve(words * 4)) return FR_ERR_OUT_OF_MEMORY;
         P.item_inv = p->item_inv.as<float>();
+        // the tap lanes, except for coil groups of 4 on tiles of up to 512 cells,
+        // where the per-warp lists' 32 warps per SM hide more latency than the
+        // lanes' 16 (3 coils, 303 k samples on a 115^3 grid: 124 us against 135; on
+        // the 32 x 32 tiles of 2D, 4 coils, 2.7 k samples: 17 against 14)
+        const int nw = lane_warps(P.K, P.L);
+        const bool lists = p->scatter_warp_lists || (R == 8 && nw == kLaneWarpsSmall);
+        if (!lists && nw > 0 && (P.kstride % 2) == 0) {
+            // one group of fewer coils than the plan's: its floats only
+            const int NF = lane_floats(std::min(channels, P.coil_group));
+            P.coil_group = std::min(P.coil_group, NF / 2);
+            return launch_lanes(p, P, NF, nlaunch, p->nsplits, s);
+        }
         switch (R) {
         case 8: return launch_taps<8>(p, P, nlaunch, p->nsplits, s);
         case 16: return launch_taps<16>(p, P, nlaunch, p->nsplits, s);
