@@ -72,7 +72,21 @@ struct GridParams {
     int *err = nullptr;       // mapped error word
     int accumulate = 0;       // add the tiles to the grid instead of overwriting it (sample partitions)
     long long kin_stride = 0; // complex values between coils of the caller's coil-major k-space (0: n)
+    // batches: per frame and coil a large |re| or |im| of dcf * k (float bits,
+    // coil_max_kernel): the sample-major copy holds every coil scaled by
+    // 2^coil_exponent, so that one fixed-point scale per item serves weak and
+    // strong coils alike; nullptr: the copy is not scaled
+    const unsigned *coil_max = nullptr;
+    float sum_limit = 1073741824.f;  // bound of an item's fixed-point sums (fixed_sum_limit)
 };
+
+// Exponent that brings a coil's measure into [1, 2) (0 for a coil of zeros);
+// 2^e and 2^-e are normal floats.
+__device__ __forceinline__ int coil_exponent(unsigned max_bits)
+{
+    const float m = __uint_as_float(max_bits);
+    return m > 0.f ? max(min(-ilogbf(m), 120), -120) : 0;
+}
 
 // Column swizzle of cell i in a row of R floats: keeps (re, im) pairs
 // adjacent and spreads the flush (lanes along cells) over all banks.
@@ -100,9 +114,10 @@ __device__ __forceinline__ unsigned smem_addr(const void *p)
 // value is acc / S at the flush.
 __device__ __forceinline__ void red_add_fx(unsigned a, float w, float vs)
 {
-    // w * vs rounded to the nearest integer: |w * vs| < 2^22, so adding
-    // 1.5 * 2^23 in the same fused operation lands in [2^23, 2^24), where the
-    // float spacing is 1, and the low mantissa bits are the integer.
+    // w * vs rounded to the nearest integer: |w * vs| <= 2^22, so adding
+    // 1.5 * 2^23 in the same fused operation lands in [2^23, 2^24], where the
+    // float spacing is 1 (2^24 itself is a float), and the low mantissa bits
+    // are the integer.
     const int i = __float_as_int(fmaf(w, vs, 12582912.f)) - 0x4B400000;
     asm volatile("red.shared.add.s32 [%0], %1;" ::"r"(a), "r"(i));
 }
@@ -315,9 +330,11 @@ __device__ __forceinline__ void stage_tables(const GridParams &P, float4 *smem4)
 // M_f = max over the item's samples of |dcf * k_f|, and |w| <= lut_absmax,
 // every partial sum is below B_f * lut_absmax and every add below
 // M_f * lut_absmax, so S_f = the largest power of two with
-// S_f * B_f * lut_absmax <= 2^30 and S_f * M_f * lut_absmax <= 2^21 keeps
-// the tile in int32 and each add exact to +-1/2.  The rounding error of an
-// add is then at most B_f / 2^31 (dense items) or 2^-23 M_f.
+// S_f * B_f * lut_absmax <= sum_limit (below 2^31 by more than half an item's
+// records, the roundings' sum: fixed_sum_limit) and S_f * M_f * lut_absmax <=
+// 2^22 (the rounding of red_add_fx) keeps the tile in int32 and each add exact
+// to +-1/2.  The rounding error of an add is then at most B_f / 2^30.9 (dense
+// items) or 2^-22 M_f; limits of 2^30 and 2^21 left twice the error.
 //
 // This warp's part of B_f and M_f over records warp, warp + NW, ... in steps
 // of kScaleBatch records with every load of a step issued before the first
@@ -389,14 +406,14 @@ __device__ __forceinline__ void scale_bounds_mag(const unsigned long long *recs,
 }
 
 // 1 / S_f from the item's B_f and M_f (exact: a power of two).
-__device__ __forceinline__ float inv_scale_of(float bsum, unsigned bmax_bits, float lut_absmax)
+__device__ __forceinline__ float inv_scale_of(float bsum, unsigned bmax_bits, float lut_absmax, float sum_limit)
 {
     const float B = __fmul_rn(bsum, lut_absmax);
     const float M = __fmul_rn(__uint_as_float(bmax_bits), lut_absmax);
     int e = 0;
     if (B > 0.f && M > 0.f) {
-        // largest power of two 2^e <= min(2^30 / B, 2^21 / M)
-        const float t = fminf(__fdiv_rn(1073741824.f, B), __fdiv_rn(2097152.f, M));
+        // largest power of two 2^e <= min(sum_limit / B, 2^22 / M)
+        const float t = fminf(__fdiv_rn(sum_limit, B), __fdiv_rn(4194304.f, M));
         frexpf(t, &e);
         e = max(min(e - 1, 100), -100);
     }
@@ -488,7 +505,7 @@ __device__ __forceinline__ void grid_item(const GridParams &P, const WorkItem &i
             atomicMax(&bmax_s[0], __float_as_uint(bm));
         }
         __syncthreads();
-        if (threadIdx.x < R) inv_s[threadIdx.x] = inv_scale_of(bsum_s[0], bmax_s[0], P.lut_absmax);
+        if (threadIdx.x < R) inv_s[threadIdx.x] = inv_scale_of(bsum_s[0], bmax_s[0], P.lut_absmax, P.sum_limit);
         __syncthreads();
     } else {
         float bs[NF], bm[NF];
@@ -503,7 +520,7 @@ __device__ __forceinline__ void grid_item(const GridParams &P, const WorkItem &i
             }
         }
         __syncthreads();
-        if (threadIdx.x < R) inv_s[threadIdx.x] = inv_scale_of(bsum_s[threadIdx.x], bmax_s[threadIdx.x], P.lut_absmax);
+        if (threadIdx.x < R) inv_s[threadIdx.x] = inv_scale_of(bsum_s[threadIdx.x], bmax_s[threadIdx.x], P.lut_absmax, P.sum_limit);
         __syncthreads();
     }
     const bool premul = P.mag != nullptr;
@@ -896,9 +913,9 @@ constexpr int kLaneWarpsSmall = 8, kLaneWarpsLarge = 16;
 // Shared-memory layout of grid_lanes_kernel from its 128-byte aligned base:
 // tile [K][32] int32 | weights [L] | per warp: value slots [32][32] floats,
 // record table [32] int4 {sample, first word | taps << 8, first group, 0} |
-// per warp one mbarrier (8 bytes).
+// per warp one mbarrier (8 bytes) | inverse scale per coil [16] (batches).
 struct LaneSmem {
-    unsigned lutw, stage, table, mbar, end;
+    unsigned lutw, stage, table, mbar, unscale, end;
 };
 __host__ __device__ __forceinline__ LaneSmem lane_smem_layout(long long K, int L, int warps)
 {
@@ -907,7 +924,8 @@ __host__ __device__ __forceinline__ LaneSmem lane_smem_layout(long long K, int L
     m.stage = m.lutw + (unsigned)((L * 4 + 127) & ~127);
     m.table = m.stage + (unsigned)(warps * kLaneBatch * 128);
     m.mbar = m.table + (unsigned)(warps * kLaneBatch * 16);
-    m.end = m.mbar + (unsigned)(warps * 8);
+    m.unscale = m.mbar + (unsigned)(warps * 8);
+    m.end = m.unscale + 64u;
     return m;
 }
 
@@ -955,6 +973,12 @@ __device__ __forceinline__ bool mbar_wait(unsigned mbar, unsigned parity)
     return false;
 }
 
+// The grid of an item's frame (a single trajectory is one frame).
+__device__ __forceinline__ float *lanes_frame_grid(const GridParams &P, long long item)
+{
+    return P.grid + (P.frame_off ? (size_t)P.items[item].pad * (size_t)P.grid_frame_floats : 0);
+}
+
 // (re, im) of coil cl at cell i of a [cell][32] tile: the sum of the row's
 // copies, `first` the copy to start from (lanes on different rows of the same
 // coil start from different copies, in different banks).
@@ -979,9 +1003,10 @@ __device__ __forceinline__ int2 lanes_cell(unsigned acc, int i, int cl, int firs
 // 32: the two halves of one 32-byte sector).  Runs of pairs are dealt to the
 // warps.
 template <int NF>
-__device__ __forceinline__ void lanes_flush(const GridParams &P, float *gridf, unsigned acc, int cg, int ox, int oy,
-                                            int oz, float inv)
+__device__ __forceinline__ void lanes_flush(const GridParams &P, long long item, unsigned acc, int cg, int ox, int oy,
+                                            int oz, float inv_item, const float *unscale)
 {
+    float *gridf = lanes_frame_grid(P, item);
     constexpr int NCL = NF / 2, NPX = 32 / NCL;
     const int Tx = P.tile[0], Ty = P.tile[1];
     const int CG = P.coil_group;
@@ -997,6 +1022,7 @@ __device__ __forceinline__ void lanes_flush(const GridParams &P, float *gridf, u
         const int hx = Tx / 2, npair = K / 2;
         const size_t cstride4 = cells >> 1;
         float4 *grid4 = reinterpret_cast<float4 *>(gridf) + (size_t)(cg * CG + cl) * cstride4;
+        const float inv = unscale ? unscale[cl] : inv_item;
         for (int u0 = warp * NPX; u0 < npair; u0 += nwarps * NPX) {
             // the warp's pairs: within one row (u0 / hx) where hx is a multiple of NPX
             const int u = u0 + px;
@@ -1021,39 +1047,31 @@ __device__ __forceinline__ void lanes_flush(const GridParams &P, float *gridf, u
         const int gx = ox + lx, gy = oy + r % Ty, gz = oz + r / Ty;
         if (gx >= P.G || gy >= P.G || gz >= Gz) continue;
         const int2 a = lanes_cell<NF>(acc, i, cl, 0);
+        const float inv = unscale ? unscale[cl] : inv_item;
         const float sg = P.checkerboard && ((gx + gy + gz) & 1) ? -inv : inv;
         put_cells(&grid[(size_t)(cg * CG + cl) * cells + ((size_t)gz * G + (size_t)gy) * G + (size_t)gx],
                   make_float2((float)a.x * sg, (float)a.y * sg), P.accumulate);
     }
 }
 
+// One work item with samples for one coil group: the tile zeroed, the item's
+// records added, the tile flushed.  `parity`: of the warp's mbarrier, which
+// carries over from item to item; the weights must be staged.
 template <int NF, int NW, typename IT>
-__global__ void __launch_bounds__(NW * 32, 16 / NW) grid_lanes_kernel(GridParams P)
+__device__ __forceinline__ void lanes_item(const GridParams &P, const WorkItem &it, long long item, int cg, float4 *smem4,
+                                           unsigned &parity)
 {
-    extern __shared__ float4 smem_raw[];
-    float4 *smem4 = aligned_smem(smem_raw);
-    const WorkItem it = P.items[blockIdx.x];
-    const int cg = blockIdx.y;
     const int K = P.K;
     const int CG = P.coil_group;
     const LaneSmem L_ = lane_smem_layout(K, P.L, NW);
     const unsigned acc = smem_addr(smem4);
-
     const int t = it.tile;
     const int ox = (t % P.ntile[0]) * P.tile[0];
     const int oy = ((t / P.ntile[0]) % P.ntile[1]) * P.tile[1];
     const int oz = (t / (P.ntile[0] * P.ntile[1])) * P.tile[2];
-    // a batch's items carry their frame
-    auto frame_grid = [&] {
-        return P.grid + (P.frame_off ? (size_t)P.items[blockIdx.x].pad * (size_t)P.grid_frame_floats : 0);
-    };
-    if (it.count == 0) {
-        if (!P.skip_empty) write_cell_group<NF>(P, frame_grid(), acc, cg, ox, oy, oz, true, nullptr);
-        return;
-    }
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    float *lutw_s = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(smem4) + L_.lutw);
+    const float *lutw_s = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(smem4) + L_.lutw);
     // the tile starts at zero, and so do the value slots of a partial coil
     // group (a slot's coils past the group's last are never copied)
     for (int i = threadIdx.x; i < K * 8; i += blockDim.x) smem4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1062,11 +1080,16 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) grid_lanes_kernel(GridParams
         for (int i = threadIdx.x; i < NW * kLaneBatch * 8; i += blockDim.x)
             stage_all[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    for (int i = threadIdx.x; i < P.L; i += blockDim.x) lutw_s[i] = P.lutw[i];
-    const float inv = P.item_inv[blockIdx.x];
+    const float inv = P.item_inv[item];
     const float sc = __fdiv_rn(1.f, inv);  // exact: a power of two
     const unsigned mbar = acc + L_.mbar + 8u * (unsigned)warp;
-    if (lane == 0) mbar_init(mbar);
+    float *unscale = nullptr;
+    if (P.coil_max) {  // a batch: the coils' own scales undone with the item's
+        unscale = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(smem4) + L_.unscale);
+        if (threadIdx.x < NF / 2 && cg * CG + (int)threadIdx.x < P.channels)
+            unscale[threadIdx.x] =
+                inv * ldexpf(1.f, -coil_exponent(P.coil_max[(size_t)it.pad * P.channels + cg * CG + threadIdx.x]));
+    }
     __syncthreads();
 
     const unsigned stage = acc + L_.stage + (unsigned)(warp * kLaneBatch * 128);
@@ -1075,7 +1098,6 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) grid_lanes_kernel(GridParams
     // bytes of a record's coil values: whole coil pairs (an odd count's pad
     // coil is zero in the sample-major copy)
     const unsigned vbytes = 16u * (unsigned)((ncl + 1) >> 1);
-    unsigned parity = 0u;
     const float *kt = P.kdata + 2 * (size_t)cg * CG;
     const unsigned *taps = P.taps;
     const IT tw = (IT)P.tap_words;
@@ -1231,22 +1253,90 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) grid_lanes_kernel(GridParams
     }
     __syncthreads();
     if (it.slot < 0) {
-        lanes_flush<NF>(P, frame_grid(), acc, cg, ox, oy, oz, inv);
+        lanes_flush<NF>(P, item, acc, cg, ox, oy, oz, inv, unscale);
     } else {
         // partial tile in the [cell][NF] layout the reduction reads: float p
         // of cell c is float p ^ swz(c) (whole pairs move)
         float4 *dst = reinterpret_cast<float4 *>(P.partials + ((size_t)it.slot * P.ngroups + cg) * (size_t)K * NF);
         for (int i4 = threadIdx.x; i4 < K * (NF / 4); i4 += blockDim.x) {
             const int c = i4 / (NF / 4), p0 = 4 * (i4 % (NF / 4)), sw = swz<NF>(c);
+            float ia = inv, ib = inv;
+            if (unscale) {
+                ia = unscale[(p0 ^ sw) >> 1];
+                ib = unscale[((p0 + 2) ^ sw) >> 1];
+            }
             if constexpr (NF == 32) {  // one copy: the plain quad, its pairs swapped for odd cells
                 int4 a = lds_s32x4(acc + ((unsigned)c << 7) + (unsigned)(4 * (p0 ^ (sw & ~3))));
                 if (sw & 2) a = make_int4(a.z, a.w, a.x, a.y);
-                dst[i4] = make_float4((float)a.x * inv, (float)a.y * inv, (float)a.z * inv, (float)a.w * inv);
+                dst[i4] = make_float4((float)a.x * ia, (float)a.y * ia, (float)a.z * ib, (float)a.w * ib);
                 continue;
             }
             const int2 a = lanes_cell<NF>(acc, c, (p0 ^ sw) >> 1, c), b = lanes_cell<NF>(acc, c, ((p0 + 2) ^ sw) >> 1, c);
-            dst[i4] = make_float4((float)a.x * inv, (float)a.y * inv, (float)b.x * inv, (float)b.y * inv);
+            dst[i4] = make_float4((float)a.x * ia, (float)a.y * ia, (float)b.x * ib, (float)b.y * ib);
         }
+    }
+}
+
+// Where the lanes' shared tables are set up: the weights, and the warps'
+// mbarriers (the item's first barrier orders both).
+template <int NW>
+__device__ __forceinline__ void lanes_setup(const GridParams &P, float4 *smem4)
+{
+    const LaneSmem L_ = lane_smem_layout(P.K, P.L, NW);
+    float *lutw_s = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(smem4) + L_.lutw);
+    for (int i = threadIdx.x; i < P.L; i += blockDim.x) lutw_s[i] = P.lutw[i];
+    if ((threadIdx.x & 31) == 0) mbar_init(smem_addr(smem4) + L_.mbar + 8u * (threadIdx.x >> 5));
+}
+
+// Zeros for the cells of a tile without samples.
+template <int NF>
+__device__ __forceinline__ void lanes_zero(const GridParams &P, const WorkItem &it, long long item, int cg, float4 *smem4)
+{
+    if (P.skip_empty) return;
+    const int t = it.tile;
+    write_cell_group<NF>(P, lanes_frame_grid(P, item), smem_addr(smem4), cg, (t % P.ntile[0]) * P.tile[0],
+                         ((t / P.ntile[0]) % P.ntile[1]) * P.tile[1], (t / (P.ntile[0] * P.ntile[1])) * P.tile[2], true,
+                         nullptr);
+}
+
+// One CTA per (work item, coil group).
+template <int NF, int NW, typename IT>
+__global__ void __launch_bounds__(NW * 32, 16 / NW) grid_lanes_kernel(GridParams P)
+{
+    extern __shared__ float4 smem_raw[];
+    float4 *smem4 = aligned_smem(smem_raw);
+    const WorkItem it = P.items[blockIdx.x];
+    if (it.count == 0) return lanes_zero<NF>(P, it, blockIdx.x, blockIdx.y, smem4);
+    unsigned parity = 0u;
+    lanes_setup<NW>(P, smem4);
+    lanes_item<NF, NW, IT>(P, it, blockIdx.x, blockIdx.y, smem4, parity);
+}
+
+// Persistent, for batches: as many CTAs as fit on the GPU, each taking work
+// indices (coil group major, then item) from a counter zeroed before the
+// launch, until none are left; the tables are set up once.
+template <int NF, int NW, typename IT>
+__global__ void __launch_bounds__(NW * 32, 16 / NW) batch_lanes_kernel(GridParams P)
+{
+    extern __shared__ float4 smem_raw[];
+    float4 *smem4 = aligned_smem(smem_raw);
+    __shared__ long long next;
+    const long long nitems = P.nwork / P.ngroups;
+    unsigned parity = 0u;
+    lanes_setup<NW>(P, smem4);
+    for (;;) {
+        __syncthreads();  // the previous item's flush is done with the tile
+        if (threadIdx.x == 0) next = atomicAdd(P.work_counter, 1);
+        __syncthreads();
+        const long long w = next;
+        if (w >= P.nwork) break;
+        const int cg = (int)(w / nitems);
+        const long long item = w - (long long)cg * nitems;
+        const WorkItem it = P.items[item];
+        if (it.count == 0)
+            lanes_zero<NF>(P, it, item, cg, smem4);
+        else
+            lanes_item<NF, NW, IT>(P, it, item, cg, smem4, parity);
     }
 }
 
@@ -1288,12 +1378,12 @@ __global__ void item_bound_kernel(const WorkItem *__restrict__ items, long long 
 // Inverse fixed-point scale of every work item from its own bound (see
 // inv_scale_of).
 __global__ void item_inv_kernel(const float2 *__restrict__ bound, long long nitems, float lut_absmax,
-                                float *__restrict__ inv)
+                                float sum_limit, float *__restrict__ inv)
 {
     for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < nitems;
          w += (long long)gridDim.x * blockDim.x) {
         const float2 b = bound[w];
-        inv[w] = inv_scale_of(b.x, __float_as_uint(b.y), lut_absmax);
+        inv[w] = inv_scale_of(b.x, __float_as_uint(b.y), lut_absmax, sum_limit);
     }
 }
 
@@ -1407,18 +1497,31 @@ int launch_reduce(const GridParams &P, long long nsplits, cudaStream_t s)
 // bound by the latency of these reads).
 constexpr int kTrSamples = 128;
 constexpr int kTrThreads = 256, kTrPer = 8;
+constexpr int kTrCoils = 96;  // the copy's shared memory holds at most 95 coils
 // The copy holds dcf * k (the product GridLut.cpp:109 forms, same rounding)
-// and mag[s] = the largest |re| or |im| of sample s's products.
+// and mag[s] = the largest |re| or |im| of sample s's products.  blocks: the
+// sample runs of a batch, one per CTA (nullptr: one trajectory).
 __global__ void __launch_bounds__(kTrThreads) transpose_kspace_kernel(const float2 *__restrict__ in,
                                                                       const float *__restrict__ dcf,
                                                                       float2 *__restrict__ out,
                                                                       float *__restrict__ mag, long long n,
-                                                                      int channels, int cstride, long long in_stride)
+                                                                      int channels, int cstride, long long in_stride,
+                                                                      const FrameRun *__restrict__ blocks,
+                                                                      const unsigned *__restrict__ coil_max)
 {
     extern __shared__ float2 tr[];  // [channels][kTrSamples + 1]
-    __shared__ float dsh[kTrSamples];
-    const long long s0 = (long long)blockIdx.x * kTrSamples;
-    const int ns = (int)min((long long)kTrSamples, n - s0);
+    __shared__ float dsh[kTrSamples], csh[kTrCoils];
+    long long s0 = (long long)blockIdx.x * kTrSamples;  // first sample, of all frames
+    int ns = (int)min((long long)kTrSamples, n - s0);
+    if (blocks) {
+        const FrameRun r = blocks[blockIdx.x];
+        s0 = r.off + r.begin;
+        ns = min(kTrSamples, r.n - r.begin);
+        in += (size_t)(channels - 1) * (size_t)r.off;  // the frame's block starts at channels * off
+        in_stride = r.n;
+        for (int c = threadIdx.x; c < channels; c += kTrThreads)
+            csh[c] = ldexpf(1.f, coil_exponent(coil_max[(size_t)r.frame * channels + c]));
+    }
     for (int j = threadIdx.x; j < ns; j += kTrThreads) dsh[j] = dcf[s0 + j];
     const int total = channels * kTrSamples;
     for (int i0 = 0; i0 < total; i0 += kTrThreads * kTrPer) {
@@ -1444,6 +1547,7 @@ __global__ void __launch_bounds__(kTrThreads) transpose_kspace_kernel(const floa
             const float2 v = tr[c * (kTrSamples + 1) + j];
             const float d = dsh[j];
             o = make_float2(__fmul_rn(d, v.x), __fmul_rn(d, v.y));
+            if (blocks) o = make_float2(o.x * csh[c], o.y * csh[c]);
         }
         out[(size_t)(s0 + j) * cstride + c] = o;
     }
@@ -1452,10 +1556,44 @@ __global__ void __launch_bounds__(kTrThreads) transpose_kspace_kernel(const floa
         float m = 0.f;
         for (int c = 0; c < channels; ++c) {
             const float2 v = tr[c * (kTrSamples + 1) + j];
-            m = fmaxf(m, fmaxf(fabsf(__fmul_rn(d, v.x)), fabsf(__fmul_rn(d, v.y))));
+            float a = fmaxf(fabsf(__fmul_rn(d, v.x)), fabsf(__fmul_rn(d, v.y)));
+            // a coil's infinities stay its own: they do not set the other coils' scale
+            if (blocks) a = isfinite(a) ? a * csh[c] : 0.f;
+            m = fmaxf(m, a);
         }
         mag[s0 + j] = m;
     }
+}
+
+// Per frame and coil the largest finite |re| or |im| of dcf * k over every
+// kCoilMaxStep-th run of samples, as float bits (the table starts at zero): a
+// measure of the coil's strength, not a bound.  A CTA per run, all its loads in
+// flight, coil maxima in shared memory.
+constexpr int kCoilMaxStep = 4;
+__global__ void __launch_bounds__(kTrThreads) coil_max_kernel(const float2 *__restrict__ in,
+                                                              const float *__restrict__ dcf,
+                                                              const FrameRun *__restrict__ runs, int channels,
+                                                              unsigned *__restrict__ coil_max)
+{
+    __shared__ unsigned mx[kTrCoils];
+    const FrameRun r = runs[blockIdx.x];
+    if ((r.begin / kTrSamples) % kCoilMaxStep != 0) return;
+    const int ns = min(kTrSamples, r.n - r.begin);
+    for (int c = threadIdx.x; c < channels; c += kTrThreads) mx[c] = 0u;
+    __syncthreads();
+    const int j = threadIdx.x % kTrSamples;
+    const float d = j < ns ? dcf[r.off + r.begin + j] : 0.f;
+    in += (size_t)channels * (size_t)r.off + r.begin + j;
+#pragma unroll 4
+    for (int c = threadIdx.x / kTrSamples; c < channels; c += kTrThreads / kTrSamples) {
+        const float2 v = j < ns ? in[(size_t)c * r.n] : make_float2(0.f, 0.f);
+        const float a = fmaxf(fabsf(__fmul_rn(d, v.x)), fabsf(__fmul_rn(d, v.y)));
+        const unsigned m = __reduce_max_sync(0xffffffffu, isfinite(a) ? __float_as_uint(a) : 0u);
+        if ((threadIdx.x & 31) == 0) atomicMax(&mx[c], m);
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < channels; c += kTrThreads)
+        if (mx[c]) atomicMax(&coil_max[(size_t)r.frame * channels + c], mx[c]);
 }
 
 int profile_events(fr_plan p, cudaEvent_t **ev);
@@ -1507,7 +1645,7 @@ int launch_item_scales(const GridParams &P, long long nitems, cudaStream_t s)
     item_bound_kernel<<<(unsigned)blocks, threads, 0, s>>>(P.items, nitems, P.trecs, P.mag, bound);
     FR_CHECK_LAUNCH("item_bound_kernel");
     item_inv_kernel<<<(unsigned)std::min<long long>((nitems + threads - 1) / threads, 152 * 8), threads, 0, s>>>(
-        bound, nitems, P.lut_absmax, const_cast<float *>(P.item_inv));
+        bound, nitems, P.lut_absmax, P.sum_limit, const_cast<float *>(P.item_inv));
     FR_CHECK_LAUNCH("item_inv_kernel");
     return FR_OK;
 }
@@ -1533,6 +1671,18 @@ template <int NF, int NW>
 int launch_lanes_t(fr_plan p, const GridParams &P, long long nitems, cudaStream_t s)
 {
     const size_t smem = lane_smem_layout(P.K, P.L, NW).end + 128;
+    if (P.frame_off) {  // a batch
+        auto kern = index32(P) ? batch_lanes_kernel<NF, NW, unsigned> : batch_lanes_kernel<NF, NW, unsigned long long>;
+        if (smem > 48 * 1024) FR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        int per_sm = 0, dev = 0, sms = 0;
+        FR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NW * 32, smem));
+        FR_CUDA(cudaGetDevice(&dev));
+        FR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        FR_CUDA(cudaMemsetAsync(P.work_counter, 0, sizeof(int), s));
+        kern<<<(unsigned)std::min<long long>(P.nwork, (long long)std::max(per_sm, 1) * sms), NW * 32, smem, s>>>(P);
+        FR_CHECK_LAUNCH("batch_lanes_kernel");
+        return FR_OK;
+    }
     auto kern = index32(P) ? grid_lanes_kernel<NF, NW, unsigned> : grid_lanes_kernel<NF, NW, unsigned long long>;
     if (smem > 48 * 1024) FR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dim3 grid((unsigned)nitems, (unsigned)P.ngroups);
@@ -1588,6 +1738,12 @@ int launch_taps(fr_plan p, const GridParams &P, long long nitems, long long nspl
 
 }  // namespace
 
+float fixed_sum_limit(int chunk)
+{
+    // 1.9 * 2^30 leaves 107 M for the roundings of the adds, half a unit each
+    return chunk <= 1 << 27 ? 2040109465.f : 1073741824.f;
+}
+
 size_t grid_smem_bytes(long long K, int R, int L)
 {
     // accumulator tile + LUT + double-buffered per-warp tap lists + tap decode
@@ -1631,7 +1787,7 @@ int kspace_prepare(fr_plan p, const float *d_kdata, const float *d_dcf, int chan
                                      (int)trsmem));
     transpose_kspace_kernel<<<(unsigned)((p->n + kTrSamples - 1) / kTrSamples), kTrThreads, trsmem, s>>>(
         reinterpret_cast<const float2 *>(d_kdata), d_dcf, p->kt.as<float2>(), p->kmag.as<float>(), (long long)p->n,
-        channels, cstride, (long long)(kin_stride ? kin_stride : p->n));
+        channels, cstride, (long long)(kin_stride ? kin_stride : p->n), nullptr, nullptr);
     FR_CHECK_LAUNCH("transpose_kspace_kernel");
     p->kt_prepared = d_kdata;
     p->kt_prepared_channels = channels;
@@ -1692,6 +1848,7 @@ int grid_run(fr_plan p, const float *d_kdata, const float *d_dcf, int channels, 
                                                   : "the plan's tap lists overflowed a sample slot (internal error)");
     }
     P.err = p->err_dev;
+    P.sum_limit = fixed_sum_limit(p->chunk);
     // the tap-list scatter reads each record's coil values from the
     // sample-major copy; the geometry scatter uses the copy from 4 coils on
     const bool taps = p->tap_words > 0 && R <= 32;
@@ -1877,6 +2034,15 @@ int batch_launch_t(const GridParams &P, int blocks, long long nsplits, cudaStrea
 }
 }  // namespace
 
+int batch_lane_floats(long long K, int coil_group, int L, int channels)
+{
+    if (channels <= 0 || channels > kTrCoils || (size_t)channels * (kTrSamples + 1) * sizeof(float2) > 96 * 1024) return 0;
+    if (floats_per_cell(coil_group) > 32 || lane_warps(K, L) == 0) return 0;
+    return lane_floats(std::min(channels, coil_group));
+}
+
+int frame_run_samples() { return kTrSamples; }
+
 int batch_grid_setup(int dim, long long K, int coil_group, int L, int *blocks)
 {
     const int R = floats_per_cell(coil_group);
@@ -1928,6 +2094,7 @@ int batch_grid_run(const BatchGrid &b, const float *d_kdata, const float *d_dcf,
     P.kc = b.kc;
     P.lut_absmax = b.lut_absmax;
     P.khalf = 0.25f;
+    P.sum_limit = b.sum_limit;
     P.checkerboard = b.checkerboard;
     P.frame_off = b.frame_off;
     const size_t cells = b.dim == 3 ? (size_t)b.G * b.G * b.G : (size_t)b.G * b.G;
@@ -1939,6 +2106,36 @@ int batch_grid_run(const BatchGrid &b, const float *d_kdata, const float *d_dcf,
     P.skip_empty = 0;
     if (P.nwork == 0) return FR_OK;
     if (P.nwork > 0x7FFFFFFFll) return fail(FR_ERR_UNSUPPORTED, "too many work items");
+    if (b.lane_floats > 0) {
+        const int cstride = channels + (channels & 1);
+        if (b.nruns > 0) {
+            const size_t trsmem = (size_t)channels * (kTrSamples + 1) * sizeof(float2);
+            if (trsmem > 48 * 1024)
+                FR_CUDA(cudaFuncSetAttribute(transpose_kspace_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)trsmem));
+            FR_CUDA(cudaMemsetAsync(b.coil_max, 0, (size_t)b.frames * channels * sizeof(unsigned), s));
+            coil_max_kernel<<<(unsigned)b.nruns, kTrThreads, 0, s>>>(reinterpret_cast<const float2 *>(d_kdata), d_dcf,
+                                                                     b.runs, channels, b.coil_max);
+            FR_CHECK_LAUNCH("coil_max_kernel");
+            transpose_kspace_kernel<<<(unsigned)b.nruns, kTrThreads, trsmem, s>>>(
+                reinterpret_cast<const float2 *>(d_kdata), d_dcf, reinterpret_cast<float2 *>(b.kt), b.kmag, b.n_total,
+                channels, cstride, 0, b.runs, b.coil_max);
+            FR_CHECK_LAUNCH("transpose_kspace_kernel");
+        }
+        P.coil_max = b.coil_max;
+        P.kdata = b.kt;
+        P.mag = b.kmag;
+        P.sample_major = 1;
+        P.kstride = cstride;
+        P.trecs = b.trecs;
+        P.taps = b.taps;
+        P.lutw = b.lutw;
+        P.tap_words = b.tap_words;
+        P.item_inv = b.item_inv;
+        P.err = b.err;
+        P.coil_group = std::min(P.coil_group, b.lane_floats / 2);
+        return launch_lanes(nullptr, P, b.lane_floats, b.nitems, b.nsplits, s);
+    }
     if (b.dim == 3) {
         switch (R) {
         case 8: return batch_launch_t<3, 8>(P, b.blocks, b.nsplits, s);

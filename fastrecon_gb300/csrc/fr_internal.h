@@ -181,6 +181,8 @@ int floats_per_cell(int coil_group);
 // Dynamic shared memory of the scatter kernel for K cells of R floats and an
 // L-entry LUT.
 size_t grid_smem_bytes(long long K, int R, int L);
+// Bound of an item's fixed-point sums for items of at most `chunk` records.
+float fixed_sum_limit(int chunk);
 
 // Exact LUT index without a square root.  The reference index
 //   ki(s) = roundf(fl(fl(sqrtf(s)) / kHW) * (L-1)),  valid iff sqrtf(s) < kHW,
@@ -259,7 +261,17 @@ struct GridInto {
 };
 size_t grid_partials_bytes(long long nslots, int channels, int coil_group, long long K);
 
-// Gridding of a batch of frames in one persistent launch (fr_batch_*).
+// A run of at most frame_run_samples() samples of one frame of a batch.
+struct FrameRun {
+    long long off;  // the frame's first sample among all frames
+    int n;          // the frame's samples
+    int begin;      // first sample of the run in the frame
+    int frame, pad;
+};
+int frame_run_samples();
+
+// Gridding of a batch of frames in one persistent launch (fr_batch_*): from the
+// frames' tap lists (lane_floats > 0), or evaluating the taps.
 struct BatchGrid {
     int dim;
     unsigned G;
@@ -279,9 +291,28 @@ struct BatchGrid {
     float *partials;
     int *work_counter;
     int blocks;                       // persistent CTAs (batch_grid_setup)
+    // tap lists of all frames, concatenated; records name samples of all frames
+    int lane_floats = 0;              // batch_lane_floats, 0: no tap lists
+    int tap_words = 0;
+    const unsigned *taps = nullptr;
+    const unsigned long long *trecs = nullptr;
+    const float *lutw = nullptr;
+    const FrameRun *runs = nullptr;
+    long long nruns = 0;
+    float *kt = nullptr;              // n_total rows of dcf * k, channels rounded up to even
+    float *kmag = nullptr;            // n_total
+    unsigned *coil_max = nullptr;     // frames x channels
+    int frames = 0;
+    float *item_inv = nullptr;        // batch_item_words(nitems)
+    int *err = nullptr;
+    float sum_limit = 1073741824.f;   // fixed_sum_limit
 };
-// Sets the kernel attributes for a configuration and returns how many
-// persistent CTAs fill the GPU.  Call outside stream capture.
+// Coil floats of the tap-lane scatter for a batch; 0 where it cannot be used.
+int batch_lane_floats(long long K, int coil_group, int L, int channels);
+// Words of per-item scratch: the scales, then (from an even word) the bounds.
+inline size_t batch_item_words(long long nitems) { return (((size_t)nitems + 1) & ~(size_t)1) + 2 * (size_t)nitems; }
+// Sets the attributes of the kernel that evaluates the taps for a configuration
+// and returns how many of its CTAs fill the GPU.  Call outside stream capture.
 int batch_grid_setup(int dim, long long K, int coil_group, int L, int *blocks);
 int batch_grid_run(const BatchGrid &b, const float *d_kdata, const float *d_dcf, int channels, float *d_grid,
                    cudaStream_t s);
