@@ -173,7 +173,8 @@ void lut_index_table_into(float hw, int L, float *thr, float *smax, float *kc)
 fr_plan_s::~fr_plan_s()
 {
     for (auto e : prof_ev) cudaEventDestroy(e);
-    if (err_host) cudaFreeHost(err_host);
+    if (counted) cudaEventDestroy(counted);
+    if (head) cudaFreeHost(head);
 }
 
 using namespace fr;
@@ -329,14 +330,17 @@ int fr_plan_create(const fr_plan_desc *d, fr_plan *out)
         delete p;
         return cuda_fail(e, "lut upload");
     }
-    // a word the kernels set on an internal error, read by the host without a copy
-    e = cudaHostAlloc(reinterpret_cast<void **>(&p->err_host), sizeof(int), cudaHostAllocMapped);
-    if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&p->err_dev), p->err_host, 0);
+    // counts, bounds and the word the kernels set on an internal error, read by the host without a copy
+    e = cudaHostAlloc(reinterpret_cast<void **>(&p->head), sizeof(PlanHead), cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&p->head_dev), p->head, 0);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->counted, cudaEventDisableTiming);
     if (e != cudaSuccess) {
         delete p;
-        return cuda_fail(e, "error word");
+        return cuda_fail(e, "plan head");
     }
-    *p->err_host = 0;
+    *p->head = PlanHead{};
+    p->err_host = &p->head->err;
+    p->err_dev = &p->head_dev->err;
     *out = p;
     return FR_OK;
 }

@@ -72,6 +72,14 @@ struct TileScan {
     long long pairs, items, slots, splits, empties;
 };
 
+// What the host reads of a plan before it goes on, in mapped pinned memory.
+struct PlanHead {
+    int err;           // set by kernels on an internal error
+    int pad;
+    TileScan total;
+    float bounds[12];  // norm lo[3], hi[3], raw lo[3], hi[3]
+};
+
 }  // namespace fr
 
 struct fr_plan_s {
@@ -102,7 +110,7 @@ struct fr_plan_s {
     float lut_smax = 0.f, lut_kc = 0.f;
     float lut_absmax = 1.f;   // max |lut[k]| (bounds every tap weight)
     fr::DevBuf traj;          // n float4, normalised
-    fr::DevBuf bounds;        // 16 floats: raw lo/hi as ordered ints, tr, scale, norm lo/hi
+    fr::DevBuf bounds;        // tr, scale, norm and raw bounds, then the partial bounds
     fr::DevBuf tile_count;    // ntiles int
     fr::DevBuf tile_fill;     // ntiles x stripes int (fill cursors)
     fr::DevBuf stripe_count;  // ntiles x stripes int (bin counts per stripe)
@@ -140,8 +148,12 @@ struct fr_plan_s {
     fr::DevBuf item_inv;       // per work item: inverse fixed-point scale, then the items' bounds
     fr::DevBuf sort_tmp;       // deterministic plans: split tiles' records (and tap records) being sorted
     fr::DevBuf sort_buckets;   // deterministic plans: SortBucket table + its count
-    int *err_host = nullptr;   // mapped pinned word the kernels set on an internal error
+    fr::PlanHead *head = nullptr, *head_dev = nullptr;  // mapped pinned; err_host and err_dev point to its error word
+    int *err_host = nullptr;
     int *err_dev = nullptr;
+    // recorded on the planning stream when the trajectory is counted (head is
+    // valid); plan_run waits for it
+    cudaEvent_t counted = nullptr;
 
     // scatter-kernel timing (fr_plan_profile)
     bool profile = false;
@@ -210,7 +222,7 @@ struct PlanInto {
     int tile[3], ntile[3];
     long long ntiles;
     int chunk;
-    int *bounds;  // 32 words
+    int *bounds;              // 32 words
     float4 *traj;
     int *tile_count;          // ntiles
     int *tile_fill;           // ntiles x plan_stripes()
