@@ -168,7 +168,7 @@ int ensure_scratch(fr_batch b, fr_batch_s::Scratch &sc, int channels, int *lane_
     const size_t rows = (size_t)std::max<long long>(b->n_total, 1);
     if (*lane_floats > 0 && (sc.kt.reserve(rows * (size_t)(channels + (channels & 1)) * 8) || sc.kmag.reserve(rows * 4) ||
                              sc.coil_max.reserve((size_t)b->frames * channels * 4) ||
-                             sc.item_inv.reserve(batch_item_words(b->nitems) * 4))) {
+                             sc.item_inv.reserve((size_t)b->nitems * 4))) {
         cudaGetLastError();  // the failed allocation
         *lane_floats = 0;
     }

@@ -1340,60 +1340,85 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) batch_lanes_kernel(GridParam
     }
 }
 
-// Per work item, from the per-sample bounds (mag[s] >= every |dcf * k| of
-// sample s), one warp per item: the sum and the maximum over the item's
-// records with taps.  The sum is exact and independent of the records'
-// order: each bound is rounded up to a multiple of 2^-e (2^e bmax = 2^40..41)
-// and the multiples are added as 64-bit integers; the float result is
-// rounded up.
-__global__ void item_bound_kernel(const WorkItem *__restrict__ items, long long nitems,
-                                  const unsigned long long *__restrict__ trecs, const float *__restrict__ mag,
-                                  float2 *__restrict__ bound)
+// Inverse fixed-point scale of every work item (inv_scale_of), from the
+// per-sample bounds (mag[s] >= every |dcf * k| of sample s): their sum and
+// maximum over the item's records with taps.  The sum is exact and independent of
+// the records' order: each bound is rounded up to a multiple of 2^-e (2^e bmax =
+// 2^40..41) and the multiples are added as 64-bit integers; the float result is
+// rounded up.  Bound by the latency of the gathers, so a CTA per item and
+// kBoundKeep of them in flight per thread, kept in registers for the second pass
+// (items hold 512 records unless a plan is large; longer ones read the rest
+// again).  A warp per item and a second kernel for the scales took 13.6 us for
+// 424 items of 512 records and 14.3 us for 4172 of up to 512, this 4.5 and 7.4.
+constexpr int kBoundThreads = 128, kBoundKeep = 4;
+__global__ void __launch_bounds__(kBoundThreads) item_scale_kernel(const WorkItem *__restrict__ items,
+                                                                   const unsigned long long *__restrict__ trecs,
+                                                                   const float *__restrict__ mag, float lut_absmax,
+                                                                   float sum_limit, float *__restrict__ inv)
 {
-    const long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= nitems) return;
-    const WorkItem it = items[w];
-    float bm = 0.f;
-    for (int j = lane; j < it.count; j += 32) {
-        const unsigned long long rw = trecs[it.begin + j];
-        if ((rw >> 40) & 0xFF) bm = fmaxf(bm, mag[(unsigned)rw]);
+    constexpr int NW = kBoundThreads / 32;
+    __shared__ unsigned wmax[NW];
+    __shared__ unsigned long long wsum[NW];
+    const WorkItem it = items[blockIdx.x];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto load = [&](int j0, float *v) {
+        unsigned long long rw[kBoundKeep];
+#pragma unroll
+        for (int k = 0; k < kBoundKeep; ++k) {
+            const int j = j0 + k * kBoundThreads;
+            rw[k] = j < it.count ? trecs[it.begin + j] : 0ull;
+        }
+#pragma unroll
+        for (int k = 0; k < kBoundKeep; ++k) v[k] = (rw[k] >> 40) & 0xFF ? mag[(unsigned)rw[k]] : 0.f;
+    };
+    float keep[kBoundKeep], bm = 0.f;
+    load(threadIdx.x, keep);
+#pragma unroll
+    for (int k = 0; k < kBoundKeep; ++k) bm = fmaxf(bm, keep[k]);
+    for (int j = threadIdx.x + kBoundKeep * kBoundThreads; j < it.count; j += kBoundKeep * kBoundThreads) {
+        float v[kBoundKeep];
+        load(j, v);
+#pragma unroll
+        for (int k = 0; k < kBoundKeep; ++k) bm = fmaxf(bm, v[k]);
     }
-    bm = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(bm)));  // bounds are >= 0
+    const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(bm));  // bounds are >= 0
+    if (lane == 0) wmax[warp] = wm;
+    __syncthreads();
+    unsigned m = wmax[0];
+#pragma unroll
+    for (int w = 1; w < NW; ++w) m = max(m, wmax[w]);
+    bm = __uint_as_float(m);
     float bs = 0.f;
     if (bm > 0.f) {
         const int e = 40 - ilogbf(bm);
         unsigned long long q = 0;
-        for (int j = lane; j < it.count; j += 32) {
-            const unsigned long long rw = trecs[it.begin + j];
-            if ((rw >> 40) & 0xFF) q += __float2ull_ru(ldexpf(mag[(unsigned)rw], e));
+#pragma unroll
+        for (int k = 0; k < kBoundKeep; ++k) q += __float2ull_ru(ldexpf(keep[k], e));
+        for (int j = threadIdx.x + kBoundKeep * kBoundThreads; j < it.count; j += kBoundKeep * kBoundThreads) {
+            float v[kBoundKeep];
+            load(j, v);
+#pragma unroll
+            for (int k = 0; k < kBoundKeep; ++k) q += __float2ull_ru(ldexpf(v[k], e));
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+        if (lane == 0) wsum[warp] = q;
+        __syncthreads();
+        q = wsum[0];
+#pragma unroll
+        for (int w = 1; w < NW; ++w) q += wsum[w];
         bs = ldexpf(__ull2float_ru(q), -e);
     }
-    if (lane == 0) bound[w] = make_float2(bs, bm);
-}
-
-// Inverse fixed-point scale of every work item from its own bound (see
-// inv_scale_of).
-__global__ void item_inv_kernel(const float2 *__restrict__ bound, long long nitems, float lut_absmax,
-                                float sum_limit, float *__restrict__ inv)
-{
-    for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < nitems;
-         w += (long long)gridDim.x * blockDim.x) {
-        const float2 b = bound[w];
-        inv[w] = inv_scale_of(b.x, __float_as_uint(b.y), lut_absmax, sum_limit);
-    }
+    if (threadIdx.x == 0) inv[blockIdx.x] = inv_scale_of(bs, m, lut_absmax, sum_limit);
 }
 
 // Sum the partial tiles of each split tile in item order and write the grid.
-// CTA (split tile, coil group, part): part z of kReduceParts holds a run of
-// the tile's rows.  The partial rows are read as contiguous float4 ([cell][R]
+// CTA (split tile, coil group, part): part z holds a run of the tile's rows
+// (launch_reduce).  The partial rows are read as contiguous float4 ([cell][R]
 // swizzled, as the scatter wrote them), summed slot after slot (the float
 // order of a plain loop over the items), staged in shared memory, and written
 // as x pairs of one coil per thread, each pair's offset computed once.
-constexpr int kReduceParts = 4, kReduceThreads = 256;
+constexpr int kReduceThreads = 256;
 
 template <int R>
 __global__ void __launch_bounds__(kReduceThreads) reduce_splits_kernel(GridParams P)
@@ -1480,8 +1505,14 @@ template <int R>
 int launch_reduce(const GridParams &P, long long nsplits, cudaStream_t s)
 {
     if (nsplits <= 0) return FR_OK;
+    // Parts of a tile: 4, and up to one float4 a thread while the CTAs do not fill
+    // the GPU: each part sums its slots one after the other, a chain of loads (13
+    // tiles of 32 x 32 x 8 coils: 21 us in 4 parts, 8 in 16; 120 tiles: 15 and 12).
     const int rows = P.tile[1] * P.tile[2];
-    const int parts = rows % kReduceParts == 0 ? kReduceParts : 1;
+    int parts = rows % 4 == 0 ? 4 : 1;
+    while (parts > 1 && rows % (2 * parts) == 0 && nsplits * P.ngroups * parts < 152 * 8 &&
+           (rows / parts) * P.tile[0] * R / 4 > kReduceThreads)
+        parts *= 2;
     const size_t smem = (size_t)(rows / parts) * P.tile[0] * R * sizeof(float);
     if (smem > 48 * 1024)
         FR_CUDA(cudaFuncSetAttribute(reduce_splits_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1634,19 +1665,12 @@ int profile_events(fr_plan p, cudaEvent_t **ev)
     return FR_OK;
 }
 
-// Per-item scales (every launched item, so the indices match blockIdx.x); the
-// bounds go to the scratch past the scales.
+// Per-item scales (every launched item, so the indices match blockIdx.x).
 int launch_item_scales(const GridParams &P, long long nitems, cudaStream_t s)
 {
-    const int threads = 256;
-    const long long blocks = (nitems * 32 + threads - 1) / threads;
-    const long long boff = (nitems + 1) & ~1ll;  // 8-byte aligned float2
-    float2 *bound = reinterpret_cast<float2 *>(const_cast<float *>(P.item_inv) + boff);
-    item_bound_kernel<<<(unsigned)blocks, threads, 0, s>>>(P.items, nitems, P.trecs, P.mag, bound);
-    FR_CHECK_LAUNCH("item_bound_kernel");
-    item_inv_kernel<<<(unsigned)std::min<long long>((nitems + threads - 1) / threads, 152 * 8), threads, 0, s>>>(
-        bound, nitems, P.lut_absmax, P.sum_limit, const_cast<float *>(P.item_inv));
-    FR_CHECK_LAUNCH("item_inv_kernel");
+    item_scale_kernel<<<(unsigned)nitems, kBoundThreads, 0, s>>>(P.items, P.trecs, P.mag, P.lut_absmax, P.sum_limit,
+                                                                 const_cast<float *>(P.item_inv));
+    FR_CHECK_LAUNCH("item_scale_kernel");
     return FR_OK;
 }
 
@@ -1880,9 +1904,7 @@ int grid_run(fr_plan p, const float *d_kdata, const float *d_dcf, int channels, 
         P.taps = p->taps.as<unsigned>();
         P.lutw = p->lut_d.as<float>();
         P.tap_words = p->tap_words;
-        // nlaunch item scales, then (from an even word) nlaunch float2 bounds
-        const size_t words = (((size_t)nlaunch + 1) & ~(size_t)1) + 2 * (size_t)nlaunch;
-        if (p->item_inv.reserve(words * 4)) return FR_ERR_OUT_OF_MEMORY;
+        if (p->item_inv.reserve((size_t)nlaunch * 4)) return FR_ERR_OUT_OF_MEMORY;
         P.item_inv = p->item_inv.as<float>();
         // the tap lanes, except for coil groups of 4 on tiles of up to 512 cells,
         // where the per-warp lists' 32 warps per SM hide more latency than the

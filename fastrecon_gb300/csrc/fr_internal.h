@@ -145,7 +145,7 @@ struct fr_plan_s {
     int tap_layout_words = 0;  // tap_slot_layout of this plan (computed once)
     fr::DevBuf taps;           // n x tap_words words
     fr::DevBuf trecs;          // npairs words, in bin order: sample | first word << 32 | taps << 40
-    fr::DevBuf item_inv;       // per work item: inverse fixed-point scale, then the items' bounds
+    fr::DevBuf item_inv;       // per work item: inverse fixed-point scale
     fr::DevBuf sort_tmp;       // deterministic plans: split tiles' records (and tap records) being sorted
     fr::DevBuf sort_buckets;   // deterministic plans: SortBucket table + its count
     fr::PlanHead *head = nullptr, *head_dev = nullptr;  // mapped pinned; err_host and err_dev point to its error word
@@ -315,14 +315,12 @@ struct BatchGrid {
     float *kmag = nullptr;            // n_total
     unsigned *coil_max = nullptr;     // frames x channels
     int frames = 0;
-    float *item_inv = nullptr;        // batch_item_words(nitems)
+    float *item_inv = nullptr;        // nitems
     int *err = nullptr;
     float sum_limit = 1073741824.f;   // fixed_sum_limit
 };
 // Coil floats of the tap-lane scatter for a batch; 0 where it cannot be used.
 int batch_lane_floats(long long K, int coil_group, int L, int channels);
-// Words of per-item scratch: the scales, then (from an even word) the bounds.
-inline size_t batch_item_words(long long nitems) { return (((size_t)nitems + 1) & ~(size_t)1) + 2 * (size_t)nitems; }
 // Sets the attributes of the kernel that evaluates the taps for a configuration
 // and returns how many of its CTAs fill the GPU.  Call outside stream capture.
 int batch_grid_setup(int dim, long long K, int coil_group, int L, int *blocks);
