@@ -461,16 +461,21 @@ const CtKernels *ct_kernels(int n)
 using FftXRegFn = void (*)(const float2 *, float2 *, long long, int, int, const float2 *, XMask);
 using FftColRegFn = void (*)(const float2 *, float2 *, int, int, int, long long, long long, long long, long long,
                              const float2 *, int, long long, float *, const float *, int, int, long long);
+// Columns per CTA of the 2D y stage: 4 (32-byte rows).  16 / 8 / 4 / 2 columns, a
+// whole 2D reconstruction of 1000 samples: 480^2 to 240^2, 16 coils 111 / 95 /
+// 87 / 83 us; 640^2 to 320^2, 32 coils 286 / 231 / 209 / 223 us; 128^2, 64 coils
+// 104 / 86 / 74 / 70 us; one coil on 64^2 is launch-bound (50 to 52).
+constexpr int kPlaneCols = 4;
 struct RegKernels {
     int n;
     FftXRegFn x;
-    FftColRegFn col, col_sos;
+    FftColRegFn col, col_sos, plane_sos;  // plane_sos: kPlaneCols columns per CTA
     size_t xsmem, colsmem;
     int xthreads, colthreads;
 };
 #define FR_REG(N)                                                                                            \
-    {N, fft_x_kernel_reg<N>, fft_col_kernel_reg<N, false>, fft_col_kernel_reg<N, true>, reg_x_smem<N>(),      \
-     reg_col_smem<N>(), kRegLinesX * RegSplit<N>::TH, kRegCols * RegSplit<N>::TH}
+    {N, fft_x_kernel_reg<N>, fft_col_kernel_reg<N, false>, fft_col_kernel_reg<N, true>,                      \
+     fft_col_kernel_reg<N, true, kPlaneCols>, reg_x_smem<N>(), reg_col_smem<N>(), kRegLinesX * RegSplit<N>::TH, kRegCols * RegSplit<N>::TH}
 const RegKernels kRegKernels[] = {
     FR_REG(64),  FR_REG(128), FR_REG(160), FR_REG(192), FR_REG(240), FR_REG(256), FR_REG(320),
     FR_REG(384), FR_REG(480), FR_REG(512), FR_REG(640),
@@ -624,7 +629,8 @@ int fftcs_execute(fr_fftcs f, const float *d_grid, int channels, const float *d_
             FR_CUDA(cudaFuncSetAttribute(rk->x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk->xsmem));
         if (rk->colsmem > 48 * 1024) {
             FR_CUDA(cudaFuncSetAttribute(rk->col, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk->colsmem));
-            FR_CUDA(cudaFuncSetAttribute(rk->col_sos, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk->colsmem));
+            FR_CUDA(cudaFuncSetAttribute(f->dim == 2 ? rk->plane_sos : rk->col_sos,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk->colsmem));
         }
         XMask xm{};
         if (tiles && tiles->bits) {
@@ -640,7 +646,7 @@ int fftcs_execute(fr_fftcs f, const float *d_grid, int channels, const float *d_
         FR_CHECK_LAUNCH("fft_x_kernel_reg");
         const int cb = (rx + kRegCols - 1) / kRegCols;
         if (f->dim == 2) {
-            rk->col_sos<<<cb, rk->colthreads, rk->colsmem, s>>>(b1, nullptr, y0, ry, rx, rx, 0, 0, rx, tw, C,
+            rk->plane_sos<<<(rx + kPlaneCols - 1) / kPlaneCols, rk->colthreads, rk->colsmem, s>>>(b1, nullptr, y0, ry, rx, rx, 0, 0, rx, tw, C,
                                                             (long long)G * rx, d_out, d_deapod, sos_mode, 1, 1);
             FR_CHECK_LAUNCH("fft_col_kernel_reg(y, sos)");
             return FR_OK;

@@ -238,7 +238,13 @@ __global__ void __launch_bounds__(kRegLinesX * RegSplit<N>::TH) fft_x_kernel_reg
 // to out[outer * out_outer_stride + (k - y0) * out_stride + column]; with it
 // |X|^2 is summed over `coils` in coil order, then sqrt (and / deapod) goes
 // to sos_out at the same offsets.
-template <int N, bool SOS>
+//
+// CC < kRegCols columns per CTA (SOS): the CTA's kRegCols lines are CC columns of
+// kRegCols / CC coils at a time, whose |X|^2 then meet by shuffles, still added
+// in coil order.  For one plane (2D), where 16 columns of one coil after the other
+// leave most of the GPU idle and the coils a serial chain (8 coils, 512^2 to 256^2:
+// 25.7 us, here 12.6; 4 coils, 128^2 to 64^2: 8.4, here 6.0).
+template <int N, bool SOS, int CC = kRegCols>
 __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) fft_col_kernel_reg(
     const float2 *__restrict__ in, float2 *__restrict__ out, int y0, int ry, int ncols, long long stride,
     long long in_outer_stride, long long out_outer_stride, long long out_stride, const float2 *__restrict__ tw_g,
@@ -256,20 +262,26 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
     // runs (whole 16-byte column pairs only).
     float2 *stage = ex + N * CB;
     for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = tw_g[i];
-    const int cblocks = (ncols + CB - 1) / CB;
+    const int cblocks = (ncols + CC - 1) / CC;
     const long long outer0 = SOS ? blockIdx.x / cblocks : (long long)(blockIdx.x / cblocks) * per;
     const long long outer = outer0;  // the SoS outer
-    const int c0 = (blockIdx.x % cblocks) * CB;
-    const int col = threadIdx.x % CB;
+    const int c0 = (blockIdx.x % cblocks) * CC;
+    constexpr int NC = CB / CC;  // coils per unit
+    static_assert(CB % CC == 0 && CC % 2 == 0 && (SOS || NC == 1), "whole coils");
+    const int line = threadIdx.x % CB;  // line of the unit: (coil, column)
+    const int col = line % CC, sub = line / CC;
     const bool col_ok = c0 + col < ncols;
-    const bool pipe = ncols % CB == 0 && ((stride | in_outer_stride | cstride) & 1) == 0 &&
+    const bool pipe = ncols % CC == 0 && ((stride | in_outer_stride | cstride) & 1) == 0 &&
                       (reinterpret_cast<uintptr_t>(in) & 15) == 0;
     auto issue = [&](int unit) {
-        const float2 *src = in + (SOS ? unit * cstride + outer0 * in_outer_stride : (outer0 + unit) * in_outer_stride) + c0;
+        const float2 *src =
+            in + (SOS ? (long long)unit * NC * cstride + outer0 * in_outer_stride : (outer0 + unit) * in_outer_stride) + c0;
         for (int i = threadIdx.x; i < N * CB / 2; i += blockDim.x) {
             const int e = i / (CB / 2), cc = 2 * (i % (CB / 2));
+            if (NC > 1 && unit * NC + cc / CC >= coils) continue;  // read as zero below
             const unsigned dst = (unsigned)__cvta_generic_to_shared(stage + e * CB + cc);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + (long long)e * stride + cc)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
+                         "l"(src + (cc / CC) * cstride + (long long)e * stride + cc % CC)
                          : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -287,10 +299,11 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
             if (k >= y0 && k < y0 + ry) acc[k2] = o[(long long)(k - y0) * out_stride];
         }
     }
-    const int nunit = SOS ? coils : (int)min((long long)per, nouter - outer0);
+    const int nunit = SOS ? (coils + NC - 1) / NC : (int)min((long long)per, nouter - outer0);
     if (pipe) issue(0);
     for (int u = 0; u < nunit; ++u) {
-        const int coil = SOS ? u : 0;
+        const int coil = SOS ? u * NC + sub : 0;
+        const bool line_ok = col_ok && (NC == 1 || coil < coils);
         const long long ou = SOS ? outer0 : outer0 + u;
         if (pipe) asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();  // twiddles staged; the previous unit's exchange is read; this unit's block landed
@@ -299,14 +312,15 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
             float2 v[M];
             if (pipe) {
 #pragma unroll
-                for (int m = 0; m < M; ++m) v[m] = stage[(t + T * m) * CB + col];
+                for (int m = 0; m < M; ++m)
+                    v[m] = NC == 1 || line_ok ? stage[(t + T * m) * CB + line] : make_float2(0.f, 0.f);
             } else {
                 const float2 *src = in + coil * cstride + ou * in_outer_stride + (long long)t * stride + c0 + col;
 #pragma unroll
-                for (int m = 0; m < M; ++m) v[m] = col_ok ? src[(long long)(T * m) * stride] : make_float2(0.f, 0.f);
+                for (int m = 0; m < M; ++m) v[m] = line_ok ? src[(long long)(T * m) * stride] : make_float2(0.f, 0.f);
             }
             rdft<M>(v);
-            float2 *dst = ex + t * CB + col;
+            float2 *dst = ex + t * CB + line;
             dst[0] = v[0];
 #pragma unroll
             for (int k1 = 1; k1 < M; ++k1) dst[k1 * T * CB] = cmul(v[k1], tw[t * k1]);
@@ -316,11 +330,21 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
         if (threadIdx.x < CB * M) {
             const int k1 = threadIdx.x / CB;
             float2 b[T];
-            const float2 *src = ex + k1 * T * CB + col;
+            const float2 *src = ex + k1 * T * CB + line;
 #pragma unroll
             for (int t = 0; t < T; ++t) b[t] = src[t * CB];
             rdft<T>(b);
-            if constexpr (SOS) {
+            if constexpr (SOS && NC > 1) {
+                // step B's threads are whole half-warps: a half-warp's 16 lines are one k1
+                const unsigned live = (threadIdx.x | 31) < CB * M ? 0xffffffffu : 0xffffu;
+#pragma unroll
+                for (int k2 = 0; k2 < T; ++k2) {
+                    const float q = __fsub_rn(__fmul_rn(b[k2].x, b[k2].x), __fmul_rn(b[k2].y, -b[k2].y));
+                    acc[k2] = __fadd_rn(acc[k2], q);  // sums of the first coil's lanes are kept
+#pragma unroll
+                    for (int c = 1; c < NC; ++c) acc[k2] = __fadd_rn(acc[k2], __shfl_down_sync(live, q, c * CC, CB));
+                }
+            } else if constexpr (SOS) {
 #pragma unroll
                 for (int k2 = 0; k2 < T; ++k2)
                     // x * conj(x) of the reference's SOS: re*re - im*(-im)
@@ -335,7 +359,7 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
             }
         }
     }
-    if (SOS && threadIdx.x < CB * M && col_ok) {
+    if (SOS && threadIdx.x < CB * M && col_ok && sub == 0) {
         const int k1 = threadIdx.x / CB;
         float *o = sos_out + outer * out_outer_stride + c0 + col;
         const float *dp = deapod ? deapod + outer * out_outer_stride + c0 + col : nullptr;
