@@ -90,3 +90,23 @@ def test_batch_weak_and_broken_coils(oracle):
     k[1, 100] = np.inf
     bad = grid(k)
     assert all(rel_l2(bad[c], want[c]) <= bound[c] for c in (0, 2, 3, 4))
+
+
+@pytest.mark.gpu
+def test_batch_quiet_runs(oracle):
+    """A coil that is all but silent in every fourth run of 128 samples, the
+    first among them, is gridded like the others."""
+    import torch
+
+    from fastrecon_gb300 import batch as fb
+    t = synth.radial_2d(32, 64)
+    rng = np.random.default_rng(6)
+    k = (rng.standard_normal((3, t.shape[0])) + 1j * rng.standard_normal((3, t.shape[0]))).astype(np.complex64)
+    k[1, (np.arange(t.shape[0]) // 128) % 4 == 0] *= np.float32(1e-37)
+    dcf = rng.uniform(0.2, 1.0, t.shape[0]).astype(np.float32)
+    lut = oracle.kb_lut(4.0, 2.0, 512)
+    b = fb.GridBatch(2, 64, 4.0, lut=lut)
+    b.set_trajectories(torch.from_numpy(t).cuda(), [t.shape[0]])
+    got = b.grid(torch.from_numpy(k.ravel()).cuda(), torch.from_numpy(dcf).cuda(), 3).cpu().numpy()[0]
+    want = oracle.grid(oracle.normalize_traj(t, 2, 64)[0], dcf, k, 2, 64, 4.0, lut, threads=4)
+    assert all(rel_l2(got[c], want[c]) <= TOL for c in range(3))
