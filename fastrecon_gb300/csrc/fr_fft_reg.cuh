@@ -163,7 +163,24 @@ struct XMask {
     const unsigned *bits;
     int sx, sy, sz, ntx, nty, G, Gz;
     FastDiv by_g, by_gz;  // line -> (y, z) without divisions
+    // 3D: the x stage leaves lines that cross no written tile out, and the y
+    // stage takes them as zero
+    int rows;
 };
+
+// Tile row (ty, tz) has a written tile.
+__device__ __forceinline__ bool xmask_row(const XMask &xm, int ty, int tz)
+{
+    const int b0 = (tz * xm.nty + ty) * xm.ntx, b1 = b0 + xm.ntx - 1;  // its first and last bit
+    unsigned any = 0u;
+    for (int w = b0 >> 5; w <= b1 >> 5; ++w) {
+        unsigned m = xm.bits[w];
+        if (w == b0 >> 5) m &= 0xffffffffu << (b0 & 31);
+        if (w == b1 >> 5) m &= 0xffffffffu >> (31 - (b1 & 31));
+        any |= m;
+    }
+    return any != 0u;
+}
 
 // x stage: kRegLinesX contiguous lines of length N per CTA, outputs
 // [x0, x0 + rx) of each line.  in: nlines x N, out: nlines x rx.
@@ -181,11 +198,12 @@ __global__ void __launch_bounds__(kRegLinesX * RegSplit<N>::TH) fft_x_kernel_reg
     float2 *ex = tw + N;
     for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = tw_g[(i % T) * (i / T)];
     const long long l0 = (long long)blockIdx.x * kRegLinesX;
-    __syncthreads();
-    if (threadIdx.x < kRegLinesX * T) {
-        const int l = threadIdx.x / T, t = threadIdx.x % T;
+    const int l = threadIdx.x / T, t = threadIdx.x % T;
+    const bool step_a = threadIdx.x < kRegLinesX * T;
+    bool some = !xm.rows;  // this thread's cells are in a written tile
+    float2 v[M];
+    if (step_a) {
         const long long line = l0 + l;
-        float2 v[M];
         if (line < nlines && xm.bits) {
             // nlines = coils * Gz * G < 2^31 (checked by the caller)
             const unsigned yz = xm.by_g.div((unsigned)line), cz = xm.by_gz.div(yz);
@@ -195,7 +213,9 @@ __global__ void __launch_bounds__(kRegLinesX * RegSplit<N>::TH) fft_x_kernel_reg
 #pragma unroll
             for (int m = 0; m < M; ++m) {
                 const int tile = tb + ((t + T * m) >> xm.sx);
-                v[m] = (xm.bits[tile >> 5] >> (tile & 31)) & 1u ? src[T * m] : make_float2(0.f, 0.f);
+                const bool on = (xm.bits[tile >> 5] >> (tile & 31)) & 1u;
+                v[m] = on ? src[T * m] : make_float2(0.f, 0.f);
+                some = some || on;
             }
         } else if (line < nlines) {
             const float2 *src = in + line * N + t;
@@ -205,6 +225,10 @@ __global__ void __launch_bounds__(kRegLinesX * RegSplit<N>::TH) fft_x_kernel_reg
 #pragma unroll
             for (int m = 0; m < M; ++m) v[m] = make_float2(0.f, 0.f);
         }
+    }
+    // twiddles staged (the lines' loads are under way); lines without a written tile are done
+    if (!__syncthreads_or(some)) return;
+    if (step_a) {
         rdft<M>(v);
         float2 *dst = ex + l * LS + t;
         dst[0] = v[0];
@@ -249,7 +273,7 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
     const float2 *__restrict__ in, float2 *__restrict__ out, int y0, int ry, int ncols, long long stride,
     long long in_outer_stride, long long out_outer_stride, long long out_stride, const float2 *__restrict__ tw_g,
     int coils, long long cstride, float *__restrict__ sos_out, const float *__restrict__ deapod, int sos_mode,
-    int per, long long nouter)
+    int per, long long nouter, XMask xm)
 {
     constexpr int T = RegSplit<N>::T, M = RegSplit<N>::M;
     constexpr int CB = kRegCols;
@@ -273,6 +297,15 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
     const bool col_ok = c0 + col < ncols;
     const bool pipe = ncols % CC == 0 && ((stride | in_outer_stride | cstride) & 1) == 0 &&
                       (reinterpret_cast<uintptr_t>(in) & 15) == 0;
+    // y stage with a tile mask: the lines of a unit's plane that the x stage left
+    // out are zero (flags of this unit and the next, by tile row)
+    __shared__ unsigned char row_on[SOS ? 1 : 2][SOS ? 1 : N];
+    const bool rows = !SOS && xm.rows;
+    auto flag_rows = [&](int unit) {
+        const int tz = (int)((outer0 + unit) % xm.Gz) >> xm.sz;
+        for (int i = blockDim.x - 1 - threadIdx.x; i < xm.nty; i += blockDim.x) row_on[SOS ? 0 : unit & 1][SOS ? 0 : i] = xmask_row(xm, i, tz);
+    };
+    auto row_zero = [&](int unit, int e) { return rows && !row_on[SOS ? 0 : unit & 1][SOS ? 0 : e >> xm.sy]; };
     auto issue = [&](int unit) {
         const float2 *src =
             in + (SOS ? (long long)unit * NC * cstride + outer0 * in_outer_stride : (outer0 + unit) * in_outer_stride) + c0;
@@ -280,9 +313,14 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
             const int e = i / (CB / 2), cc = 2 * (i % (CB / 2));
             if (NC > 1 && unit * NC + cc / CC >= coils) continue;  // read as zero below
             const unsigned dst = (unsigned)__cvta_generic_to_shared(stage + e * CB + cc);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
-                         "l"(src + (cc / CC) * cstride + (long long)e * stride + cc % CC)
-                         : "memory");
+            if constexpr (SOS)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
+                             "l"(src + (cc / CC) * cstride + (long long)e * stride + cc % CC)
+                             : "memory");
+            else  // of a zero line nothing is read, zeros are written
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst),
+                             "l"(src + (long long)e * stride + cc), "r"(row_zero(unit, e) ? 0 : 16)
+                             : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -300,6 +338,10 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
         }
     }
     const int nunit = SOS ? (coils + NC - 1) / NC : (int)min((long long)per, nouter - outer0);
+    if (rows) {
+        flag_rows(0);
+        __syncthreads();
+    }
     if (pipe) issue(0);
     for (int u = 0; u < nunit; ++u) {
         const int coil = SOS ? u * NC + sub : 0;
@@ -317,7 +359,8 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
             } else {
                 const float2 *src = in + coil * cstride + ou * in_outer_stride + (long long)t * stride + c0 + col;
 #pragma unroll
-                for (int m = 0; m < M; ++m) v[m] = line_ok ? src[(long long)(T * m) * stride] : make_float2(0.f, 0.f);
+                for (int m = 0; m < M; ++m)
+                    v[m] = line_ok && !row_zero(u, t + T * m) ? src[(long long)(T * m) * stride] : make_float2(0.f, 0.f);
             }
             rdft<M>(v);
             float2 *dst = ex + t * CB + line;
@@ -325,6 +368,7 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
 #pragma unroll
             for (int k1 = 1; k1 < M; ++k1) dst[k1 * T * CB] = cmul(v[k1], tw[t * k1]);
         }
+        if (rows && u + 1 < nunit) flag_rows(u + 1);
         __syncthreads();
         if (pipe && u + 1 < nunit) issue(u + 1);  // the block is free: every thread passed step A
         if (threadIdx.x < CB * M) {
