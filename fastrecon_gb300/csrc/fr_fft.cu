@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 #include <cufft.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <new>
@@ -458,6 +459,14 @@ const CtKernels *ct_kernels(int n)
 }
 
 // Register two-step stages (fr_fft_reg.cuh) for the specialised sizes.
+int sm_count()
+{
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        n = 148;
+    return n;
+}
+
 using FftXRegFn = void (*)(const float2 *, float2 *, long long, int, int, const float2 *, XMask);
 using FftColRegFn = void (*)(const float2 *, float2 *, int, int, int, long long, long long, long long, long long,
                              const float2 *, int, long long, float *, const float *, int, int, long long, XMask);
@@ -470,12 +479,23 @@ struct RegKernels {
     int n;
     FftXRegFn x;
     FftColRegFn col, col_sos, plane_sos;  // plane_sos: kPlaneCols columns per CTA
-    size_t xsmem, colsmem;
-    int xthreads, colthreads;
+    size_t (*xsmem)(int);  // of a warp count
+    size_t colsmem;
+    int xwarps, xthreads;  // most warps per CTA of the x stage by warps, or (0) threads of the one by CTAs
+    int colthreads;
 };
-#define FR_REG(N)                                                                                            \
-    {N, fft_x_kernel_reg<N>, fft_col_kernel_reg<N, false>, fft_col_kernel_reg<N, true>,                      \
-     fft_col_kernel_reg<N, true, kPlaneCols>, reg_x_smem<N>(), reg_col_smem<N>(), kRegLinesX * RegSplit<N>::TH, kRegCols * RegSplit<N>::TH}
+template <int N>
+constexpr FftXRegFn reg_x_kernel()
+{
+    if constexpr (kXWarps<N> > 0)
+        return fft_x_warps_kernel<N>;
+    else
+        return fft_x_kernel_reg<N>;
+}
+#define FR_REG(N)                                                                                                \
+    {N, reg_x_kernel<N>(), fft_col_kernel_reg<N, false>, fft_col_kernel_reg<N, true>,                            \
+     fft_col_kernel_reg<N, true, kPlaneCols>, reg_x_smem<N>, reg_col_smem<N>(), kXWarps<N>,                      \
+     kRegLinesX * RegSplit<N>::TH, kRegCols * RegSplit<N>::TH}
 const RegKernels kRegKernels[] = {
     FR_REG(64),  FR_REG(128), FR_REG(160), FR_REG(192), FR_REG(240), FR_REG(256), FR_REG(320),
     FR_REG(384), FR_REG(480), FR_REG(512), FR_REG(640),
@@ -625,8 +645,20 @@ int fftcs_execute(fr_fftcs f, const float *d_grid, int channels, const float *d_
     const long long nl = (long long)C * Gz * G;
     if (const RegKernels *rk = f->reg) {
         // register two-step stages: x (cropped), y (cropped), z or y with SoS
-        if (rk->xsmem > 48 * 1024)
-            FR_CUDA(cudaFuncSetAttribute(rk->x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk->xsmem));
+        // the x stage by warps: fewer warps per CTA where the pairs of lines would not reach all SMs
+        const int sms = sm_count();
+        const long long npairs = (nl + 1) / 2;
+        const int xw = rk->xwarps == 0 ? 0 : (int)std::min<long long>(rk->xwarps, std::max<long long>(2, npairs / sms));
+        const int xthreads = xw > 0 ? xw * 32 : rk->xthreads;
+        const size_t xsmem = rk->xsmem(xw);
+        if (xsmem > 48 * 1024)
+            FR_CUDA(cudaFuncSetAttribute(rk->x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xsmem));
+        long long xblocks = (nl + kRegLinesX - 1) / kRegLinesX;
+        if (xw > 0) {
+            int per_sm = 0;
+            FR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rk->x, xthreads, xsmem));
+            xblocks = std::min<long long>((npairs + xw - 1) / xw, (long long)std::max(per_sm, 1) * sms);
+        }
         if (rk->colsmem > 48 * 1024) {
             FR_CUDA(cudaFuncSetAttribute(rk->col, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk->colsmem));
             FR_CUDA(cudaFuncSetAttribute(f->dim == 2 ? rk->plane_sos : rk->col_sos,
@@ -641,8 +673,7 @@ int fftcs_execute(fr_fftcs f, const float *d_grid, int channels, const float *d_
                 return fail(FR_ERR_UNSUPPORTED, "tile masks need power-of-two tile edges");
             if (nl >= (1ll << 31)) return fail(FR_ERR_UNSUPPORTED, "more than 2^31 lines in a tile-masked transform");
         }
-        rk->x<<<(unsigned)((nl + kRegLinesX - 1) / kRegLinesX), rk->xthreads, rk->xsmem, s>>>(grid, b1, nl, x0, rx, tw,
-                                                                                          xm);
+        rk->x<<<(unsigned)xblocks, xthreads, xsmem, s>>>(grid, b1, nl, x0, rx, tw, xm);
         FR_CHECK_LAUNCH("fft_x_kernel_reg");
         const int cb = (rx + kRegCols - 1) / kRegCols;
         if (f->dim == 2) {

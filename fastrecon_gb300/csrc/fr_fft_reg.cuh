@@ -255,6 +255,114 @@ __global__ void __launch_bounds__(kRegLinesX * RegSplit<N>::TH) fft_x_kernel_reg
     }
 }
 
+// The x stage for lines of 240 and more: as above, but every warp takes its own
+// pairs of lines, so that no barrier of the CTA makes its warps wait for each
+// other's loads (nor a third of them idle in step A): step A 16 lanes a line, step B
+// the pair's 2 M transforms of 16 points 32 at a time.  Warps are persistent and
+// load their next pair while step B runs; a pair without a written tile costs its
+// mask bits only.  Bound: HBM with every cell read (16 coils, 384^3: 6.6 TB/s), else
+// the latency of the loads at 16 warps per SM.  x stage alone, cells of a ball, per
+// CTA / per warp: 8 coils, 240^3 195 / 184 us; 16 coils, 384^3 1540 / 1374; 4 coils,
+// 480^3 1194 / 667 and 512^3 1132 / 796; 2 coils, 640^3 2138 / 1200; but 16 coils,
+// 192^3 198 / 200 and 128^3 68 / 74, where the 128 threads of a CTA all work in
+// both steps and ten CTAs fit on an SM.
+template <int N>
+constexpr int kXWarps = N <= 192 ? 0 : N <= 256 ? 4 : 8;  // most warps per CTA; 0: fft_x_kernel_reg
+
+template <int N>
+__global__ void __launch_bounds__(kXWarps<N> * 32, N <= 256 ? 5 : 2) fft_x_warps_kernel(
+    const float2 *__restrict__ in, float2 *__restrict__ out, long long nlines, int x0, int rx,
+    const float2 *__restrict__ tw_g, XMask xm)
+{
+    constexpr int T = 16, M = N / T;
+    constexpr int LS = M * (T + 1);  // [k1][t] with one pad slot per row
+    static_assert(RegSplit<N>::T == T, "16 x M");
+    extern __shared__ float2 sm[];
+    float2 *tw = sm;  // [k1][t] as above
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    float2 *ex = tw + N + warp * (2 * LS);
+    for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = tw_g[(i % T) * (i / T)];
+    const int l = lane / T, t = lane % T;
+    const long long npairs = (nlines + 1) / 2;
+    float2 v[M];
+    // false: all cells of the pair are in tiles without samples
+    auto load = [&](long long pair) -> bool {
+        const long long line = pair * 2 + l;
+        const float2 *src = in + line * N + t;
+        bool some = !xm.rows;
+        if (line >= nlines) {
+#pragma unroll
+            for (int m = 0; m < M; ++m) v[m] = make_float2(0.f, 0.f);
+        } else if (xm.bits) {
+            const unsigned yz = xm.by_g.div((unsigned)line), cz = xm.by_gz.div(yz);
+            const int y = (int)((unsigned)line - yz * (unsigned)xm.G), z = (int)(yz - cz * (unsigned)xm.Gz);
+            const int tb = ((z >> xm.sz) * xm.nty + (y >> xm.sy)) * xm.ntx;
+            if (N <= 512 && xm.sx == 3) {
+                // the row's N / 8 bits at once: lane t's cells are in tiles t / 8 + 2 m
+                const int w0 = tb >> 5, w1 = (tb + N / 8 - 1) >> 5, sh = tb & 31;
+                const unsigned a = xm.bits[w0], b = xm.bits[min(w0 + 1, w1)], c = xm.bits[min(w0 + 2, w1)];
+                unsigned lo = __funnelshift_r(a, b, sh), hi = __funnelshift_r(b, c, sh);
+                lo = __funnelshift_r(lo, hi, t >> 3);
+                hi >>= t >> 3;
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    const bool on = ((m < 16 ? lo : hi) >> (2 * m & 31)) & 1u;
+                    v[m] = on ? src[T * m] : make_float2(0.f, 0.f);
+                    some = some || on;
+                }
+            } else {
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    const int tile = tb + ((t + T * m) >> xm.sx);
+                    const bool on = (xm.bits[tile >> 5] >> (tile & 31)) & 1u;
+                    v[m] = on ? src[T * m] : make_float2(0.f, 0.f);
+                    some = some || on;
+                }
+            }
+        } else {
+#pragma unroll
+            for (int m = 0; m < M; ++m) v[m] = src[T * m];
+        }
+        return __any_sync(0xffffffffu, some);
+    };
+    const long long step = (long long)gridDim.x * nwarps;
+    long long pair = blockIdx.x * (long long)nwarps + warp;
+    bool some = pair < npairs && load(pair);
+    __syncthreads();  // twiddles staged
+    while (pair < npairs) {
+        const long long cur = pair;
+        const bool done = some;
+        if (done) {
+            rdft<M>(v);
+            float2 *dst = ex + l * LS + t;
+            dst[0] = v[0];
+#pragma unroll
+            for (int k1 = 1; k1 < M; ++k1) dst[k1 * (T + 1)] = cmul(v[k1], tw[k1 * T + t]);
+        }
+        __syncwarp();
+        pair += step;
+        some = pair < npairs && load(pair);
+        if (done) {
+#pragma unroll 1
+            for (int i = lane; i < 2 * M; i += 32) {
+                const int lb = i / M, k1 = i - lb * M;
+                const long long line = cur * 2 + lb;
+                if (line >= nlines) continue;
+                float2 b[T];
+                const float2 *src = ex + lb * LS + k1 * (T + 1);
+#pragma unroll
+                for (int q = 0; q < T; ++q) b[q] = src[q];
+                rdft<T>(b);
+                float2 *o = out + line * rx + (k1 - x0);
+#pragma unroll
+                for (int k2 = 0; k2 < T; ++k2)
+                    if ((unsigned)(k1 - x0 + M * k2) < (unsigned)rx) o[M * k2] = b[k2];
+            }
+        }
+        __syncwarp();  // the exchange is read
+    }
+}
+
 // Column stage: for each (outer, block of kRegCols columns) transform the
 // lines along an axis of length N with element stride `stride`, keep outputs
 // [y0, y0 + ry).  Input index: coil * cstride + outer * in_outer_stride +
@@ -422,10 +530,12 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
     }
 }
 
+// Shared memory of the x stage for `warps` warps per CTA (0: fft_x_kernel_reg).
 template <int N>
-constexpr size_t reg_x_smem()
+constexpr size_t reg_x_smem(int warps)
 {
-    return (size_t)(N + kRegLinesX * RegSplit<N>::M * (RegSplit<N>::T + 1)) * sizeof(float2);
+    constexpr int LS = RegSplit<N>::M * (RegSplit<N>::T + 1);
+    return (size_t)(N + (warps > 0 ? 2 * warps : kRegLinesX) * LS) * sizeof(float2);
 }
 // twiddles, exchange buffer and the next unit's input block
 template <int N>
