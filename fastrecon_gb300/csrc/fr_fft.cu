@@ -469,7 +469,7 @@ int sm_count()
 
 using FftXRegFn = void (*)(const float2 *, float2 *, long long, int, int, const float2 *, XMask);
 using FftColRegFn = void (*)(const float2 *, float2 *, int, int, int, long long, long long, long long, long long,
-                             const float2 *, int, long long, float *, const float *, int, int, long long, XMask);
+                             const float2 *, int, long long, float *, const float *, int, int, long long);
 // Columns per CTA of the 2D y stage: 4 (32-byte rows).  16 / 8 / 4 / 2 columns, a
 // whole 2D reconstruction of 1000 samples: 480^2 to 240^2, 16 coils 111 / 95 /
 // 87 / 83 us; 640^2 to 320^2, 32 coils 286 / 231 / 209 / 223 us; 128^2, 64 coils
@@ -668,7 +668,7 @@ int fftcs_execute(fr_fftcs f, const float *d_grid, int channels, const float *d_
         if (tiles && tiles->bits) {
             auto lg = [](int v) { return (v & (v - 1)) == 0 ? __builtin_ctz((unsigned)v) : -1; };
             xm = XMask{tiles->bits, lg(tiles->tile[0]), lg(tiles->tile[1]), lg(tiles->tile[2]), tiles->ntile[0],
-                       tiles->ntile[1], G, (int)Gz, FastDiv((unsigned)G), FastDiv((unsigned)Gz), f->dim == 3};
+                       tiles->ntile[1], G, (int)Gz, FastDiv((unsigned)G), FastDiv((unsigned)Gz)};
             if (xm.sx < 0 || xm.sy < 0 || xm.sz < 0)
                 return fail(FR_ERR_UNSUPPORTED, "tile masks need power-of-two tile edges");
             if (nl >= (1ll << 31)) return fail(FR_ERR_UNSUPPORTED, "more than 2^31 lines in a tile-masked transform");
@@ -678,7 +678,7 @@ int fftcs_execute(fr_fftcs f, const float *d_grid, int channels, const float *d_
         const int cb = (rx + kRegCols - 1) / kRegCols;
         if (f->dim == 2) {
             rk->plane_sos<<<(rx + kPlaneCols - 1) / kPlaneCols, rk->colthreads, rk->colsmem, s>>>(b1, nullptr, y0, ry, rx, rx, 0, 0, rx, tw, C,
-                                                            (long long)G * rx, d_out, d_deapod, sos_mode, 1, 1, XMask{});
+                                                            (long long)G * rx, d_out, d_deapod, sos_mode, 1, 1);
             FR_CHECK_LAUNCH("fft_col_kernel_reg(y, sos)");
             return FR_OK;
         }
@@ -687,11 +687,11 @@ int fftcs_execute(fr_fftcs f, const float *d_grid, int channels, const float *d_
         const long long nouter = (long long)C * G;
         rk->col<<<(unsigned)((nouter + kColPer - 1) / kColPer * cb), rk->colthreads, rk->colsmem, s>>>(
             b1, b2, y0, ry, rx, rx, (long long)G * rx, (long long)ry * rx, rx, tw, 1, 0, nullptr, nullptr, 0, kColPer,
-            nouter, xm);
+            nouter);
         FR_CHECK_LAUNCH("fft_col_kernel_reg(y)");
         rk->col_sos<<<(unsigned)((long long)ry * cb), rk->colthreads, rk->colsmem, s>>>(
             b2, nullptr, z0, rz, rx, (long long)ry * rx, rx, rx, (long long)ry * rx, tw, C, (long long)G * ry * rx, d_out,
-            d_deapod, sos_mode, 1, ry, XMask{});
+            d_deapod, sos_mode, 1, ry);
         FR_CHECK_LAUNCH("fft_col_kernel_reg(z, sos)");
         return FR_OK;
     }

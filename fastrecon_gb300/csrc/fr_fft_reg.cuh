@@ -163,23 +163,13 @@ struct XMask {
     const unsigned *bits;
     int sx, sy, sz, ntx, nty, G, Gz;
     FastDiv by_g, by_gz;  // line -> (y, z) without divisions
-    // 3D: the x stage leaves lines that cross no written tile out, and the y
-    // stage takes them as zero
-    int rows;
 };
 
-// Tile row (ty, tz) has a written tile.
-__device__ __forceinline__ bool xmask_row(const XMask &xm, int ty, int tz)
+// The zeros of lines [line, end) that cross no written tile, by `threads` threads.
+__device__ __forceinline__ void zero_lines(float2 *out, long long line, long long end, int rx, int thread, int threads)
 {
-    const int b0 = (tz * xm.nty + ty) * xm.ntx, b1 = b0 + xm.ntx - 1;  // its first and last bit
-    unsigned any = 0u;
-    for (int w = b0 >> 5; w <= b1 >> 5; ++w) {
-        unsigned m = xm.bits[w];
-        if (w == b0 >> 5) m &= 0xffffffffu << (b0 & 31);
-        if (w == b1 >> 5) m &= 0xffffffffu >> (31 - (b1 & 31));
-        any |= m;
-    }
-    return any != 0u;
+    const int n = (int)(end - line) * rx;
+    for (int i = thread; i < n; i += threads) out[line * rx + i] = make_float2(0.f, 0.f);
 }
 
 // x stage: kRegLinesX contiguous lines of length N per CTA, outputs
@@ -200,7 +190,7 @@ __global__ void __launch_bounds__(kRegLinesX * RegSplit<N>::TH) fft_x_kernel_reg
     const long long l0 = (long long)blockIdx.x * kRegLinesX;
     const int l = threadIdx.x / T, t = threadIdx.x % T;
     const bool step_a = threadIdx.x < kRegLinesX * T;
-    bool some = !xm.rows;  // this thread's cells are in a written tile
+    bool some = !xm.bits;  // one of this thread's cells is in a written tile
     float2 v[M];
     if (step_a) {
         const long long line = l0 + l;
@@ -226,8 +216,8 @@ __global__ void __launch_bounds__(kRegLinesX * RegSplit<N>::TH) fft_x_kernel_reg
             for (int m = 0; m < M; ++m) v[m] = make_float2(0.f, 0.f);
         }
     }
-    // twiddles staged (the lines' loads are under way); lines without a written tile are done
-    if (!__syncthreads_or(some)) return;
+    // twiddles staged (the lines' loads are under way)
+    if (!__syncthreads_or(some)) return zero_lines(out, l0, min(l0 + kRegLinesX, nlines), rx, threadIdx.x, blockDim.x);
     if (step_a) {
         rdft<M>(v);
         float2 *dst = ex + l * LS + t;
@@ -260,7 +250,7 @@ __global__ void __launch_bounds__(kRegLinesX * RegSplit<N>::TH) fft_x_kernel_reg
 // other's loads (nor a third of them idle in step A): step A 16 lanes a line, step B
 // the pair's 2 M transforms of 16 points 32 at a time.  Warps are persistent and
 // load their next pair while step B runs; a pair without a written tile costs its
-// mask bits only.  Bound: HBM with every cell read (16 coils, 384^3: 6.6 TB/s), else
+// mask bits and zeros only.  Bound: HBM with every cell read (16 coils, 384^3: 6.6 TB/s), else
 // the latency of the loads at 16 warps per SM.  x stage alone, cells of a ball, per
 // CTA / per warp: 8 coils, 240^3 195 / 184 us; 16 coils, 384^3 1540 / 1374; 4 coils,
 // 480^3 1194 / 667 and 512^3 1132 / 796; 2 coils, 640^3 2138 / 1200; but 16 coils,
@@ -289,7 +279,7 @@ __global__ void __launch_bounds__(kXWarps<N> * 32, N <= 256 ? 5 : 2) fft_x_warps
     auto load = [&](long long pair) -> bool {
         const long long line = pair * 2 + l;
         const float2 *src = in + line * N + t;
-        bool some = !xm.rows;
+        bool some = !xm.bits;
         if (line >= nlines) {
 #pragma unroll
             for (int m = 0; m < M; ++m) v[m] = make_float2(0.f, 0.f);
@@ -358,6 +348,8 @@ __global__ void __launch_bounds__(kXWarps<N> * 32, N <= 256 ? 5 : 2) fft_x_warps
                 for (int k2 = 0; k2 < T; ++k2)
                     if ((unsigned)(k1 - x0 + M * k2) < (unsigned)rx) o[M * k2] = b[k2];
             }
+        } else {
+            zero_lines(out, cur * 2, min(cur * 2 + 2, nlines), rx, lane, 32);
         }
         __syncwarp();  // the exchange is read
     }
@@ -381,7 +373,7 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
     const float2 *__restrict__ in, float2 *__restrict__ out, int y0, int ry, int ncols, long long stride,
     long long in_outer_stride, long long out_outer_stride, long long out_stride, const float2 *__restrict__ tw_g,
     int coils, long long cstride, float *__restrict__ sos_out, const float *__restrict__ deapod, int sos_mode,
-    int per, long long nouter, XMask xm)
+    int per, long long nouter)
 {
     constexpr int T = RegSplit<N>::T, M = RegSplit<N>::M;
     constexpr int CB = kRegCols;
@@ -405,15 +397,6 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
     const bool col_ok = c0 + col < ncols;
     const bool pipe = ncols % CC == 0 && ((stride | in_outer_stride | cstride) & 1) == 0 &&
                       (reinterpret_cast<uintptr_t>(in) & 15) == 0;
-    // y stage with a tile mask: the lines of a unit's plane that the x stage left
-    // out are zero (flags of this unit and the next, by tile row)
-    __shared__ unsigned char row_on[SOS ? 1 : 2][SOS ? 1 : N];
-    const bool rows = !SOS && xm.rows;
-    auto flag_rows = [&](int unit) {
-        const int tz = (int)((outer0 + unit) % xm.Gz) >> xm.sz;
-        for (int i = blockDim.x - 1 - threadIdx.x; i < xm.nty; i += blockDim.x) row_on[SOS ? 0 : unit & 1][SOS ? 0 : i] = xmask_row(xm, i, tz);
-    };
-    auto row_zero = [&](int unit, int e) { return rows && !row_on[SOS ? 0 : unit & 1][SOS ? 0 : e >> xm.sy]; };
     auto issue = [&](int unit) {
         const float2 *src =
             in + (SOS ? (long long)unit * NC * cstride + outer0 * in_outer_stride : (outer0 + unit) * in_outer_stride) + c0;
@@ -421,14 +404,9 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
             const int e = i / (CB / 2), cc = 2 * (i % (CB / 2));
             if (NC > 1 && unit * NC + cc / CC >= coils) continue;  // read as zero below
             const unsigned dst = (unsigned)__cvta_generic_to_shared(stage + e * CB + cc);
-            if constexpr (SOS)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
-                             "l"(src + (cc / CC) * cstride + (long long)e * stride + cc % CC)
-                             : "memory");
-            else  // of a zero line nothing is read, zeros are written
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst),
-                             "l"(src + (long long)e * stride + cc), "r"(row_zero(unit, e) ? 0 : 16)
-                             : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
+                         "l"(src + (cc / CC) * cstride + (long long)e * stride + cc % CC)
+                         : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -446,10 +424,6 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
         }
     }
     const int nunit = SOS ? (coils + NC - 1) / NC : (int)min((long long)per, nouter - outer0);
-    if (rows) {
-        flag_rows(0);
-        __syncthreads();
-    }
     if (pipe) issue(0);
     for (int u = 0; u < nunit; ++u) {
         const int coil = SOS ? u * NC + sub : 0;
@@ -467,8 +441,7 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
             } else {
                 const float2 *src = in + coil * cstride + ou * in_outer_stride + (long long)t * stride + c0 + col;
 #pragma unroll
-                for (int m = 0; m < M; ++m)
-                    v[m] = line_ok && !row_zero(u, t + T * m) ? src[(long long)(T * m) * stride] : make_float2(0.f, 0.f);
+                for (int m = 0; m < M; ++m) v[m] = line_ok ? src[(long long)(T * m) * stride] : make_float2(0.f, 0.f);
             }
             rdft<M>(v);
             float2 *dst = ex + t * CB + line;
@@ -476,7 +449,6 @@ __global__ void __launch_bounds__(kRegCols * RegSplit<N>::TH, N <= 384 ? 2 : 1) 
 #pragma unroll
             for (int k1 = 1; k1 < M; ++k1) dst[k1 * T * CB] = cmul(v[k1], tw[t * k1]);
         }
-        if (rows && u + 1 < nunit) flag_rows(u + 1);
         __syncthreads();
         if (pipe && u + 1 < nunit) issue(u + 1);  // the block is free: every thread passed step A
         if (threadIdx.x < CB * M) {

@@ -1,6 +1,6 @@
 """GPU: a reconstruction after one that filled the whole grid: the transform's
-lines without samples, which its first stage leaves out, are zero and not what
-the other reconstruction left there."""
+lines without samples, whose cells the gridding leaves unwritten, are zero and
+not what the other reconstruction left there."""
 import numpy as np
 import pytest
 
