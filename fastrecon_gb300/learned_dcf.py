@@ -175,13 +175,28 @@ def energy_weight(traj, dim, recon, w_pipe, seed=0, power=0.25):
 
 def kernel_mass(lut, kernel_width: float, dim: int, steps: int = 100000) -> float:
     """Integral of the radial LUT kernel over the plane (2D) or space (3D),
-    with the gridding's LUT index rule: M = int K(|x|) d^d x."""
+    with the gridding's LUT index rule: M = int K(|x|) d^d x, the midpoint sum
+    over ``steps`` radii.  The kernel is constant over the radii of one LUT
+    entry, whose sum of r or r^2 has a closed form: a sum over the entries
+    instead of the radii (learned_dcf on 12 k samples 540 us with the 100,000
+    radii, which the network waited for, 160 us so)."""
     lut = np.asarray(lut, np.float64)
     hw = kernel_width / 2
-    r = (np.arange(steps) + 0.5) * (hw / steps)
-    k = lut[np.minimum(np.rint(r / hw * (len(lut) - 1)).astype(np.int64), len(lut) - 1)]
-    shell = 2 * np.pi * r if dim == 2 else 4 * np.pi * r * r
-    return float(np.sum(k * shell) * (hw / steps))
+    last = len(lut) - 1
+    # first radius of every entry: the index rule looked at around its analytic place
+    edge = np.zeros(last + 2, np.int64)
+    edge[-1] = steps
+    if last > 0:
+        k = np.arange(1, last + 1)
+        near = np.ceil((k - 0.5) * (steps / last) - 0.5).astype(np.int64)[:, None] + np.array([-1, 0, 1])
+        below = np.rint((near + 0.5) * (hw / steps) / hw * last) < k[:, None]
+        edge[1:-1] = np.clip(near[:, 0] + below.sum(1), 0, steps)
+    # sums over j < i of 2 j + 1 and of 3 (2 j + 1)^2: whole numbers, exact below 2^63
+    if dim == 2:
+        total = np.diff(edge * edge) * (np.pi * (hw / steps))
+    else:
+        total = np.diff(4 * edge ** 3 - edge) * (np.pi / 3 * (hw / steps) ** 2)
+    return float(np.sum(lut * total) * (hw / steps))
 
 
 def target_offset(lut, kernel_width: float, dim: int) -> float:
