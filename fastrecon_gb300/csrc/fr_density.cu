@@ -156,33 +156,46 @@ __global__ void scan_outer_kernel(int *a, long long columns, int len, long long 
     }
 }
 
-__device__ __forceinline__ long long sat_at(const int *sat, int G, int x, int y, int z)
+// Samples in the boxes of every radius around a sample's cell, from the table's
+// corners.  Two lanes a sample, one for each end of the boxes in x: the two corners of
+// a row are 2 r + 1 cells apart, mostly in one 128-byte line, which one load of the
+// pair then touches once; four radii's corners in flight.  Bound: the lines a
+// load touches, one a cycle and SM.  5.1 M samples, 320^3 table, radii 1, 2, 4, 8:
+// 488 us with a thread a sample and eight corners in flight, 398 us so.
+// (Whole numbers modulo 2^32: the differences are counts below it.)
+constexpr int kBoxRadii = 4;
+__global__ void __launch_bounds__(256) box_count_kernel(const float4 *__restrict__ traj, long long n, int dim, int G,
+                                                        const int *__restrict__ sat, Radii R, int *__restrict__ counts)
 {
-    if (x < 0 || y < 0 || z < 0) return 0;
-    return sat[((size_t)z * G + y) * G + x];
-}
-
-__global__ void box_count_kernel(const float4 *__restrict__ traj, long long n, int dim, int G, const int *sat,
-                                 Radii R, int *counts)
-{
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float4 p = traj[i];
+    const int upper = threadIdx.x & 1;
+    const long long pairs = (long long)gridDim.x * (blockDim.x / 2);
+    // all lanes of a warp go round together (the pair meets by a shuffle)
+    for (long long b = blockIdx.x * (long long)(blockDim.x / 2) + (threadIdx.x & ~31u) / 2; b < n; b += pairs) {
+        const long long i = b + (threadIdx.x & 31) / 2;
+        const bool live = i < n;
+        const float4 p = live ? traj[i] : make_float4(0.f, 0.f, 0.f, 0.f);
         const int cx = nearest_cell(p.x, G), cy = nearest_cell(p.y, G), cz = dim == 3 ? nearest_cell(p.z, G) : 0;
-        for (int k = 0; k < R.n; ++k) {
-            const int r = R.r[k];
-            const int x0 = max(cx - r, 0) - 1, x1 = min(cx + r, G - 1);
-            const int y0 = max(cy - r, 0) - 1, y1 = min(cy + r, G - 1);
-            long long s;
-            if (dim == 3) {
-                const int z0 = max(cz - r, 0) - 1, z1 = min(cz + r, G - 1);
-                s = sat_at(sat, G, x1, y1, z1) - sat_at(sat, G, x0, y1, z1) - sat_at(sat, G, x1, y0, z1) -
-                    sat_at(sat, G, x1, y1, z0) + sat_at(sat, G, x0, y0, z1) + sat_at(sat, G, x0, y1, z0) +
-                    sat_at(sat, G, x1, y0, z0) - sat_at(sat, G, x0, y0, z0);
-            } else {
-                s = sat_at(sat, G, x1, y1, 0) - sat_at(sat, G, x0, y1, 0) - sat_at(sat, G, x1, y0, 0) +
-                    sat_at(sat, G, x0, y0, 0);
+        for (int k0 = 0; k0 < R.n; k0 += kBoxRadii) {
+            unsigned v[kBoxRadii];
+#pragma unroll
+            for (int k = 0; k < kBoxRadii; ++k) {
+                const int r = k0 + k < R.n ? R.r[k0 + k] : 0;
+                const int x = upper ? min(cx + r, G - 1) : max(cx - r, 0) - 1;
+                const int y0 = max(cy - r, 0) - 1, y1 = min(cy + r, G - 1);
+                const int z0 = dim == 3 ? max(cz - r, 0) - 1 : -1, z1 = dim == 3 ? min(cz + r, G - 1) : 0;
+                const bool on = live && k0 + k < R.n && x >= 0;  // a corner before the table counts nothing
+                auto at = [&](int y, int z) {
+                    return on && y >= 0 && z >= 0 ? (unsigned)__ldg(&sat[((size_t)z * G + y) * G + x]) : 0u;
+                };
+                v[k] = (at(y1, z1) - at(y0, z1)) - (at(y1, z0) - at(y0, z0));
             }
-            counts[i * R.n + k] = (int)s;
+#pragma unroll
+            for (int k = 0; k < kBoxRadii; ++k) {
+                const unsigned other = __shfl_xor_sync(0xffffffffu, v[k], 1);
+                // half of the radii are written by each lane
+                if (live && k0 + k < R.n && (k >= kBoxRadii / 2) == (upper != 0))
+                    counts[i * R.n + k0 + k] = (int)(upper ? v[k] - other : other - v[k]);
+            }
         }
     }
 }
@@ -289,7 +302,7 @@ int density_counts_run(fr_plan p, const int *radii, int nradii, int *d_counts, c
         scan_outer_kernel<<<blocks_for((long long)G * G, 128), 128, 0, s>>>(sat, (long long)G * G, G, (long long)G * G, 0);
         FR_CHECK_LAUNCH("scan_outer_kernel");
     }
-    box_count_kernel<<<blocks_for(n, 256), 256, 0, s>>>(traj, n, p->dim, G, sat, R, d_counts);
+    box_count_kernel<<<blocks_for(2 * n, 256), 256, 0, s>>>(traj, n, p->dim, G, sat, R, d_counts);
     FR_CHECK_LAUNCH("box_count_kernel");
     return FR_OK;
 }
