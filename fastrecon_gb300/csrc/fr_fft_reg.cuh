@@ -250,12 +250,13 @@ __global__ void __launch_bounds__(kRegLinesX * RegSplit<N>::TH) fft_x_kernel_reg
 // other's loads (nor a third of them idle in step A): step A 16 lanes a line, step B
 // the pair's 2 M transforms of 16 points 32 at a time.  Warps are persistent and
 // load their next pair while step B runs; a pair without a written tile costs its
-// mask bits and zeros only.  Bound: HBM with every cell read (16 coils, 384^3: 6.6 TB/s), else
-// the latency of the loads at 16 warps per SM.  x stage alone, cells of a ball, per
-// CTA / per warp: 8 coils, 240^3 195 / 184 us; 16 coils, 384^3 1540 / 1374; 4 coils,
-// 480^3 1194 / 667 and 512^3 1132 / 796; 2 coils, 640^3 2138 / 1200; but 16 coils,
-// 192^3 198 / 200 and 128^3 68 / 74, where the 128 threads of a CTA all work in
-// both steps and ten CTAs fit on an SM.
+// mask bits and zeros only.  Bound: HBM with every cell read (16 coils, 384^3:
+// 6.6 TB/s), else the latency of the loads at 16 warps per SM.  x stage alone, cells
+// of a ball (its empty lines not written on either side; their zeros cost 4 to 8 %
+// more), per CTA / per warp: 8 coils, 240^3 195 / 184 us; 16 coils, 384^3 1540 /
+// 1374; 4 coils, 480^3 1194 / 667 and 512^3 1132 / 796; 2 coils, 640^3 2138 / 1200;
+// but 16 coils, 192^3 198 / 200 and 128^3 68 / 74, where the 128 threads of a CTA
+// all work in both steps and ten CTAs fit on an SM.
 template <int N>
 constexpr int kXWarps = N <= 192 ? 0 : N <= 256 ? 4 : 8;  // most warps per CTA; 0: fft_x_kernel_reg
 
