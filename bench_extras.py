@@ -90,7 +90,7 @@ def batched_spiral(torch, steps=20, warmup=3, frames=64, coils=12, recon=192, os
                          "best_ms": tune_ms, "seconds": round(tune_s, 2)},
             "graph_replays_per_batch": launches,
             "roofline": _roofline(n * (4 * 2 + 4) + n * coils * 8 + frames * coils * G * G * 8, ms,
-                                  "grid_persistent_kernel + split reduction (the replayed graph, all frames)"),
+                                  "batch_lanes_kernel, k-space copy and split reduction (the replayed graph, all frames)"),
             "workload": f"2D dynamic spiral: {frames} frames x 4-24 variable-density interleaves x {samples} "
                         f"samples (seeded), {coils} coils, {recon}^2 matrix, os {os_} -> {G}^2 grid; one "
                         "persistent launch per batch, replayed from a CUDA graph; tiling from the autotuner"}
