@@ -168,8 +168,9 @@ __global__ void __launch_bounds__(kDegridThreads, 2) degrid_tiles_kernel(DegridP
     int2 *lists = reinterpret_cast<int2 *>(blk + (size_t)B[0] * B[1] * B[2] * T.stride);
     float *thr = reinterpret_cast<float *>(lists + (kDegridThreads / LP) * LE);
     float *lut = thr + P.L;
-    // {sample, its footprint: first cell in the part, 5 bits an axis, cells, 3 bits}
-    uint2 *queue = reinterpret_cast<uint2 *>(lut + P.L + (P.L & 1));
+    // {sample, its footprint: first cell in the part, 6 bits an axis, cells, 3 bits};
+    // 2 L floats past thr, so on 8 bytes for odd tables too
+    uint2 *queue = reinterpret_cast<uint2 *>(thr + 2 * P.L);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     const WorkItem it = T.items[blockIdx.x];
@@ -839,7 +840,7 @@ int degrid_tiles(fr_plan p, const DegridParams &P, cudaStream_t s)
     }
     for (int d = 0; d < 3; ++d) parts *= T.nbox[d];
     if (parts > 65535 || groups > 65535) return -1;
-    const size_t smem = bytes() + (size_t)(kDegridThreads / LP) * degrid_list(RR) * 8 + (size_t)(P.L + 1) * 8 + kDegridRound * 8;
+    const size_t smem = bytes() + (size_t)(kDegridThreads / LP) * degrid_list(RR) * 8 + (size_t)P.L * 8 + kDegridRound * 8;
     const dim3 grid((unsigned)p->nitems_occupied, (unsigned)parts, (unsigned)groups);
     degrid_outside_kernel<<<(int)std::min<long long>((P.n + 255) / 256, (long long)sm_count() * 8), 256, 0, s>>>(P);
     FR_CHECK_LAUNCH("degrid_outside_kernel");
