@@ -16,8 +16,10 @@
 // kernel that evaluates the taps.  Frame f's k-space is the block channels x
 // n_f at complex offset channels * offset[f] and its grid the block
 // channels x G^d at f * channels * G^d.
+// Either way a work item's fixed-point sums have a scale per coil float, from that
+// float's sum and largest value in the item: a weak coil keeps its bits beside strong ones.
 // 64 frames of 8 k to 49 k samples, 12 coils, 384^2 grids: 1312 us evaluating the
-// taps (one CTA of 128 KB per SM), 831 us from the lists.
+// taps (one CTA of 128 KB per SM), 821 us from the lists.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,7 +42,7 @@ struct fr_batch_s {
     // per-call buffers; a captured graph has its own, which later calls with
     // more channels cannot move
     struct Scratch {
-        DevBuf partials, kt, kmag, coil_max, item_inv;
+        DevBuf partials, kt, float_inv;
     } direct, captured;
     long long n_total = 0, npairs = 0, nitems = 0, nslots = 0, nsplits = 0;
     int blocks = 0;
@@ -147,10 +149,7 @@ int fill_batch_grid(fr_batch b, fr_batch_s::Scratch &sc, int lane_floats, BatchG
         g->runs = b->runs.as<FrameRun>();
         g->nruns = b->nruns;
         g->kt = sc.kt.as<float>();
-        g->kmag = sc.kmag.as<float>();
-        g->coil_max = sc.coil_max.as<unsigned>();
-        g->frames = b->frames;
-        g->item_inv = sc.item_inv.as<float>();
+        g->float_inv = sc.float_inv.as<float>();
         g->err = p->err_dev;
     }
     return FR_OK;
@@ -166,9 +165,8 @@ int ensure_scratch(fr_batch b, fr_batch_s::Scratch &sc, int channels, int *lane_
         return FR_ERR_OUT_OF_MEMORY;
     *lane_floats = b->tap_words > 0 ? batch_lane_floats(K, p->coil_group, p->L, channels) : 0;
     const size_t rows = (size_t)std::max<long long>(b->n_total, 1);
-    if (*lane_floats > 0 && (sc.kt.reserve(rows * (size_t)(channels + (channels & 1)) * 8) || sc.kmag.reserve(rows * 4) ||
-                             sc.coil_max.reserve((size_t)b->frames * channels * 4) ||
-                             sc.item_inv.reserve((size_t)b->nitems * 4))) {
+    const size_t row = (size_t)(channels + (channels & 1)) * 8;  // bytes
+    if (*lane_floats > 0 && (sc.kt.reserve(rows * row) || sc.float_inv.reserve((size_t)b->nitems * row))) {
         cudaGetLastError();  // the failed allocation
         *lane_floats = 0;
     }

@@ -17,6 +17,7 @@
 // weight * dcf * sample into the shared tile.  The weight is computed once
 // per sample and reused for every coil of the group.
 #include <cuda_runtime.h>
+#include <float.h>
 
 #include <algorithm>
 
@@ -73,21 +74,12 @@ struct GridParams {
     int *err = nullptr;       // mapped error word
     int accumulate = 0;       // add the tiles to the grid instead of overwriting it (sample partitions)
     long long kin_stride = 0; // complex values between coils of the caller's coil-major k-space (0: n)
-    // batches: per frame and coil the largest |re| or |im| of dcf * k (float bits,
-    // coil_max_kernel): the sample-major copy holds every coil scaled by
-    // 2^coil_exponent, so that one fixed-point scale per item serves weak and
-    // strong coils alike; nullptr: the copy is not scaled
-    const unsigned *coil_max = nullptr;
+    // batches: inverse fixed-point scale per work item and float of a
+    // sample-major row (2 kstride of them, item_float_scale_kernel), so that a
+    // coil that is weak in an item keeps its bits beside the strong ones
+    const float *float_inv = nullptr;
     float sum_limit = 1073741824.f;  // bound of an item's fixed-point sums (fixed_sum_limit)
 };
-
-// Exponent that brings a coil's measure into [1, 2) (0 for a coil of zeros);
-// 2^e and 2^-e are normal floats.
-__device__ __forceinline__ int coil_exponent(unsigned max_bits)
-{
-    const float m = __uint_as_float(max_bits);
-    return m > 0.f ? max(min(-ilogbf(m), 120), -120) : 0;
-}
 
 // Column swizzle of cell i in a row of R floats: keeps (re, im) pairs
 // adjacent and spreads the flush (lanes along cells) over all banks.
@@ -406,6 +398,8 @@ __device__ __forceinline__ void scale_bounds_mag(const unsigned long long *recs,
     }
 }
 
+constexpr float kAddLimit = 4194304.f;  // most an add of the fixed-point tile may be: 2^22 (red_add_fx)
+
 // 1 / S_f from the item's B_f and M_f (exact: a power of two).
 __device__ __forceinline__ float inv_scale_of(float bsum, unsigned bmax_bits, float lut_absmax, float sum_limit)
 {
@@ -414,7 +408,7 @@ __device__ __forceinline__ float inv_scale_of(float bsum, unsigned bmax_bits, fl
     int e = 0;
     if (B > 0.f && M > 0.f) {
         // largest power of two 2^e <= min(sum_limit / B, 2^22 / M)
-        const float t = fminf(__fdiv_rn(sum_limit, B), __fdiv_rn(4194304.f, M));
+        const float t = fminf(__fdiv_rn(sum_limit, B), __fdiv_rn(kAddLimit, M));
         frexpf(t, &e);
         e = max(min(e - 1, 100), -100);
     }
@@ -914,7 +908,7 @@ constexpr int kLaneWarpsSmall = 8, kLaneWarpsLarge = 16;
 // Shared-memory layout of grid_lanes_kernel from its 128-byte aligned base:
 // tile [K][32] int32 | weights [L] | per warp: value slots [32][32] floats,
 // record table [32] int4 {sample, first word | taps << 8, first group, 0} |
-// per warp one mbarrier (8 bytes) | inverse scale per coil [16] (batches).
+// per warp one mbarrier (8 bytes) | inverse scale per coil float [32] (batches).
 struct LaneSmem {
     unsigned lutw, stage, table, mbar, unscale, end;
 };
@@ -926,7 +920,7 @@ __host__ __device__ __forceinline__ LaneSmem lane_smem_layout(long long K, int L
     m.table = m.stage + (unsigned)(warps * kLaneBatch * 128);
     m.mbar = m.table + (unsigned)(warps * kLaneBatch * 16);
     m.unscale = m.mbar + (unsigned)(warps * 8);
-    m.end = m.unscale + 64u;
+    m.end = m.unscale + 128u;
     return m;
 }
 
@@ -1006,7 +1000,8 @@ __device__ __forceinline__ int2 lanes_cell(unsigned acc, int i, int cl, int firs
 // first loads under the clearing and the next item fetched ahead (batches): 64
 // frames, 12 coils, 2.1 M samples 883 -> 801 us; 64 sparse frames, 16 coils, 0.2 M
 // samples 592 -> 527; a 3D plan of 8 coils, 2.6 M samples 1107 -> 1083.
-template <int NF>
+// unscale: inverse scale per coil float (PF), else inv_item.
+template <int NF, bool PF>
 __device__ __forceinline__ void lanes_flush(const GridParams &P, long long item, unsigned acc, int cg, int ox, int oy,
                                             int oz, float inv_item, const float *unscale)
 {
@@ -1026,9 +1021,12 @@ __device__ __forceinline__ void lanes_flush(const GridParams &P, long long item,
         const int hx = Tx / 2, npair = K / 2;
         const size_t cstride4 = cells >> 1;
         float4 *grid4 = reinterpret_cast<float4 *>(gridf) + (size_t)(cg * CG + cl) * cstride4;
-        float inv[HALVES];
+        float invx[HALVES], invy[HALVES];
 #pragma unroll
-        for (int h = 0; h < HALVES; ++h) inv[h] = unscale ? unscale[cl + NCL * h] : inv_item;
+        for (int h = 0; h < HALVES; ++h) {
+            invx[h] = PF ? unscale[2 * (cl + NCL * h)] : inv_item;
+            invy[h] = PF ? unscale[2 * (cl + NCL * h) + 1] : inv_item;
+        }
         // a lane's pair u = r hx + xh of row r = lz Ty + ly, advanced without divisions
         const int step = nwarps * NPX, du = step / hx, dxh = step - du * hx, dlz = du / Ty, dly = du - dlz * Ty;
         int u = warp * NPX + px;
@@ -1056,9 +1054,9 @@ __device__ __forceinline__ void lanes_flush(const GridParams &P, long long item,
                 if (cl + NCL * h >= ncl) break;
                 const int2 a = lanes_cell<NF>(acc, i, cl + NCL * h, px);
                 const int2 b = lanes_cell<NF>(acc, i + 1, cl + NCL * h, px);
-                const float sa = odd ? -inv[h] : inv[h];
-                const float sb = P.checkerboard ? -sa : inv[h];
-                const float4 v = make_float4((float)a.x * sa, (float)a.y * sa, (float)b.x * sb, (float)b.y * sb);
+                const float ax = odd ? -invx[h] : invx[h], ay = odd ? -invy[h] : invy[h];
+                const float bx = P.checkerboard ? -ax : invx[h], by = P.checkerboard ? -ay : invy[h];
+                const float4 v = make_float4((float)a.x * ax, (float)a.y * ay, (float)b.x * bx, (float)b.y * by);
                 put_cells(dst + (size_t)(NCL * h) * cstride4, v, P.accumulate);
             }
         }
@@ -1071,18 +1069,19 @@ __device__ __forceinline__ void lanes_flush(const GridParams &P, long long item,
         const int gx = ox + lx, gy = oy + r % Ty, gz = oz + r / Ty;
         if (gx >= P.G || gy >= P.G || gz >= Gz) continue;
         const int2 a = lanes_cell<NF>(acc, i, cl, 0);
-        const float inv = unscale ? unscale[cl] : inv_item;
-        const float sg = P.checkerboard && ((gx + gy + gz) & 1) ? -inv : inv;
+        const float ix = PF ? unscale[2 * cl] : inv_item, iy = PF ? unscale[2 * cl + 1] : inv_item;
+        const bool odd = P.checkerboard && ((gx + gy + gz) & 1);
         put_cells(&grid[(size_t)(cg * CG + cl) * cells + ((size_t)gz * G + (size_t)gy) * G + (size_t)gx],
-                  make_float2((float)a.x * sg, (float)a.y * sg), P.accumulate);
+                  make_float2((float)a.x * (odd ? -ix : ix), (float)a.y * (odd ? -iy : iy)), P.accumulate);
     }
 }
 
 // One work item with samples for one coil group: the tile zeroed, the item's
 // records added, the tile flushed.  `parity`: of the warp's mbarrier, which
 // carries over from item to item; the weights must be staged.
-// before_flush runs when the records are added.
-template <int NF, int NW, typename IT, typename Fn>
+// before_flush runs when the records are added.  PF: a fixed-point scale per coil
+// float (batches), which goes on the values; else one for the item, on the weights.
+template <int NF, int NW, bool PF, typename IT, typename Fn>
 __device__ __forceinline__ void lanes_item(const GridParams &P, const WorkItem &it, long long item, int cg, float4 *smem4,
                                            unsigned &parity, Fn before_flush)
 {
@@ -1129,13 +1128,15 @@ __device__ __forceinline__ void lanes_item(const GridParams &P, const WorkItem &
     // part-done: its first tap word and tap count advanced past the done
     // groups) move to the front and the window fills up from the next records.
     unsigned long long rw = load_rw(0), rw_next = load_rw(kLaneBatch);
-    const float inv = P.item_inv[item];
-    float *unscale = nullptr;
-    if (P.coil_max) {  // a batch: the coils' own scales undone with the item's
-        unscale = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(smem4) + L_.unscale);
-        if (threadIdx.x < NF / 2 && cg * CG + (int)threadIdx.x < P.channels)
-            unscale[threadIdx.x] =
-                inv * ldexpf(1.f, -coil_exponent(P.coil_max[(size_t)it.pad * P.channels + cg * CG + threadIdx.x]));
+    const float inv = PF ? 1.f : P.item_inv[item];
+    const float *unscale = nullptr;
+    if constexpr (PF) {
+        float *u = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(smem4) + L_.unscale);
+        if (threadIdx.x < NF)
+            u[threadIdx.x] = (int)threadIdx.x < 2 * ncl
+                                 ? P.float_inv[(size_t)item * (size_t)(2 * P.kstride) + 2 * cg * CG + threadIdx.x]
+                                 : 1.f;
+        unscale = u;
     }
     // the tile starts at zero, and so do the value slots of a partial coil
     // group (a slot's coils past the group's last are never copied).  The barrier
@@ -1149,6 +1150,7 @@ __device__ __forceinline__ void lanes_item(const GridParams &P, const WorkItem &
     }
     const float sc = __fdiv_rn(1.f, inv);  // exact: a power of two
     const unsigned mbar = acc + L_.mbar + 8u * (unsigned)warp;
+    float fsc[PF ? NF : 1];  // scale of the coil float this lane adds at step f
     bool zeroed = false;
     for (int wbase = 0; wbase < nrec;) {
         // this lane's record of the window: its tap groups (kLaneTaps taps
@@ -1251,6 +1253,12 @@ __device__ __forceinline__ void lanes_item(const GridParams &P, const WorkItem &
         if (!zeroed) {
             __syncthreads();
             zeroed = true;
+            if constexpr (PF) {
+                // 1 / unscale: a power of two within 2^+-100
+#pragma unroll
+                for (int f = 0; f < NF; ++f)
+                    fsc[f] = __uint_as_float(0x7F000000u - __float_as_uint(unscale[(f ^ lane) & (NF - 1)]));
+            }
         }
         for (int p0 = 0; p0 < total; p0 += 32) {
             const int cr = cr_n, nl = nl_n;
@@ -1267,12 +1275,16 @@ __device__ __forceinline__ void lanes_item(const GridParams &P, const WorkItem &
 #pragma unroll
                 for (int k = 0; k < kLaneTaps; ++k) {
                     a[k] = (acc + (min(t[k] & cmask, (unsigned)(K - 1)) << 7)) | lane4;
-                    w[k] = k < nl ? __fmul_rn(lutw_s[min(t[k] >> kTapCellBits, (unsigned)(P.L - 1))], sc) : 0.f;
+                    w[k] = k < nl ? lutw_s[min(t[k] >> kTapCellBits, (unsigned)(P.L - 1))] : 0.f;
+                    if (!PF) w[k] = __fmul_rn(w[k], sc);
                 }
                 const unsigned va = (stage + ((unsigned)cr << 7)) | lane4;
                 float v[NF];
 #pragma unroll
-                for (int f = 0; f < NF; ++f) v[f] = lds_f32_v(va ^ ((unsigned)f << 2));
+                for (int f = 0; f < NF; ++f) {
+                    v[f] = lds_f32_v(va ^ ((unsigned)f << 2));
+                    if constexpr (PF) v[f] = __fmul_rn(v[f], fsc[f]);
+                }
 #pragma unroll
                 for (int k = 0; k < kLaneTaps; ++k) {
                     if (k < nl) {
@@ -1288,26 +1300,24 @@ __device__ __forceinline__ void lanes_item(const GridParams &P, const WorkItem &
     __syncthreads();
     before_flush();
     if (it.slot < 0) {
-        lanes_flush<NF>(P, item, acc, cg, ox, oy, oz, inv, unscale);
+        lanes_flush<NF, PF>(P, item, acc, cg, ox, oy, oz, inv, unscale);
     } else {
         // partial tile in the [cell][NF] layout the reduction reads: float p
         // of cell c is float p ^ swz(c) (whole pairs move)
         float4 *dst = reinterpret_cast<float4 *>(P.partials + ((size_t)it.slot * P.ngroups + cg) * (size_t)K * NF);
         for (int i4 = threadIdx.x; i4 < K * (NF / 4); i4 += blockDim.x) {
             const int c = i4 / (NF / 4), p0 = 4 * (i4 % (NF / 4)), sw = swz<NF>(c);
-            float ia = inv, ib = inv;
-            if (unscale) {
-                ia = unscale[(p0 ^ sw) >> 1];
-                ib = unscale[((p0 + 2) ^ sw) >> 1];
-            }
+            const int g0 = p0 ^ sw, g1 = (p0 + 2) ^ sw;
+            const float ax = PF ? unscale[g0] : inv, ay = PF ? unscale[g0 + 1] : inv;
+            const float bx = PF ? unscale[g1] : inv, by = PF ? unscale[g1 + 1] : inv;
             if constexpr (NF == 32) {  // one copy: the plain quad, its pairs swapped for odd cells
                 int4 a = lds_s32x4(acc + ((unsigned)c << 7) + (unsigned)(4 * (p0 ^ (sw & ~3))));
                 if (sw & 2) a = make_int4(a.z, a.w, a.x, a.y);
-                dst[i4] = make_float4((float)a.x * ia, (float)a.y * ia, (float)a.z * ib, (float)a.w * ib);
+                dst[i4] = make_float4((float)a.x * ax, (float)a.y * ay, (float)a.z * bx, (float)a.w * by);
                 continue;
             }
-            const int2 a = lanes_cell<NF>(acc, c, (p0 ^ sw) >> 1, c), b = lanes_cell<NF>(acc, c, ((p0 + 2) ^ sw) >> 1, c);
-            dst[i4] = make_float4((float)a.x * ia, (float)a.y * ia, (float)b.x * ib, (float)b.y * ib);
+            const int2 a = lanes_cell<NF>(acc, c, g0 >> 1, c), b = lanes_cell<NF>(acc, c, g1 >> 1, c);
+            dst[i4] = make_float4((float)a.x * ax, (float)a.y * ay, (float)b.x * bx, (float)b.y * by);
         }
     }
 }
@@ -1345,7 +1355,7 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) grid_lanes_kernel(GridParams
     if (it.count == 0) return lanes_zero<NF>(P, it, blockIdx.x, blockIdx.y, smem4);
     unsigned parity = 0u;
     lanes_setup<NW>(P, smem4);
-    lanes_item<NF, NW, IT>(P, it, blockIdx.x, blockIdx.y, smem4, parity, [] {});
+    lanes_item<NF, NW, false, IT>(P, it, blockIdx.x, blockIdx.y, smem4, parity, [] {});
 }
 
 // Persistent, for batches: as many CTAs as fit on the GPU, each taking work
@@ -1385,7 +1395,7 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) batch_lanes_kernel(GridParam
             lanes_zero<NF>(P, it, item, cg, smem4);
             fetch();
         } else {
-            lanes_item<NF, NW, IT>(P, it, item, cg, smem4, parity, fetch);
+            lanes_item<NF, NW, true, IT>(P, it, item, cg, smem4, parity, fetch);
         }
     }
 }
@@ -1461,6 +1471,86 @@ __global__ void __launch_bounds__(kBoundThreads) item_scale_kernel(const WorkIte
         bs = ldexpf(__ull2float_ru(q), -e);
     }
     if (threadIdx.x == 0) inv[blockIdx.x] = inv_scale_of(bs, m, lut_absmax, sum_limit);
+}
+
+// The same per coil float of a work item, for batches: thread (row, quad) takes
+// 4 floats of every rows-th record's sample-major row (`quads` float4 each, at
+// most kFloatQuads), first their maxima, then, where it matters, their sums as whole
+// multiples of 2^-e, rounded up (2^e max = 2^22..23): exact and in no order.  A sum
+// of up to sum_limit / kAddLimit records is below that many maxima, so the limit of
+// the adds is the lower one: no second pass.  Values that are not finite count as zero.
+// Bound by the latency of the gathers (item, records, rows), so small CTAs, many per
+// SM: 64 frames, 12 coils, 2.1 M samples 66 us; with 256 threads, both passes always,
+// 128 us, and 195 us with 8 rows in flight per thread kept for the second pass.  (A scale
+// per coil and frame and one per item beside it took 61 us, and cost a coil that is
+// weak in an item, strong elsewhere in the frame, its bits.)
+constexpr int kFloatThreads = 128, kFloatLoads = 4, kFloatQuads = 48;
+__global__ void __launch_bounds__(kFloatThreads, 10) item_float_scale_kernel(
+    const WorkItem *__restrict__ items, const unsigned long long *__restrict__ trecs, const float4 *__restrict__ kt,
+    int quads, float lut_absmax, float sum_limit, float *__restrict__ inv)
+{
+    const WorkItem it = items[blockIdx.x];
+    if (it.count == 0) return;  // its scales are not read
+    __shared__ unsigned mx[4 * kFloatQuads];
+    __shared__ unsigned long long sums[4][kFloatThreads];
+    const int rows = kFloatThreads / quads, row = threadIdx.x / quads, quad = threadIdx.x - row * quads;
+    const int count = row < rows ? it.count : 0;
+    for (int i = threadIdx.x; i < 4 * quads; i += kFloatThreads) mx[i] = 0u;
+    __syncthreads();
+    auto each = [&](auto use) {
+        for (int j0 = row; j0 < count; j0 += kFloatLoads * rows) {
+            unsigned long long rw[kFloatLoads];
+            float4 v[kFloatLoads];
+#pragma unroll
+            for (int k = 0; k < kFloatLoads; ++k)
+                rw[k] = j0 + k * rows < count ? __ldg(trecs + it.begin + j0 + k * rows) : 0ull;
+#pragma unroll
+            for (int k = 0; k < kFloatLoads; ++k)
+                v[k] = (rw[k] >> 40) & 0xFF ? __ldg(kt + (size_t)(unsigned)rw[k] * quads + quad)
+                                            : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < kFloatLoads; ++k) {
+                const float a[4] = {fabsf(v[k].x), fabsf(v[k].y), fabsf(v[k].z), fabsf(v[k].w)};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) use(c, a[c] <= FLT_MAX ? a[c] : 0.f);
+            }
+        }
+    };
+    float m[4] = {0.f, 0.f, 0.f, 0.f};
+    each([&](int c, float a) { m[c] = fmaxf(m[c], a); });
+    if (row < rows) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) atomicMax(&mx[4 * quad + c], __float_as_uint(m[c]));
+    }
+    __syncthreads();
+    const bool sum = (float)it.count > sum_limit / kAddLimit;
+    if (sum) {
+        float up[4][2];  // 2^e in two factors
+        unsigned long long q[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const unsigned b = mx[4 * quad + c];
+            const int e = b ? 22 - ilogbf(__uint_as_float(b)) : 0;
+            up[c][0] = __int_as_float((e / 2 + 127) << 23);
+            up[c][1] = __int_as_float((e - e / 2 + 127) << 23);
+        }
+        // below 2^23 the float a + 2^23 is 2^23 plus a rounded up to a whole number
+        each([&](int c, float a) {
+            q[c] += __float_as_uint(__fadd_ru(a * up[c][0] * up[c][1], 8388608.f)) - 0x4B000000u;
+        });
+#pragma unroll
+        for (int c = 0; c < 4; ++c) sums[c][threadIdx.x] = q[c];
+        __syncthreads();
+    }
+    for (int f = threadIdx.x; f < 4 * quads; f += kFloatThreads) {
+        float b = __uint_as_float(mx[f]);  // a sum that does not lower the scale
+        if (sum) {
+            unsigned long long q = 0;
+            for (int r = 0; r < rows; ++r) q += sums[f & 3][r * quads + (f >> 2)];
+            b = b > 0.f ? ldexpf(__ull2float_ru(q), ilogbf(b) - 22) : 0.f;
+        }
+        inv[(size_t)blockIdx.x * (4 * quads) + f] = inv_scale_of(b, mx[f], lut_absmax, sum_limit);
+    }
 }
 
 // Sum the partial tiles of each split tile in item order and write the grid.
@@ -1579,31 +1669,26 @@ int launch_reduce(const GridParams &P, long long nsplits, cudaStream_t s)
 // bound by the latency of these reads).
 constexpr int kTrSamples = 128;
 constexpr int kTrThreads = 256, kTrPer = 8;
-constexpr int kTrCoils = 96;  // the copy's shared memory holds at most 95 coils
 // The copy holds dcf * k (the product GridLut.cpp:109 forms, same rounding)
-// and mag[s] = the largest |re| or |im| of sample s's products.  blocks: the
-// sample runs of a batch, one per CTA (nullptr: one trajectory).
+// and (unless null) mag[s] = the largest |re| or |im| of sample s's products.
+// blocks: the sample runs of a batch, one per CTA (nullptr: one trajectory).
 __global__ void __launch_bounds__(kTrThreads) transpose_kspace_kernel(const float2 *__restrict__ in,
                                                                       const float *__restrict__ dcf,
                                                                       float2 *__restrict__ out,
                                                                       float *__restrict__ mag, long long n,
                                                                       int channels, int cstride, long long in_stride,
-                                                                      const FrameRun *__restrict__ blocks,
-                                                                      const unsigned *__restrict__ coil_max)
+                                                                      const FrameRun *__restrict__ blocks)
 {
     extern __shared__ float2 tr[];  // [channels][kTrSamples + 1]
-    __shared__ float dsh[kTrSamples], csh[kTrCoils];
+    __shared__ float dsh[kTrSamples];
     long long s0 = (long long)blockIdx.x * kTrSamples;  // first sample, of all frames
     int ns = (int)min((long long)kTrSamples, n - s0);
     if (blocks) {
-        // last runs first: coil_max_kernel has just read them
-        const FrameRun r = blocks[gridDim.x - 1 - blockIdx.x];
+        const FrameRun r = blocks[blockIdx.x];
         s0 = r.off + r.begin;
         ns = min(kTrSamples, r.n - r.begin);
         in += (size_t)(channels - 1) * (size_t)r.off;  // the frame's block starts at channels * off
         in_stride = r.n;
-        for (int c = threadIdx.x; c < channels; c += kTrThreads)
-            csh[c] = ldexpf(1.f, coil_exponent(coil_max[(size_t)r.frame * channels + c]));
     }
     for (int j = threadIdx.x; j < ns; j += kTrThreads) dsh[j] = dcf[s0 + j];
     const int total = channels * kTrSamples;
@@ -1630,52 +1715,19 @@ __global__ void __launch_bounds__(kTrThreads) transpose_kspace_kernel(const floa
             const float2 v = tr[c * (kTrSamples + 1) + j];
             const float d = dsh[j];
             o = make_float2(__fmul_rn(d, v.x), __fmul_rn(d, v.y));
-            if (blocks) o = make_float2(o.x * csh[c], o.y * csh[c]);
         }
         out[(size_t)(s0 + j) * cstride + c] = o;
     }
+    if (!mag) return;
     for (int j = threadIdx.x; j < ns; j += kTrThreads) {
         const float d = dsh[j];
         float m = 0.f;
         for (int c = 0; c < channels; ++c) {
             const float2 v = tr[c * (kTrSamples + 1) + j];
-            float a = fmaxf(fabsf(__fmul_rn(d, v.x)), fabsf(__fmul_rn(d, v.y)));
-            // a coil's infinities stay its own: they do not set the other coils' scale
-            if (blocks) a = isfinite(a) ? a * csh[c] : 0.f;
-            m = fmaxf(m, a);
+            m = fmaxf(m, fmaxf(fabsf(__fmul_rn(d, v.x)), fabsf(__fmul_rn(d, v.y))));
         }
         mag[s0 + j] = m;
     }
-}
-
-// Per frame and coil the largest finite |re| or |im| of dcf * k, as float bits (the
-// table starts at zero): a bound of the scaled values, which then cannot overflow.
-// A CTA per run of samples, all its loads in flight, coil maxima in shared memory.
-// Bound: HBM (64 frames, 12 coils, 2.1 M samples: 25 us of 831 more than a measure
-// taken from every fourth run, which is no bound).
-__global__ void __launch_bounds__(kTrThreads) coil_max_kernel(const float2 *__restrict__ in,
-                                                              const float *__restrict__ dcf,
-                                                              const FrameRun *__restrict__ runs, int channels,
-                                                              unsigned *__restrict__ coil_max)
-{
-    __shared__ unsigned mx[kTrCoils];
-    const FrameRun r = runs[blockIdx.x];
-    const int ns = min(kTrSamples, r.n - r.begin);
-    for (int c = threadIdx.x; c < channels; c += kTrThreads) mx[c] = 0u;
-    __syncthreads();
-    const int j = threadIdx.x % kTrSamples;
-    const float d = j < ns ? dcf[r.off + r.begin + j] : 0.f;
-    in += (size_t)channels * (size_t)r.off + r.begin + j;
-#pragma unroll 4
-    for (int c = threadIdx.x / kTrSamples; c < channels; c += kTrThreads / kTrSamples) {
-        const float2 v = j < ns ? in[(size_t)c * r.n] : make_float2(0.f, 0.f);
-        const float a = fmaxf(fabsf(__fmul_rn(d, v.x)), fabsf(__fmul_rn(d, v.y)));
-        const unsigned m = __reduce_max_sync(0xffffffffu, isfinite(a) ? __float_as_uint(a) : 0u);
-        if ((threadIdx.x & 31) == 0) atomicMax(&mx[c], m);
-    }
-    __syncthreads();
-    for (int c = threadIdx.x; c < channels; c += kTrThreads)
-        if (mx[c]) atomicMax(&coil_max[(size_t)r.frame * channels + c], mx[c]);
 }
 
 int profile_events(fr_plan p, cudaEvent_t **ev);
@@ -1719,6 +1771,13 @@ int profile_events(fr_plan p, cudaEvent_t **ev)
 // Per-item scales (every launched item, so the indices match blockIdx.x).
 int launch_item_scales(const GridParams &P, long long nitems, cudaStream_t s)
 {
+    if (P.float_inv) {  // a batch
+        item_float_scale_kernel<<<(unsigned)nitems, kFloatThreads, 0, s>>>(
+            P.items, P.trecs, reinterpret_cast<const float4 *>(P.kdata), (int)(P.kstride / 2), P.lut_absmax, P.sum_limit,
+            const_cast<float *>(P.float_inv));
+        FR_CHECK_LAUNCH("item_float_scale_kernel");
+        return FR_OK;
+    }
     item_scale_kernel<<<(unsigned)nitems, kBoundThreads, 0, s>>>(P.items, P.trecs, P.mag, P.lut_absmax, P.sum_limit,
                                                                  const_cast<float *>(P.item_inv));
     FR_CHECK_LAUNCH("item_scale_kernel");
@@ -1865,7 +1924,7 @@ int kspace_prepare(fr_plan p, const float *d_kdata, const float *d_dcf, int chan
                                      (int)trsmem));
     transpose_kspace_kernel<<<(unsigned)((p->n + kTrSamples - 1) / kTrSamples), kTrThreads, trsmem, s>>>(
         reinterpret_cast<const float2 *>(d_kdata), d_dcf, p->kt.as<float2>(), p->kmag.as<float>(), (long long)p->n,
-        channels, cstride, (long long)(kin_stride ? kin_stride : p->n), nullptr, nullptr);
+        channels, cstride, (long long)(kin_stride ? kin_stride : p->n), nullptr);
     FR_CHECK_LAUNCH("transpose_kspace_kernel");
     p->kt_prepared = d_kdata;
     p->kt_prepared_channels = channels;
@@ -2112,7 +2171,7 @@ int batch_launch_t(const GridParams &P, int blocks, long long nsplits, cudaStrea
 
 int batch_lane_floats(long long K, int coil_group, int L, int channels)
 {
-    if (channels <= 0 || channels > kTrCoils || (size_t)channels * (kTrSamples + 1) * sizeof(float2) > 96 * 1024) return 0;
+    if (channels <= 0 || channels > 2 * kFloatQuads || (size_t)channels * (kTrSamples + 1) * sizeof(float2) > 96 * 1024) return 0;
     if (floats_per_cell(coil_group) > 32 || lane_warps(K, L) == 0) return 0;
     return lane_floats(std::min(channels, coil_group));
 }
@@ -2189,25 +2248,19 @@ int batch_grid_run(const BatchGrid &b, const float *d_kdata, const float *d_dcf,
             if (trsmem > 48 * 1024)
                 FR_CUDA(cudaFuncSetAttribute(transpose_kspace_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)trsmem));
-            FR_CUDA(cudaMemsetAsync(b.coil_max, 0, (size_t)b.frames * channels * sizeof(unsigned), s));
-            coil_max_kernel<<<(unsigned)b.nruns, kTrThreads, 0, s>>>(reinterpret_cast<const float2 *>(d_kdata), d_dcf,
-                                                                     b.runs, channels, b.coil_max);
-            FR_CHECK_LAUNCH("coil_max_kernel");
             transpose_kspace_kernel<<<(unsigned)b.nruns, kTrThreads, trsmem, s>>>(
-                reinterpret_cast<const float2 *>(d_kdata), d_dcf, reinterpret_cast<float2 *>(b.kt), b.kmag, b.n_total,
-                channels, cstride, 0, b.runs, b.coil_max);
+                reinterpret_cast<const float2 *>(d_kdata), d_dcf, reinterpret_cast<float2 *>(b.kt), nullptr, b.n_total,
+                channels, cstride, 0, b.runs);
             FR_CHECK_LAUNCH("transpose_kspace_kernel");
         }
-        P.coil_max = b.coil_max;
         P.kdata = b.kt;
-        P.mag = b.kmag;
         P.sample_major = 1;
         P.kstride = cstride;
         P.trecs = b.trecs;
         P.taps = b.taps;
         P.lutw = b.lutw;
         P.tap_words = b.tap_words;
-        P.item_inv = b.item_inv;
+        P.float_inv = b.float_inv;
         P.err = b.err;
         P.coil_group = std::min(P.coil_group, b.lane_floats / 2);
         return launch_lanes(nullptr, P, b.lane_floats, b.nitems, b.nsplits, s);

@@ -312,10 +312,7 @@ struct BatchGrid {
     const FrameRun *runs = nullptr;
     long long nruns = 0;
     float *kt = nullptr;              // n_total rows of dcf * k, channels rounded up to even
-    float *kmag = nullptr;            // n_total
-    unsigned *coil_max = nullptr;     // frames x channels
-    int frames = 0;
-    float *item_inv = nullptr;        // nitems
+    float *float_inv = nullptr;       // nitems x floats of a row
     int *err = nullptr;
     float sum_limit = 1073741824.f;   // fixed_sum_limit
 };
