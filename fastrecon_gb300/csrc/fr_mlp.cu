@@ -156,24 +156,29 @@ __device__ __forceinline__ float rcp_approx(float a)
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
     return r;
 }
-// tanh of two values, branch-free: x + x t Q(t), t = x^2, below 0.55 (Q of degree
-// 4, a least-maximum relative fit: 1e-9, in floats within 0.72 ulp), and
-// 1 - 2 / (e^2x + 1) above (absolute error about 1e-7, falling with x; the limits
-// +-1 and NaN come out by themselves).  About 9 issue slots a value.
+// tanh of two values, branch-free.  Below 0.65: x + x t Q(t), t = x^2, Q the polynomial
+// of degree 4 through (tanh(sqrt t) / sqrt t - 1) / t at the 5 Chebyshev points of
+// [0, 0.65^2] (relative error of the result 2.6e-8, in floats within 1.1 ulp).  Above: the
+// identity 1 - 2 / (e^2|x| + 1) with x's sign, whose errors are those of the approximate
+// exponential and reciprocal times the subtracted term over the result, 0.75 at 0.65
+// and falling (+-1 and NaN come out by themselves).  Within 1.7 ulp of FP64 at 1.0 M
+// points, where tanhf promises 2.  A split further out costs the polynomial a degree
+// for each 0.1 to 0.2: 5.1 M samples 602 us, at 0.75 with degree 5 625 us and 1.5 ulp, at 1
+// with degree 6 641 us and 1.2 ulp; without the absolute value and sign 590 us, but
+// 1 - 2 / (e^2x + 1) of a negative x cancels: 3.8 ulp.
 __device__ __forceinline__ f32x2 tanh2(f32x2 x)
 {
     const f32x2 one = pack2(1.f, 1.f);
     const f32x2 t = mul2(x, x);
-    f32x2 q = fma2(t, pack2(-0.0062742396f, -0.0062742396f), pack2(0.021071678f, 0.021071678f));
-    q = fma2(q, t, pack2(-0.05385231f, -0.05385231f));
-    q = fma2(q, t, pack2(0.13332586f, 0.13332586f));
-    q = fma2(q, t, pack2(-0.33333316f, -0.33333316f));
-    const float2 p = unpack2(fma2(mul2(q, t), x, x));
-    const float2 a = unpack2(mul2(x, pack2(2.885390081777927f, 2.885390081777927f)));  // 2 / ln 2
-    const float2 e = unpack2(add2(pack2(ex2_approx(a.x), ex2_approx(a.y)), one));
+    f32x2 q = fma2(t, pack2(-0.0059237261f, -0.0059237261f), pack2(0.020873461f, 0.020873461f));
+    q = fma2(q, t, pack2(-0.053823758f, -0.053823758f));
+    q = fma2(q, t, pack2(0.13332583f, 0.13332583f));
+    q = fma2(q, t, pack2(-0.33333328f, -0.33333328f));
+    const float2 p = unpack2(fma2(mul2(q, t), x, x)), v = unpack2(x);
+    constexpr float k = 2.885390081777927f;  // 2 / ln 2
+    const float2 e = unpack2(add2(pack2(ex2_approx(fabsf(v.x) * k), ex2_approx(fabsf(v.y) * k)), one));
     const float2 h = unpack2(fma2(pack2(rcp_approx(e.x), rcp_approx(e.y)), pack2(-2.f, -2.f), one));
-    const float2 v = unpack2(x);
-    return pack2(fabsf(v.x) < 0.55f ? p.x : h.x, fabsf(v.y) < 0.55f ? p.y : h.y);
+    return pack2(fabsf(v.x) < 0.65f ? p.x : copysignf(h.x, v.x), fabsf(v.y) < 0.65f ? p.y : copysignf(h.y, v.y));
 }
 
 // The forward pass with the hidden layer (64 x 64) on the tensor cores:
@@ -189,7 +194,7 @@ __device__ __forceinline__ f32x2 tanh2(f32x2 x)
 // Bound: the pipes of tanh (special functions 45 %, FMA 39 % of the time), the
 // tensor pipe (34 %) and issue (51 %).  5.1 M samples: 775 us with W2 rows of
 // 128 bytes (8-way bank conflicts, the shared pipe 83 % busy), tanhf, and
-// first-layer weights read as single BF16; 600 us so.
+// first-layer weights read as single BF16; 612 us so.
 __device__ __forceinline__ unsigned pack_bf16(float lo_half, float hi_half)
 {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo_half, hi_half);
