@@ -90,25 +90,14 @@ __global__ void append_trecs_kernel(const unsigned long long *__restrict__ src, 
 int grow_keep(DevBuf &b, size_t used, size_t need, cudaStream_t s)
 {
     if (need <= b.bytes && b.ptr) return FR_OK;
-    size_t want = std::max<size_t>(need, b.bytes + b.bytes / 2);
-    void *p = nullptr;
-    cudaError_t e = cudaMalloc(&p, std::max<size_t>(want, 256));
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc");
+    DevBuf grown;
+    if (grown.reserve(std::max<size_t>(need, b.bytes + b.bytes / 2))) return FR_ERR_OUT_OF_MEMORY;
     if (used) {
-        e = cudaMemcpyAsync(p, b.ptr, used, cudaMemcpyDeviceToDevice, s);
-        if (e != cudaSuccess) {
-            cudaFree(p);
-            return cuda_fail(e, "cudaMemcpyAsync");
-        }
-        e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
-            cudaFree(p);
-            return cuda_fail(e, "cudaStreamSynchronize");
-        }
+        FR_CUDA(cudaMemcpyAsync(grown.ptr, b.ptr, used, cudaMemcpyDeviceToDevice, s));
+        FR_CUDA(cudaStreamSynchronize(s));
     }
-    b.release();
-    b.ptr = p;
-    b.bytes = std::max<size_t>(want, 256);
+    std::swap(b.ptr, grown.ptr);
+    std::swap(b.bytes, grown.bytes);
     return FR_OK;
 }
 
@@ -166,10 +155,8 @@ int ensure_scratch(fr_batch b, fr_batch_s::Scratch &sc, int channels, int *lane_
     *lane_floats = b->tap_words > 0 ? batch_lane_floats(K, p->coil_group, p->L, channels) : 0;
     const size_t rows = (size_t)std::max<long long>(b->n_total, 1);
     const size_t row = (size_t)(channels + (channels & 1)) * 8;  // bytes
-    if (*lane_floats > 0 && (sc.kt.reserve(rows * row) || sc.float_inv.reserve((size_t)b->nitems * row))) {
-        cudaGetLastError();  // the failed allocation
+    if (*lane_floats > 0 && (sc.kt.reserve(rows * row) || sc.float_inv.reserve((size_t)b->nitems * row)))
         *lane_floats = 0;
-    }
     return FR_OK;
 }
 
@@ -270,7 +257,6 @@ int fr_batch_set_trajectories(fr_batch b, const float *d_traj, const size_t *off
                 b->tap_words = p->tap_words;
             taps = p->tap_words > 0 && b->tap_words > 0;
             if (taps && grow_keep(b->trecs, (size_t)npairs * 8, (size_t)(npairs + p->npairs) * 8, s)) taps = false;
-            if (!taps) cudaGetLastError();  // a failed allocation: the batch evaluates its taps
         }
         if (nf > 0 && taps) {
             FR_CUDA(cudaMemcpyAsync(b->taps.as<unsigned>() + offsets[f] * (size_t)b->tap_words, p->taps.ptr,
@@ -314,10 +300,8 @@ int fr_batch_set_trajectories(fr_batch b, const float *d_traj, const size_t *off
         nslots += p->nslots;
         nsplits += p->nsplits;
     }
-    if (!taps || b->tap_words == 0 || b->runs.reserve(std::max<size_t>(runs.size(), 1) * sizeof(FrameRun))) {
-        cudaGetLastError();
+    if (!taps || b->tap_words == 0 || b->runs.reserve(std::max<size_t>(runs.size(), 1) * sizeof(FrameRun)))
         b->tap_words = 0;
-    }
     b->nruns = (long long)runs.size();
     if (b->tap_words > 0 && !runs.empty())
         FR_CUDA(cudaMemcpyAsync(b->runs.ptr, runs.data(), runs.size() * sizeof(FrameRun), cudaMemcpyHostToDevice, s));

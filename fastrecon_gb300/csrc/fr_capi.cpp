@@ -43,7 +43,8 @@ void DevBuf::release()
 
 // Host-side fault injection for the out-of-memory paths: with
 // FR_FAIL_ALLOC_BYTES=B in the environment, every device reservation of B
-// bytes or more fails as cudaMalloc would (nothing is allocated).
+// bytes or more asks cudaMalloc for more than any GPU has, and fails as one
+// that does not fit would (nothing is allocated).
 static bool injected_alloc_failure(size_t want)
 {
     const char *v = std::getenv("FR_FAIL_ALLOC_BYTES");
@@ -57,13 +58,12 @@ int DevBuf::reserve(size_t n)
     if (n <= bytes && ptr) return 0;
     release();
     size_t want = std::max<size_t>(n, 256);
-    if (injected_alloc_failure(want)) {
-        fail(FR_ERR_OUT_OF_MEMORY, "device allocation refused (FR_FAIL_ALLOC_BYTES)");
-        return 1;
-    }
-    cudaError_t e = cudaMalloc(&ptr, want);
+    const bool refused = injected_alloc_failure(want);
+    const cudaError_t e = cudaMalloc(&ptr, refused ? (size_t)1 << 60 : want);
     if (e != cudaSuccess) {
         ptr = nullptr;
+        cudaGetLastError();  // callers that do without the memory launch on: not their error
+        if (refused) return fail(FR_ERR_OUT_OF_MEMORY, "device allocation refused (FR_FAIL_ALLOC_BYTES)");
         cuda_fail(e, "cudaMalloc");
         return 1;
     }

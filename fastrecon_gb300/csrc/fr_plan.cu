@@ -1313,10 +1313,8 @@ int plan_run(fr_plan p, const float *d_traj, size_t n, cudaStream_t s)
         const long long more = most / p->chunk;  // items beyond one a tile, and split tiles
         if (p->pairs.reserve(std::max<long long>(most, 1) * 8) || p->items.reserve((p->ntiles + more) * sizeof(WorkItem)) ||
             p->splits.reserve(std::max<long long>(more, 1) * sizeof(SplitTile)) ||
-            (taps_possible(p, n, recmax) && p->trecs.reserve(std::max<long long>(most, 1) * 8))) {
-            cudaGetLastError();  // the counts' own sizes may fit
-            small = false;
-        }
+            (taps_possible(p, n, recmax) && p->trecs.reserve(std::max<long long>(most, 1) * 8)))
+            small = false;  // the counts' own sizes may fit
     }
     TileScan *scan = p->tile_scan.as<TileScan>();
     if (small) {
