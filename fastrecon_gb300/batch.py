@@ -14,7 +14,7 @@ from .capi import check
 from .gridding import _ptr, _stream, _torch, kb_lut
 
 
-def _desc(dim, grid_size, kernel_width, lut, tile=(0, 0, 0), coil_group=0, chunk=0, checkerboard=False):
+def _desc(dim, grid_size, kernel_width, lut, tile=(0, 0, 0), coil_group=0, chunk=0, checkerboard=False, tap_lists=True):
     d = capi.PlanDesc()
     d.dim = dim
     d.grid_size = grid_size
@@ -25,7 +25,7 @@ def _desc(dim, grid_size, kernel_width, lut, tile=(0, 0, 0), coil_group=0, chunk
         d.tile[i] = int(tile[i]) if i < len(tile) else 0
     d.coil_group = coil_group
     d.chunk = chunk
-    d.flags = capi.FR_PLAN_CHECKERBOARD if checkerboard else 0
+    d.flags = (capi.FR_PLAN_CHECKERBOARD if checkerboard else 0) | (0 if tap_lists else capi.FR_PLAN_NO_TAP_LISTS)
     return d
 
 
@@ -37,16 +37,18 @@ def _offsets(counts):
 
 class GridBatch:
     """Frames f = 0..F-1 with counts[f] samples each; k-space frame-major
-    (frame f: channels x counts[f]), grid out frames x channels x G^d."""
+    (frame f: channels x counts[f]), grid out frames x channels x G^d.
+    tap_lists=False evaluates the taps in the scatter: slower, without the lists
+    and the sample-major copy of the k-space."""
 
     def __init__(self, dim: int, grid_size: int, kernel_width: float = 4.0, lut=None, lut_length: int = 512,
                  overgrid_factor: float = 2.0, tile=(0, 0, 0), coil_group: int = 0, chunk: int = 0,
-                 checkerboard: bool = False):
+                 checkerboard: bool = False, tap_lists: bool = True):
         self.lib = capi.load()
         if lut is None:
             lut = kb_lut(kernel_width, overgrid_factor, lut_length)
         self.lut = np.ascontiguousarray(lut, np.float32)
-        self.desc = _desc(dim, grid_size, kernel_width, self.lut, tile, coil_group, chunk, checkerboard)
+        self.desc = _desc(dim, grid_size, kernel_width, self.lut, tile, coil_group, chunk, checkerboard, tap_lists)
         h = C.c_void_p()
         check(self.lib.fr_batch_create(C.byref(self.desc), C.byref(h)), "fr_batch_create")
         self.h = h
@@ -57,7 +59,8 @@ class GridBatch:
     def from_desc(cls, desc: capi.PlanDesc, lut):
         tile = [desc.tile[i] for i in range(3)]
         return cls(desc.dim, desc.grid_size, desc.kernel_width, lut=lut, tile=tile, coil_group=desc.coil_group,
-                   chunk=desc.chunk, checkerboard=bool(desc.flags & capi.FR_PLAN_CHECKERBOARD))
+                   chunk=desc.chunk, checkerboard=bool(desc.flags & capi.FR_PLAN_CHECKERBOARD),
+                   tap_lists=not desc.flags & capi.FR_PLAN_NO_TAP_LISTS)
 
     def __del__(self):
         if getattr(self, "h", None) is not None and self.h.value:

@@ -12,8 +12,8 @@
 // offsets.  Gridding: one sample-major copy of all frames' dcf * k, then a
 // persistent scatter kernel that takes (coil group, item) work indices from a
 // counter until the batch is done: the tap lanes, or without tap lists (a
-// kernel too wide for them, coil groups of 32, tiles too large, no memory) the
-// kernel that evaluates the taps.  Frame f's k-space is the block channels x
+// kernel too wide for them, coil groups of 32, tiles too large, refused, or more
+// than half of the free memory) the kernel that evaluates the taps.  Frame f's k-space is the block channels x
 // n_f at complex offset channels * offset[f] and its grid the block
 // channels x G^d at f * channels * G^d.
 // Either way a work item's fixed-point sums have a scale per coil float, from that
@@ -144,18 +144,46 @@ int fill_batch_grid(fr_batch b, fr_batch_s::Scratch &sc, int lane_floats, BatchG
     return FR_OK;
 }
 
+// Tap lists and the copy of the k-space are a choice of speed: a buffer for them grows
+// only into half of the free memory, and is given up where that runs out all the
+// same, so that what fits without them still fits, and its caller's grids too.
+int reserve_spare(DevBuf &b, size_t need)
+{
+    if (need <= b.bytes && b.ptr) return FR_OK;
+    b.release();
+    return need <= device_bytes_free() / 2 ? b.reserve(need) : fail(FR_ERR_OUT_OF_MEMORY, "no spare device memory");
+}
+
+// false: there was nothing to give up.  A captured graph reads the lists and its copy.
+bool drop_tap_lists(fr_batch b)
+{
+    fr_plan p = b->plan;
+    if (b->exec || (!b->taps.ptr && !p->taps.ptr && !b->direct.kt.ptr && !b->captured.kt.ptr)) return false;
+    b->tap_words = 0;
+    p->taps_enabled = false;  // until the next trajectories
+    for (DevBuf *d : {&b->taps, &b->trecs, &p->taps, &p->trecs}) d->release();
+    for (fr_batch_s::Scratch *sc : {&b->direct, &b->captured}) {
+        sc->kt.release();
+        sc->float_inv.release();
+    }
+    return true;
+}
+
 // The buffers of a call, and whether it takes the tap lists (*lane_floats > 0):
 // where their copy of the k-space does not fit, the taps are evaluated.
 int ensure_scratch(fr_batch b, fr_batch_s::Scratch &sc, int channels, int *lane_floats)
 {
     fr_plan p = b->plan;
     const long long K = (long long)p->tile[0] * p->tile[1] * p->tile[2];
-    if (b->nslots > 0 && sc.partials.reserve(grid_partials_bytes(b->nslots, channels, p->coil_group, K)))
-        return FR_ERR_OUT_OF_MEMORY;
+    const size_t part = b->nslots > 0 ? grid_partials_bytes(b->nslots, channels, p->coil_group, K) : 0;
     *lane_floats = b->tap_words > 0 ? batch_lane_floats(K, p->coil_group, p->L, channels) : 0;
+    if (part > 0 && sc.partials.reserve(part)) {
+        if (!drop_tap_lists(b) || sc.partials.reserve(part)) return FR_ERR_OUT_OF_MEMORY;
+        *lane_floats = 0;
+    }
     const size_t rows = (size_t)std::max<long long>(b->n_total, 1);
     const size_t row = (size_t)(channels + (channels & 1)) * 8;  // bytes
-    if (*lane_floats > 0 && (sc.kt.reserve(rows * row) || sc.float_inv.reserve((size_t)b->nitems * row)))
+    if (*lane_floats > 0 && (reserve_spare(sc.kt, rows * row) || reserve_spare(sc.float_inv, (size_t)b->nitems * row)))
         *lane_floats = 0;
     return FR_OK;
 }
@@ -237,26 +265,48 @@ int fr_batch_set_trajectories(fr_batch b, const float *d_traj, const size_t *off
     b->frames = frames;
     b->off.assign(offsets, offsets + frames + 1);
     b->n_total = (long long)offsets[frames];
-    if (b->traj.reserve(std::max<long long>(b->n_total, 1) * 16) ||
-        b->frame_off.reserve((size_t)(frames + 1) * 8) || b->counter.reserve(256))
-        return FR_ERR_OUT_OF_MEMORY;
+    auto first = [&] {
+        return b->traj.reserve(std::max<long long>(b->n_total, 1) * 16) || b->frame_off.reserve((size_t)(frames + 1) * 8) ||
+               b->counter.reserve(256);
+    };
+    p->taps_enabled = !(p->flags & FR_PLAN_NO_TAP_LISTS);
+    if (first() && (!drop_tap_lists(b) || first())) return FR_ERR_OUT_OF_MEMORY;  // (lists of the last trajectories)
     FR_CUDA(cudaMemcpyAsync(b->frame_off.ptr, b->off.data(), (size_t)(frames + 1) * 8, cudaMemcpyHostToDevice, s));
     long long npairs = 0, nitems = 0, nslots = 0, nsplits = 0;
     b->tap_words = 0;
     b->chunk = 0;
     bool taps = b->n_total <= 0x7FFFFFFFll;
     std::vector<FrameRun> runs;
+    // true: memory ran out beside the tap lists, which are now given up
+    auto without_lists = [&](int st) {
+        if (st != FR_ERR_OUT_OF_MEMORY || !drop_tap_lists(b)) return false;
+        taps = false;
+        return true;
+    };
     for (int f = 0; f < frames; ++f) {
         const size_t nf = offsets[f + 1] - offsets[f];
         int st = plan_run(p, d_traj + 4 * offsets[f], nf, s);  // synchronises s
+        if (without_lists(st)) st = plan_run(p, d_traj + 4 * offsets[f], nf, s);
         if (st) return st;
         b->chunk = std::max(b->chunk, p->chunk);
+        if (nslots + p->nslots > 0x7FFFFFFFll || nitems + p->nitems > 0x7FFFFFFFll)
+            return fail(FR_ERR_UNSUPPORTED, "batch too large for 32-bit item indices");
+        auto grow = [&] {
+            int e = grow_keep(b->recs, (size_t)npairs * 8, (size_t)(npairs + p->npairs) * 8, s);
+            if (!e) e = grow_keep(b->items, (size_t)nitems * sizeof(WorkItem), (size_t)(nitems + p->nitems) * sizeof(WorkItem), s);
+            if (!e) e = grow_keep(b->splits, (size_t)nsplits * sizeof(SplitTile),
+                                  (size_t)(nsplits + std::max<long long>(p->nsplits, 0)) * sizeof(SplitTile), s);
+            return e;
+        };
+        st = grow();
+        if (without_lists(st)) st = grow();
+        if (st) return st;
         if (nf > 0 && taps) {
-            if (p->tap_words > 0 && b->tap_words == 0 &&
-                !b->taps.reserve((size_t)b->n_total * p->tap_words * 4))
+            if (p->tap_words > 0 && b->tap_words == 0 && !reserve_spare(b->taps, (size_t)b->n_total * p->tap_words * 4))
                 b->tap_words = p->tap_words;
-            taps = p->tap_words > 0 && b->tap_words > 0;
-            if (taps && grow_keep(b->trecs, (size_t)npairs * 8, (size_t)(npairs + p->npairs) * 8, s)) taps = false;
+            taps = p->tap_words > 0 && b->tap_words > 0 &&
+                   !grow_keep(b->trecs, (size_t)npairs * 8, (size_t)(npairs + p->npairs) * 8, s);
+            if (!taps) drop_tap_lists(b);
         }
         if (nf > 0 && taps) {
             FR_CUDA(cudaMemcpyAsync(b->taps.as<unsigned>() + offsets[f] * (size_t)b->tap_words, p->taps.ptr,
@@ -270,13 +320,6 @@ int fr_batch_set_trajectories(fr_batch b, const float *d_traj, const size_t *off
             for (size_t k = 0; k < nf; k += (size_t)frame_run_samples())
                 runs.push_back(FrameRun{(long long)offsets[f], (int)nf, (int)k, f, 0});
         }
-        if (nslots + p->nslots > 0x7FFFFFFFll || nitems + p->nitems > 0x7FFFFFFFll)
-            return fail(FR_ERR_UNSUPPORTED, "batch too large for 32-bit item indices");
-        if ((st = grow_keep(b->recs, (size_t)npairs * 8, (size_t)(npairs + p->npairs) * 8, s)) ||
-            (st = grow_keep(b->items, (size_t)nitems * sizeof(WorkItem), (size_t)(nitems + p->nitems) * sizeof(WorkItem), s)) ||
-            (st = grow_keep(b->splits, (size_t)nsplits * sizeof(SplitTile),
-                            (size_t)(nsplits + std::max<long long>(p->nsplits, 0)) * sizeof(SplitTile), s)))
-            return st;
         if (nf) FR_CUDA(cudaMemcpyAsync(b->traj.as<float4>() + offsets[f], p->traj.ptr, nf * 16, cudaMemcpyDeviceToDevice, s));
         if (p->npairs)
             FR_CUDA(cudaMemcpyAsync(b->recs.as<unsigned long long>() + npairs, p->pairs.ptr, (size_t)p->npairs * 8,
@@ -301,7 +344,7 @@ int fr_batch_set_trajectories(fr_batch b, const float *d_traj, const size_t *off
         nsplits += p->nsplits;
     }
     if (!taps || b->tap_words == 0 || b->runs.reserve(std::max<size_t>(runs.size(), 1) * sizeof(FrameRun)))
-        b->tap_words = 0;
+        drop_tap_lists(b);
     b->nruns = (long long)runs.size();
     if (b->tap_words > 0 && !runs.empty())
         FR_CUDA(cudaMemcpyAsync(b->runs.ptr, runs.data(), runs.size() * sizeof(FrameRun), cudaMemcpyHostToDevice, s));

@@ -32,41 +32,64 @@ int cuda_fail(cudaError_t e, const char *what)
     return FR_ERR_CUDA;
 }
 
+// Host-side fault injection for the out-of-memory paths: with
+// FR_FAIL_ALLOC_BYTES=B in the environment, every device reservation of B
+// bytes or more, and with FR_ALLOC_LIMIT_BYTES=B every one that would take the
+// reservations held above B, asks cudaMalloc for more than any GPU has, and fails
+// as one that does not fit would (nothing is allocated).
+static std::atomic<size_t> g_held{0};  // bytes of all DevBufs
+
+static size_t env_bytes(const char *name)
+{
+    const char *v = std::getenv(name);
+    return v ? (size_t)std::strtoull(v, nullptr, 10) : 0;
+}
+
+static bool injected_alloc_failure(size_t want)
+{
+    const size_t one = env_bytes("FR_FAIL_ALLOC_BYTES"), all = env_bytes("FR_ALLOC_LIMIT_BYTES");
+    return (one > 0 && want >= one) || (all > 0 && g_held + want > all);
+}
+
+size_t device_bytes_free()
+{
+    size_t avail = 0, total = 0;
+    if (cudaMemGetInfo(&avail, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    const size_t all = env_bytes("FR_ALLOC_LIMIT_BYTES"), held = g_held;
+    return all > 0 ? std::min(avail, all > held ? all - held : 0) : avail;
+}
+
 DevBuf::~DevBuf() { release(); }
 
 void DevBuf::release()
 {
-    if (ptr) cudaFree(ptr);
+    if (ptr) {
+        cudaFree(ptr);
+        g_held -= bytes;
+    }
     ptr = nullptr;
     bytes = 0;
-}
-
-// Host-side fault injection for the out-of-memory paths: with
-// FR_FAIL_ALLOC_BYTES=B in the environment, every device reservation of B
-// bytes or more asks cudaMalloc for more than any GPU has, and fails as one
-// that does not fit would (nothing is allocated).
-static bool injected_alloc_failure(size_t want)
-{
-    const char *v = std::getenv("FR_FAIL_ALLOC_BYTES");
-    if (!v || !*v) return false;
-    const unsigned long long b = std::strtoull(v, nullptr, 10);
-    return b > 0 && want >= b;
 }
 
 int DevBuf::reserve(size_t n)
 {
     if (n <= bytes && ptr) return 0;
     release();
-    size_t want = std::max<size_t>(n, 256);
+    const size_t want = std::max<size_t>(n, 256);
     const bool refused = injected_alloc_failure(want);
     const cudaError_t e = cudaMalloc(&ptr, refused ? (size_t)1 << 60 : want);
     if (e != cudaSuccess) {
         ptr = nullptr;
         cudaGetLastError();  // callers that do without the memory launch on: not their error
-        if (refused) return fail(FR_ERR_OUT_OF_MEMORY, "device allocation refused (FR_FAIL_ALLOC_BYTES)");
+        if (refused)
+            return fail(FR_ERR_OUT_OF_MEMORY, "device allocation refused (FR_FAIL_ALLOC_BYTES, FR_ALLOC_LIMIT_BYTES)");
         cuda_fail(e, "cudaMalloc");
         return 1;
     }
+    g_held += want;
     bytes = want;
     return 0;
 }

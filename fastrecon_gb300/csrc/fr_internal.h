@@ -39,6 +39,8 @@ struct DevBuf {
     void release();
     template <typename T> T *as() const { return static_cast<T *>(ptr); }
 };
+// Device memory that reservations can still take (0 if unknown).
+size_t device_bytes_free();
 
 // One work item of the scatter: a tile and a chunk of its sorted bin.
 struct WorkItem {

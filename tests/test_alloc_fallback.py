@@ -1,7 +1,9 @@
 """GPU: an allocation that fails and is done without leaves no error behind for
 the next launch: plans and batches whose tap lists do not fit evaluate the
 taps (FR_FAIL_ALLOC_BYTES: reservations of that many bytes or more fail in
-cudaMalloc)."""
+cudaMalloc), and whatever memory a batch without tap lists can be planned and
+gridded in is enough for the same batch with them (FR_ALLOC_LIMIT_BYTES: the
+reservations held may not exceed that)."""
 import numpy as np
 import pytest
 
@@ -52,3 +54,46 @@ def test_batch_without_tap_lists(oracle, refuse):
     kd = torch.from_numpy(np.concatenate([c["kdata"].ravel()] * frames)).cuda()
     got = b.grid(kd, torch.from_numpy(np.concatenate([c["dcf"]] * frames)).cuda(), c["kdata"].shape[0]).cpu().numpy()
     assert all(rel_l2(got[f], c["grid"]) <= TOL for f in range(frames))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("chunk", [0, 256])
+def test_batch_within_any_limit(chunk, monkeypatch):
+    import gc
+
+    import torch
+
+    import fastrecon_gb300 as fr
+    from fastrecon_gb300 import batch as fb
+    from fastrecon_gb300.capi import FastreconError
+    c = load_case("radial2d_small")
+    n, frames, coils = c["traj"].shape[0], 6, c["kdata"].shape[0]
+    traj = torch.from_numpy(np.concatenate([c["traj"]] * frames)).cuda()
+    kd = torch.from_numpy(np.concatenate([c["kdata"].ravel()] * frames)).cuda()
+    dcf = torch.from_numpy(np.concatenate([c["dcf"]] * frames)).cuda()
+
+    def run(limit, lists):
+        gc.collect()
+        monkeypatch.delenv("FR_ALLOC_LIMIT_BYTES", raising=False)
+        b = fb.GridBatch(2, c["G"], c["W"], lut=c["lut"], chunk=chunk, tap_lists=lists)
+        monkeypatch.setenv("FR_ALLOC_LIMIT_BYTES", str(limit))
+        try:
+            for _ in range(2):  # planned again over the buffers of the first time
+                b.set_trajectories(traj, [n] * frames)
+                before = fr.kernel_launches()
+                got = b.grid(kd, dcf, coils).cpu().numpy()
+                launches = fr.kernel_launches() - before
+        except FastreconError as e:
+            assert e.status == 3
+            return None
+        assert all(rel_l2(got[f], c["grid"]) <= TOL for f in range(frames))
+        return launches
+
+    seen = set()
+    for limit in np.geomspace(2e5, 2e7, 60).astype(int):
+        plain, lists = run(limit, False), run(limit, True)
+        assert (plain is None) == (lists is None) or plain is None, limit
+        seen.add((plain, lists))
+    assert (None, None) in seen
+    kinds = {b for a, b in seen if a is not None}
+    assert len(kinds) == 2  # with and without the lists
