@@ -968,6 +968,16 @@ __device__ __forceinline__ bool mbar_wait(unsigned mbar, unsigned parity)
     return false;
 }
 
+// The barrier between a tile's clearing and its first adds, which the CTA's NW warps
+// reach at two places (with records, and without): a named barrier counts the warps
+// that arrive, wherever they do, where __syncthreads in a branch is defined only if
+// all of the block takes it.
+template <int NW>
+__device__ __forceinline__ void tile_cleared()
+{
+    asm volatile("barrier.cta.sync.aligned 1, %0;" ::"n"(NW * 32) : "memory");
+}
+
 // The grid of an item's frame (a single trajectory is one frame).
 __device__ __forceinline__ float *lanes_frame_grid(const GridParams &P, long long item)
 {
@@ -1251,7 +1261,7 @@ __device__ __forceinline__ void lanes_item(const GridParams &P, const WorkItem &
             parity ^= 1u;
         }
         if (!zeroed) {
-            __syncthreads();
+            tile_cleared<NW>();
             zeroed = true;
             if constexpr (PF) {
                 // 1 / unscale: a power of two within 2^+-100
@@ -1296,7 +1306,7 @@ __device__ __forceinline__ void lanes_item(const GridParams &P, const WorkItem &
         }
         __syncwarp();  // the next window rewrites the table and the slots
     }
-    if (!zeroed) __syncthreads();  // a warp without records
+    if (!zeroed) tile_cleared<NW>();  // a warp without records
     __syncthreads();
     before_flush();
     if (it.slot < 0) {
