@@ -368,7 +368,13 @@ int fr_batch_stats(fr_batch b, long long *frames, long long *samples, long long 
     if (samples) *samples = b->n_total;
     if (items) *items = b->nitems;
     if (slots) *slots = b->nslots;
-    if (persistent_ctas) *persistent_ctas = b->blocks;
+    if (persistent_ctas) {
+        fr_plan p = b->plan;
+        const long long K = (long long)p->tile[0] * p->tile[1] * p->tile[2];
+        *persistent_ctas = b->blocks;
+        if (b->ready && b->tap_words > 0 && batch_lane_floats(K, p->coil_group, p->L, 1) > 0)
+            return batch_lane_ctas(K, p->coil_group, p->L, persistent_ctas);
+    }
     return FR_OK;
 }
 

@@ -1811,19 +1811,30 @@ int lane_warps(long long K, int L)
 // Coil floats of the tap-lane scatter for a group of `coils` coils.
 int lane_floats(int coils) { return coils > 8 ? 32 : coils > 4 ? 16 : 8; }
 
+// The CTAs of a persistent kernel that fill the GPU.
+template <typename K>
+int resident_ctas(K kern, int threads, size_t smem, int *ctas)
+{
+    int per_sm = 0, dev = 0, sms = 0;
+    if (smem > 48 * 1024) FR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    FR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
+    FR_CUDA(cudaGetDevice(&dev));
+    FR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    *ctas = std::max(per_sm, 1) * sms;
+    return FR_OK;
+}
+
 template <int NF, int NW>
 int launch_lanes_t(fr_plan p, const GridParams &P, long long nitems, cudaStream_t s)
 {
     const size_t smem = lane_smem_layout(P.K, P.L, NW).end + 128;
     if (P.frame_off) {  // a batch
         auto kern = index32(P) ? batch_lanes_kernel<NF, NW, unsigned> : batch_lanes_kernel<NF, NW, unsigned long long>;
-        if (smem > 48 * 1024) FR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        int per_sm = 0, dev = 0, sms = 0;
-        FR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NW * 32, smem));
-        FR_CUDA(cudaGetDevice(&dev));
-        FR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        int ctas = 0;
+        const int st = resident_ctas(kern, NW * 32, smem, &ctas);
+        if (st) return st;
         FR_CUDA(cudaMemsetAsync(P.work_counter, 0, sizeof(int), s));
-        kern<<<(unsigned)std::min<long long>(P.nwork, (long long)std::max(per_sm, 1) * sms), NW * 32, smem, s>>>(P);
+        kern<<<(unsigned)std::min<long long>(P.nwork, ctas), NW * 32, smem, s>>>(P);
         FR_CHECK_LAUNCH("batch_lanes_kernel");
         return FR_OK;
     }
@@ -2184,6 +2195,19 @@ int batch_lane_floats(long long K, int coil_group, int L, int channels)
     if (channels <= 0 || channels > 2 * kFloatQuads || (size_t)channels * (kTrSamples + 1) * sizeof(float2) > 96 * 1024) return 0;
     if (floats_per_cell(coil_group) > 32 || lane_warps(K, L) == 0) return 0;
     return lane_floats(std::min(channels, coil_group));
+}
+
+int batch_lane_ctas(long long K, int coil_group, int L, int *ctas)
+{
+    const int NF = lane_floats(coil_group), NW = lane_warps(K, L);
+    const size_t smem = lane_smem_layout(K, L, NW).end + 128;
+    auto of = [&](auto large, auto small) {
+        return NW == kLaneWarpsLarge ? resident_ctas(large, NW * 32, smem, ctas) : resident_ctas(small, NW * 32, smem, ctas);
+    };
+    constexpr int A = kLaneWarpsLarge, B = kLaneWarpsSmall;
+    if (NF == 8) return of(batch_lanes_kernel<8, A, unsigned>, batch_lanes_kernel<8, B, unsigned>);
+    if (NF == 16) return of(batch_lanes_kernel<16, A, unsigned>, batch_lanes_kernel<16, B, unsigned>);
+    return of(batch_lanes_kernel<32, A, unsigned>, batch_lanes_kernel<32, B, unsigned>);
 }
 
 int frame_run_samples() { return kTrSamples; }

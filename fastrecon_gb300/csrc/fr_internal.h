@@ -320,6 +320,8 @@ struct BatchGrid {
 };
 // Coil floats of the tap-lane scatter for a batch; 0 where it cannot be used.
 int batch_lane_floats(long long K, int coil_group, int L, int channels);
+// Persistent CTAs of the tap-lane scatter for whole coil groups, where it can be used.
+int batch_lane_ctas(long long K, int coil_group, int L, int *ctas);
 // Sets the attributes of the kernel that evaluates the taps for a configuration
 // and returns how many of its CTAs fill the GPU.  Call outside stream capture.
 int batch_grid_setup(int dim, long long K, int coil_group, int L, int *blocks);
