@@ -674,7 +674,7 @@ int fftcs_execute(fr_fftcs f, const float *d_grid, int channels, const float *d_
             if (nl >= (1ll << 31)) return fail(FR_ERR_UNSUPPORTED, "more than 2^31 lines in a tile-masked transform");
         }
         rk->x<<<(unsigned)xblocks, xthreads, xsmem, s>>>(grid, b1, nl, x0, rx, tw, xm);
-        FR_CHECK_LAUNCH("fft_x_kernel_reg");
+        FR_CHECK_LAUNCH(xw > 0 ? "fft_x_warps_kernel" : "fft_x_kernel_reg");
         const int cb = (rx + kRegCols - 1) / kRegCols;
         if (f->dim == 2) {
             rk->plane_sos<<<(rx + kPlaneCols - 1) / kPlaneCols, rk->colthreads, rk->colsmem, s>>>(b1, nullptr, y0, ry, rx, rx, 0, 0, rx, tw, C,
