@@ -143,8 +143,8 @@ def make_inputs(w, torch, device):
 
 def scatter_kernel(taps: bool, coils: int) -> str:
     """The scatter kernel the recon launches: with tap lists, the tap-lane
-    scatter (but for at most 4 coils in 3D) unless FR_SCATTER_WARP_LISTS=1, the
-    per-warp tap-list scatter otherwise."""
+    scatter for more than 4 coils unless FR_SCATTER_WARP_LISTS=1, the per-warp
+    tap-list scatter otherwise (a recon's tiles have at most 512 cells)."""
     if not taps:
         return "grid_tiles_kernel"
     if coils > 4 and os.environ.get("FR_SCATTER_WARP_LISTS", "0") in ("", "0"):

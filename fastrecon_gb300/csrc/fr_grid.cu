@@ -2042,8 +2042,10 @@ int grid_run(fr_plan p, const float *d_kdata, const float *d_dcf, int channels, 
         P.item_inv = p->item_inv.as<float>();
         // the tap lanes, except for coil groups of 4 on tiles of up to 512 cells,
         // where the per-warp lists' 32 warps per SM hide more latency than the
-        // lanes' 16 (3 coils, 303 k samples on a 115^3 grid: 124 us against 135; on
-        // the 32 x 32 tiles of 2D, 4 coils, 2.7 k samples: 17 against 14)
+        // lanes' 16 (whole gridding, 4 coils, lists / lanes: 300 k samples on a 115^3
+        // grid 162 / 174 us, 1.9 M on 192^3 730 / 729; 32 x 16 tiles in 2D, 2.7 k samples
+        // 20.6 / 22.7, 131 k 48.9 / 51.2, 1 M 220 / 232; the scatter alone on 32 x 32
+        // tiles, 2.7 k samples: 17 / 14)
         const int nw = lane_warps(P.K, P.L);
         const bool lists = p->scatter_warp_lists || (R == 8 && nw == kLaneWarpsSmall);
         if (!lists && nw > 0 && (P.kstride % 2) == 0) {
