@@ -1470,8 +1470,8 @@ int plan_chunk(size_t n, int dim)
     int dev = 0, sms = 152;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         sms = 152;
-    // ~2.7 records per sample with 8^3 tiles in 3D, ~1.2 with 32^2 tiles in 2D;
-    // 2 CTAs per SM, at least 8 items each
+    // ~2.7 records per sample with 8^3 tiles in 3D, ~1.2 with 32^2 tiles in 2D (1.6
+    // with a recon's 16^2, which take the same chunk); 2 CTAs per SM, at least 8 items each
     const double records = (double)n * (dim == 3 ? 2.7 : 1.2);
     const double per = records / ((double)sms * 2 * 8);
     int c = 512;
