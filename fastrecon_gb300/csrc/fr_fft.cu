@@ -470,15 +470,30 @@ int sm_count()
 using FftXRegFn = void (*)(const float2 *, float2 *, long long, int, int, const float2 *, XMask);
 using FftColRegFn = void (*)(const float2 *, float2 *, int, int, int, long long, long long, long long, long long,
                              const float2 *, int, long long, float *, const float *, int, int, long long);
-// Columns per CTA of the 2D y stage: 4 (32-byte rows).  16 / 8 / 4 / 2 columns, a
-// whole 2D reconstruction of 1000 samples: 480^2 to 240^2, 16 coils 111 / 95 /
-// 87 / 83 us; 640^2 to 320^2, 32 coils 286 / 231 / 209 / 223 us; 128^2, 64 coils
-// 104 / 86 / 74 / 70 us; one coil on 64^2 is launch-bound (50 to 52).
-constexpr int kPlaneCols = 4;
+// Columns per CTA of the 2D y stage (4: 32-byte rows), whose CTAs take 16 lines, columns
+// times coils, in turn: the fewest rounds of CTAs times turns, the most columns where that
+// is equal.  16 / 8 / 4 / 2 columns, a whole 2D reconstruction of 1000 samples: 480^2 to
+// 240^2, 16 coils 111 / 95 / 87 / 83 us; 640^2 to 320^2, 32 coils 286 / 231 / 209 / 223 us;
+// 128^2, 64 coils 104 / 86 / 74 / 70 us; one coil on 64^2 is launch-bound (50 to 52).
+// Transform alone to 640^2 (160 CTAs of 4 columns: two rounds), the rule's / 4 / 16
+// columns: 1 coil 18.5 / 29.3 / 18.5, 2 coils 21.9 / 29.9 / 24.6, 16 coils 72 / 83 / 102.
+int plane_cols(int columns, int coils, int sms)
+{
+    int best = 0;
+    long long least = 0;
+    for (int c : {4, 8, 16}) {
+        const long long rounds = ((columns + c - 1) / c + sms - 1) / sms, turns = ((long long)coils * c + 15) / 16;
+        if (best == 0 || rounds * turns <= least) {
+            best = c;
+            least = rounds * turns;
+        }
+    }
+    return best;
+}
 struct RegKernels {
     int n;
     FftXRegFn x;
-    FftColRegFn col, col_sos, plane_sos;  // plane_sos: kPlaneCols columns per CTA
+    FftColRegFn col, col_sos, sos4, sos8;  // SoS stages of 16, 4 and 8 columns per CTA
     size_t (*xsmem)(int);  // of a warp count
     size_t colsmem;
     int xwarps, xthreads;  // most warps per CTA of the x stage by warps, or (0) threads of the one by CTAs
@@ -494,7 +509,7 @@ constexpr FftXRegFn reg_x_kernel()
 }
 #define FR_REG(N)                                                                                                \
     {N, reg_x_kernel<N>(), fft_col_kernel_reg<N, false>, fft_col_kernel_reg<N, true>,                            \
-     fft_col_kernel_reg<N, true, kPlaneCols>, reg_x_smem<N>, reg_col_smem<N>(), kXWarps<N>,                      \
+     fft_col_kernel_reg<N, true, 4>, fft_col_kernel_reg<N, true, 8>, reg_x_smem<N>, reg_col_smem<N>(), kXWarps<N>, \
      kRegLinesX * RegSplit<N>::TH, kRegCols * RegSplit<N>::TH}
 const RegKernels kRegKernels[] = {
     FR_REG(64),  FR_REG(128), FR_REG(160), FR_REG(192), FR_REG(240), FR_REG(256), FR_REG(320),
@@ -661,8 +676,8 @@ int fftcs_execute(fr_fftcs f, const float *d_grid, int channels, const float *d_
         }
         if (rk->colsmem > 48 * 1024) {
             FR_CUDA(cudaFuncSetAttribute(rk->col, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk->colsmem));
-            FR_CUDA(cudaFuncSetAttribute(f->dim == 2 ? rk->plane_sos : rk->col_sos,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk->colsmem));
+            for (FftColRegFn k : {rk->col_sos, rk->sos4, rk->sos8})
+                FR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk->colsmem));
         }
         XMask xm{};
         if (tiles && tiles->bits) {
@@ -677,8 +692,10 @@ int fftcs_execute(fr_fftcs f, const float *d_grid, int channels, const float *d_
         FR_CHECK_LAUNCH(xw > 0 ? "fft_x_warps_kernel" : "fft_x_kernel_reg");
         const int cb = (rx + kRegCols - 1) / kRegCols;
         if (f->dim == 2) {
-            rk->plane_sos<<<(rx + kPlaneCols - 1) / kPlaneCols, rk->colthreads, rk->colsmem, s>>>(b1, nullptr, y0, ry, rx, rx, 0, 0, rx, tw, C,
-                                                            (long long)G * rx, d_out, d_deapod, sos_mode, 1, 1);
+            const int cc = plane_cols(rx, C, sms);
+            const FftColRegFn plane = cc == 4 ? rk->sos4 : cc == 8 ? rk->sos8 : rk->col_sos;
+            plane<<<(rx + cc - 1) / cc, rk->colthreads, rk->colsmem, s>>>(b1, nullptr, y0, ry, rx, rx, 0, 0, rx, tw, C,
+                                                                          (long long)G * rx, d_out, d_deapod, sos_mode, 1, 1);
             FR_CHECK_LAUNCH("fft_col_kernel_reg(y, sos)");
             return FR_OK;
         }
