@@ -492,7 +492,7 @@ int plane_cols(int columns, int coils, int sms)
 }
 struct RegKernels {
     int n;
-    FftXRegFn x;
+    FftXRegFn x, xfew;  // xfew: by CTAs of 8 lines
     FftColRegFn col, col_sos, sos4, sos8;  // SoS stages of 16, 4 and 8 columns per CTA
     size_t (*xsmem)(int);  // of a warp count
     size_t colsmem;
@@ -508,7 +508,7 @@ constexpr FftXRegFn reg_x_kernel()
         return fft_x_kernel_reg<N>;
 }
 #define FR_REG(N)                                                                                                \
-    {N, reg_x_kernel<N>(), fft_col_kernel_reg<N, false>, fft_col_kernel_reg<N, true>,                            \
+    {N, reg_x_kernel<N>(), fft_x_kernel_reg<N>, fft_col_kernel_reg<N, false>, fft_col_kernel_reg<N, true>,                            \
      fft_col_kernel_reg<N, true, 4>, fft_col_kernel_reg<N, true, 8>, reg_x_smem<N>, reg_col_smem<N>(), kXWarps<N>, \
      kRegLinesX * RegSplit<N>::TH, kRegCols * RegSplit<N>::TH}
 const RegKernels kRegKernels[] = {
@@ -567,6 +567,8 @@ struct fr_fftcs_s {
     DevBuf b2;    // y-stage output (3D)
     int lines_x = 8;
     const RegKernels *reg = nullptr;  // register two-step stages for this G (else Stockham passes)
+    int sms = 0;                      // register stages: SMs, and resident CTAs of the x stage by 1 to 8 warps
+    int xctas[9] = {0};
     cufftHandle xplan = 0;  // 3D, specialised G without register stages: batched 1D x transforms
     DevBuf bx;              // their output: channels x G^3 complex
     ~fr_fftcs_s()
@@ -574,6 +576,26 @@ struct fr_fftcs_s {
         if (xplan) cufftDestroy(xplan);
     }
 };
+
+namespace {
+// What the register stages' launches need of the device, asked once per object: per call
+// these questions cost a transform of one small image a tenth (240^2: 10.3 -> 11.6 us).
+int reg_setup(fr_fftcs f)
+{
+    const RegKernels *rk = f->reg;
+    f->sms = sm_count();
+    FR_CUDA(cudaFuncSetAttribute(rk->x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk->xsmem(rk->xwarps)));
+    FR_CUDA(cudaFuncSetAttribute(rk->xfew, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk->xsmem(0)));
+    for (int w = 1; w <= rk->xwarps; ++w) {
+        int per_sm = 0;
+        FR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rk->x, w * 32, rk->xsmem(w)));
+        f->xctas[w] = std::max(per_sm, 1) * f->sms;
+    }
+    for (FftColRegFn k : {rk->col, rk->col_sos, rk->sos4, rk->sos8})
+        FR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk->colsmem));
+    return FR_OK;
+}
+}  // namespace
 
 extern "C" {
 
@@ -628,6 +650,11 @@ int fr_fft_crop_sos_create(int dim, unsigned G, int channels, const unsigned *ou
         return cuda_fail(e, "twiddle upload");
     }
     f->lines_x = 8;
+    const int st = f->reg ? reg_setup(f) : FR_OK;
+    if (st) {
+        delete f;
+        return st;
+    }
     *out = f;
     return FR_OK;
 }
@@ -660,25 +687,18 @@ int fftcs_execute(fr_fftcs f, const float *d_grid, int channels, const float *d_
     const long long nl = (long long)C * Gz * G;
     if (const RegKernels *rk = f->reg) {
         // register two-step stages: x (cropped), y (cropped), z or y with SoS
-        // the x stage by warps: fewer warps per CTA where the pairs of lines would not reach all SMs
-        const int sms = sm_count();
+        // the x stage by warps: fewer warps per CTA where the pairs of lines would not reach all
+        // SMs; by CTAs of 8 lines, all of whose threads work on step B, where even these do not
+        // fill the GPU (transform to half the size, us: 320^2, 1 coil 12.0 by warps, 10.3 so; 640^2
+        // 18.5, 16.4; 320^2, 3 coils 12.3, 11.3; 4 coils, past the line, 14.3 by warps)
+        const int sms = f->sms;
         const long long npairs = (nl + 1) / 2;
-        const int xw = rk->xwarps == 0 ? 0 : (int)std::min<long long>(rk->xwarps, std::max<long long>(2, npairs / sms));
+        const bool few = nl <= (long long)kRegLinesX * sms;
+        const int xw = rk->xwarps == 0 || few ? 0 : (int)std::min<long long>(rk->xwarps, std::max<long long>(2, npairs / sms));
         const int xthreads = xw > 0 ? xw * 32 : rk->xthreads;
         const size_t xsmem = rk->xsmem(xw);
-        if (xsmem > 48 * 1024)
-            FR_CUDA(cudaFuncSetAttribute(rk->x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xsmem));
-        long long xblocks = (nl + kRegLinesX - 1) / kRegLinesX;
-        if (xw > 0) {
-            int per_sm = 0;
-            FR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rk->x, xthreads, xsmem));
-            xblocks = std::min<long long>((npairs + xw - 1) / xw, (long long)std::max(per_sm, 1) * sms);
-        }
-        if (rk->colsmem > 48 * 1024) {
-            FR_CUDA(cudaFuncSetAttribute(rk->col, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk->colsmem));
-            for (FftColRegFn k : {rk->col_sos, rk->sos4, rk->sos8})
-                FR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk->colsmem));
-        }
+        const long long xblocks = xw > 0 ? std::min<long long>((npairs + xw - 1) / xw, f->xctas[xw])
+                                         : (nl + kRegLinesX - 1) / kRegLinesX;
         XMask xm{};
         if (tiles && tiles->bits) {
             auto lg = [](int v) { return (v & (v - 1)) == 0 ? __builtin_ctz((unsigned)v) : -1; };
@@ -688,7 +708,7 @@ int fftcs_execute(fr_fftcs f, const float *d_grid, int channels, const float *d_
                 return fail(FR_ERR_UNSUPPORTED, "tile masks need power-of-two tile edges");
             if (nl >= (1ll << 31)) return fail(FR_ERR_UNSUPPORTED, "more than 2^31 lines in a tile-masked transform");
         }
-        rk->x<<<(unsigned)xblocks, xthreads, xsmem, s>>>(grid, b1, nl, x0, rx, tw, xm);
+        (xw > 0 ? rk->x : rk->xfew)<<<(unsigned)xblocks, xthreads, xsmem, s>>>(grid, b1, nl, x0, rx, tw, xm);
         FR_CHECK_LAUNCH(xw > 0 ? "fft_x_warps_kernel" : "fft_x_kernel_reg");
         const int cb = (rx + kRegCols - 1) / kRegCols;
         if (f->dim == 2) {
