@@ -12,8 +12,8 @@
 // offsets.  Gridding: one sample-major copy of all frames' dcf * k, then a
 // persistent scatter kernel that takes (coil group, item) work indices from a
 // counter until the batch is done: the tap lanes, or without tap lists (a
-// kernel too wide for them, coil groups of 32, tiles too large, refused, or more
-// than half of the free memory) the kernel that evaluates the taps.  Frame f's k-space is the block channels x
+// kernel too wide for them, coil groups of 32, tiles too large, refused, more
+// than half of the free memory, or sparse frames: lanes_pay) the kernel that evaluates the taps.  Frame f's k-space is the block channels x
 // n_f at complex offset channels * offset[f] and its grid the block
 // channels x G^d at f * channels * G^d.
 // Either way a work item's fixed-point sums have a scale per coil float, from that
@@ -169,6 +169,22 @@ bool drop_tap_lists(fr_batch b)
     return true;
 }
 
+// Whether the tap lanes of `floats` coil floats are the faster scatter of this batch: sparse
+// frames cost their tiles' clearing and writing, which the evaluating kernel's 16 warps and
+// plain coil rows do faster, and the lists' copy and scales come on top. The lines, in
+// samples per cell, are where the two crossed (lists / evaluating, us): 2D, 64 frames of
+// 384^2, 16 coils 0.028 a cell 566 / 477, 0.056 626 / 593, 0.11 741 / 808; 32 of 256^2, 9 coils
+// 0.031 117 / 102, 0.062 128 / 128; 6 coils 0.016 84 / 78, 0.031 95 / 95; 3 coils 0.016 70 / 66,
+// 0.031 78 / 81; 3D, 8 frames of 96^3, 16 coils 0.005 308 / 287, 0.018 409 / 404, 0.036
+// 467 / 509, 8 coils 0.001 158 / 169.
+bool lanes_pay(fr_batch b, int floats)
+{
+    fr_plan p = b->plan;
+    const double cells = (double)b->frames * p->ntiles * p->tile[0] * p->tile[1] * p->tile[2];
+    const double line = p->dim == 3 ? (floats > 16 ? 0.0175 : 0.0) : floats > 16 ? 0.075 : floats > 8 ? 0.03 : 0.02;
+    return floats > 0 && (double)b->n_total >= line * cells;
+}
+
 // The buffers of a call, and whether it takes the tap lists (*lane_floats > 0):
 // where their copy of the k-space does not fit, the taps are evaluated.
 int ensure_scratch(fr_batch b, fr_batch_s::Scratch &sc, int channels, int *lane_floats)
@@ -177,6 +193,7 @@ int ensure_scratch(fr_batch b, fr_batch_s::Scratch &sc, int channels, int *lane_
     const long long K = (long long)p->tile[0] * p->tile[1] * p->tile[2];
     const size_t part = b->nslots > 0 ? grid_partials_bytes(b->nslots, channels, p->coil_group, K) : 0;
     *lane_floats = b->tap_words > 0 ? batch_lane_floats(K, p->coil_group, p->L, channels) : 0;
+    if (!lanes_pay(b, *lane_floats)) *lane_floats = 0;
     if (part > 0 && sc.partials.reserve(part)) {
         if (!drop_tap_lists(b) || sc.partials.reserve(part)) return FR_ERR_OUT_OF_MEMORY;
         *lane_floats = 0;
@@ -372,7 +389,7 @@ int fr_batch_stats(fr_batch b, long long *frames, long long *samples, long long 
         fr_plan p = b->plan;
         const long long K = (long long)p->tile[0] * p->tile[1] * p->tile[2];
         *persistent_ctas = b->blocks;
-        if (b->ready && b->tap_words > 0 && batch_lane_floats(K, p->coil_group, p->L, 1) > 0)
+        if (b->ready && b->tap_words > 0 && lanes_pay(b, batch_lane_floats(K, p->coil_group, p->L, p->coil_group)))
             return batch_lane_ctas(K, p->coil_group, p->L, persistent_ctas);
     }
     return FR_OK;
