@@ -694,7 +694,14 @@ int fftcs_execute(fr_fftcs f, const float *d_grid, int channels, const float *d_
         const int sms = f->sms;
         const long long npairs = (nl + 1) / 2;
         const bool few = nl <= (long long)kRegLinesX * sms;
-        const int xw = rk->xwarps == 0 || few ? 0 : (int)std::min<long long>(rk->xwarps, std::max<long long>(2, npairs / sms));
+        // and for volumes whose every cell is read and more than 3/5 of the outputs are kept, at
+        // sizes up to 384 that are no power of two: the stores, not the loads' latency, bound
+        // those (4 coils, whole transform, by warps / blocks, us: 384^3 to 256^3 1046 / 1032, to 384^3
+        // 1654 / 1598, to 192^3 793 / 818; 320^3 to 320^3 994 / 959; but 480^3, 2 coils, to 432^3
+        // 1820 / 1864, 256^3, 8 coils, to 228^3 963 / 985; with the tiles of a ball 16 coils of 320^3 to
+        // 256^3, reconstructed, 4289 / 4332)
+        const bool stores = f->dim == 3 && !(tiles && tiles->bits) && 5 * rx > 3 * G && G <= 384 && (G & (G - 1)) != 0;
+        const int xw = rk->xwarps == 0 || few || stores ? 0 : (int)std::min<long long>(rk->xwarps, std::max<long long>(2, npairs / sms));
         const int xthreads = xw > 0 ? xw * 32 : rk->xthreads;
         const size_t xsmem = rk->xsmem(xw);
         const long long xblocks = xw > 0 ? std::min<long long>((npairs + xw - 1) / xw, f->xctas[xw])
