@@ -163,9 +163,9 @@ __device__ __forceinline__ float rcp_approx(float a)
 // exponential and reciprocal times the subtracted term over the result, 0.75 at 0.65
 // and falling (+-1 and NaN come out by themselves).  Within 1.7 ulp of FP64 at 1.0 M
 // points, where tanhf promises 2.  A split further out costs the polynomial a degree
-// for each 0.1 to 0.2: 5.1 M samples 602 us, at 0.75 with degree 5 625 us and 1.5 ulp, at 1
-// with degree 6 641 us and 1.2 ulp; without the absolute value and sign 590 us, but
-// 1 - 2 / (e^2x + 1) of a negative x cancels: 3.8 ulp.
+// for each 0.1 to 0.2: 5.1 M samples 602 us (588 since the tables are staged faster), at 0.75
+// with degree 5 625 us and 1.5 ulp, at 1 with degree 6 641 us and 1.2 ulp; without the absolute
+// value and sign 590 us, but 1 - 2 / (e^2x + 1) of a negative x cancels: 3.8 ulp.
 __device__ __forceinline__ f32x2 tanh2(f32x2 x)
 {
     const f32x2 one = pack2(1.f, 1.f);
@@ -194,7 +194,7 @@ __device__ __forceinline__ f32x2 tanh2(f32x2 x)
 // Bound: the pipes of tanh (special functions 45 %, FMA 39 % of the time), the
 // tensor pipe (34 %) and issue (51 %).  5.1 M samples: 775 us with W2 rows of
 // 128 bytes (8-way bank conflicts, the shared pipe 83 % busy), tanhf, and
-// first-layer weights read as single BF16; 612 us so.
+// first-layer weights read as single BF16; 600 us so.
 __device__ __forceinline__ unsigned pack_bf16(float lo_half, float hi_half)
 {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo_half, hi_half);
